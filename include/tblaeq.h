@@ -275,7 +275,14 @@ int tblaeq_set_two_wave(tblaeq_handle* h, int on);
  * either. No counterpart in the reference. */
 int tblaeq_set_knn_probe(tblaeq_handle* h, uint32_t beam, int node_major_completion);
 
-/* Wave 1 of a two-wave KNN batch reads every point of each query's ceil(scale * K / leaf) + 1
+/* With every option at its default (two waves, a beam above 0, the node-major completion, point
+ * groups) and the index resident, a KNN batch runs as a probe and one sweep: the beam walks down to
+ * each query's nearest clusters, their points bound its K-th distance, and every cluster is tested
+ * against that bound at once. The options below then tune the probe (tblaeq_set_knn_wave1: its width,
+ * twelve times as many clusters without a scorer) or do not apply (the refinement: the probe's bound
+ * leaves it nothing). Other choices run the level-synchronous walk. Same results either way.
+ *
+ * Wave 1 of a two-wave KNN batch reads every point of each query's ceil(scale * K / leaf) + 1
  * best-ranked finest clusters (at least 2, at most 32; leaf = the index's points per finest cluster)
  * and takes the K-th distance among them as the bound the rest of the batch prunes with. A larger
  * wave 1 costs more rows up front and tightens the bound (default scale 16). Same results for every

@@ -1,5 +1,6 @@
 // Device-resident index and its derived position-space arrays.
 #include "device_index.hpp"
+#include "knnsweep.cuh"
 #include "traverse.cuh"
 
 #include <omp.h>
@@ -111,7 +112,11 @@ DerivedArrays computeDerived(const HostIndex& idx) {
 
     out.nodeX.resize(H - 1);
     for (uint64_t m = 0; m + 1 < H; ++m) out.nodeX[m] = dec[m];
-    if (floatPointsSupported(D) && H >= 2) {
+    // Rows of the float copies and boxes are padded to 16 bytes with zeros.
+    const uint64_t DP = paddedDims(D);
+    for (const auto& mesh : dec)
+        for (double v : mesh) out.maxAbs = std::max(out.maxAbs, std::fabs(v));
+    if (H >= 2 && D <= 32) {
         // Point groups: every finest cluster's rows, reordered within the cluster's own row range by
         // median splits along the widest dimension until at most kPointGroup rows remain, and the
         // float copy of the points in that order.
@@ -126,10 +131,10 @@ DerivedArrays computeDerived(const HostIndex& idx) {
             out.clusterGroup[c + 1] = out.clusterGroup[c] + (out.ccnt[H - 2][c] ? leaves(out.ccnt[H - 2][c]) : 0u);
         const uint64_t G = out.clusterGroup[nCl];
         out.pointPerm.resize(nRows);
-        out.pointsF.resize(nRows * D);
+        out.pointsF.assign(nRows * DP, 0.f);
         out.groupFirst.resize(G);
         out.groupCount.resize(G);
-        out.groupBox.resize(G * 2 * D);
+        out.groupBox.assign(G * 2 * DP, 0.f);
         auto down = [](double v) {
             float f = static_cast<float>(v);
             if (static_cast<double>(f) > v) f = std::nextafter(f, -std::numeric_limits<float>::infinity());
@@ -155,7 +160,7 @@ DerivedArrays computeDerived(const HostIndex& idx) {
                 if (k <= kPointGroup) {
                     out.groupFirst[g] = b + f;
                     out.groupCount[g] = k;
-                    float* box = &out.groupBox[static_cast<size_t>(g) * 2 * D];
+                    float* box = &out.groupBox[static_cast<size_t>(g) * 2 * DP];
                     for (uint64_t d = 0; d < D; ++d) {
                         double lo = std::numeric_limits<double>::infinity(), hi = -lo;
                         for (uint32_t i = f; i < f + k; ++i) {
@@ -163,7 +168,7 @@ DerivedArrays computeDerived(const HostIndex& idx) {
                             hi = std::max(hi, pts[rows[i] * D + d]);
                         }
                         box[d] = down(lo);
-                        box[D + d] = up(hi);
+                        box[DP + d] = up(hi);
                     }
                     ++g;
                     continue;
@@ -193,7 +198,7 @@ DerivedArrays computeDerived(const HostIndex& idx) {
             for (uint32_t i = 0; i < n; ++i) {
                 out.pointPerm[b + i] = rows[i];
                 for (uint64_t d = 0; d < D; ++d)
-                    out.pointsF[(static_cast<size_t>(b) + i) * D + d] = static_cast<float>(pts[static_cast<size_t>(rows[i]) * D + d]);
+                    out.pointsF[(static_cast<size_t>(b) + i) * DP + d] = static_cast<float>(pts[static_cast<size_t>(rows[i]) * D + d]);
             }
         }
     }
@@ -427,6 +432,9 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
     di->leaf.resize(idx.height - 1);
     di->aabb.resize(idx.height - 1);
     di->nodeX.resize(idx.height - 1);
+    di->nodeXF.resize(idx.height - 1);
+    di->radF.resize(idx.height - 1);
+    di->maxAbs = der.maxAbs;
     for (uint64_t m = 0; m + 1 < idx.height; ++m) {
         const size_t n = der.cbeg[m].size();
         std::vector<NodeRec> ref(n), sub(n);
@@ -439,6 +447,17 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
         di->leaf[m] = upload(der.leaf[m], s);
         di->aabb[m] = upload(der.aabb[m], s);
         di->nodeX[m] = upload(der.nodeX[m], s);
+        // Padded float centres and rounded-up subtree radii, for the KNN probe and sweep.
+        const uint64_t DP = paddedDims(idx.D);
+        std::vector<float> xf(n * DP, 0.f), rf(n);
+        for (size_t i = 0; i < n; ++i) {
+            for (uint64_t d = 0; d < idx.D; ++d) xf[i * DP + d] = static_cast<float>(der.nodeX[m][i * idx.D + d]);
+            float r = static_cast<float>(der.radSub[m][i]);
+            if (static_cast<double>(r) < der.radSub[m][i]) r = std::nextafter(r, std::numeric_limits<float>::infinity());
+            rf[i] = r;
+        }
+        di->nodeXF[m] = upload(xf, s);
+        di->radF[m] = upload(rf, s);
         TBLAEQ_CUDA(cudaStreamSynchronize(s));
     }
     if (!der.pointsD.empty() && idx.intervals > 0 && res(idx.intervals - 1) == kResident) {
@@ -477,7 +496,7 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
 
 size_t DeviceIndex::deviceBytes() const {
     size_t t = coarseVals.bytes() + coarseIds.bytes();
-    for (auto* v : {&pvals, &nodeRef, &nodeSub, &leaf, &aabb, &nodeX, &nodeOrig, &maps})
+    for (auto* v : {&pvals, &nodeRef, &nodeSub, &leaf, &aabb, &nodeX, &nodeXF, &radF, &nodeOrig, &maps})
         for (auto& m : *v) t += m.bytes();
     return t + pointsD.bytes() + pointsF.bytes() + pointPerm.bytes() + groupRec.bytes() + groupBox.bytes() + clusterGroups.bytes();
 }

@@ -83,8 +83,8 @@ struct DerivedArrays {
     // Decoded coordinates of every node (position order, D per node), as the traversal rebuilds
     // them (y = P[j] * x_parent, one rounded multiply per level).
     std::vector<std::vector<double>> nodeX;
-    // Point groups of the finest exact range level (empty where its float test has no kernel: D not
-    // 4, 8, 16). Every finest cluster's rows are reordered within the cluster's own row range by
+    // Point groups of the finest exact levels. Float rows here and in groupBox are padded with zeros
+    // to paddedDims(D) floats, 16-byte pieces. Every finest cluster's rows are reordered within the cluster's own row range by
     // median splits along the widest dimension until at most kPointGroup rows remain; each run so
     // formed is a point group, with the box of its points.
     std::vector<float> pointsF;          // decoded finest points in that order, floats rounded to nearest
@@ -96,6 +96,7 @@ struct DerivedArrays {
     // Decoded finest points (y = P[j] * x_parent, one rounded multiply per dimension), in
     // point-group order when the groups exist (pointPerm maps back to rows), else in row order.
     std::vector<double> pointsD;
+    double maxAbs = 0.0;                 // largest |coordinate| of any mesh
 };
 
 // Most points of one point group.
@@ -150,6 +151,8 @@ struct DeviceIndex {
     std::vector<DeviceMem> leaf;             // mesh m < height-1: finest points below each node (uint32)
     std::vector<DeviceMem> aabb;             // mesh m < height-1: outward-rounded float box of the points below
     std::vector<DeviceMem> nodeX;            // mesh m < height-1: decoded coordinates (D doubles per node)
+    std::vector<DeviceMem> nodeXF, radF;     // mesh m < height-1: the same as padded floats; subtree radius, rounded up
+    double maxAbs = 0.0;                     // largest |coordinate| of any mesh
     // Finest exact range level, when the last interval's rows are device-resident (else empty): the
     // points as floats in point-group order (DerivedArrays::pointsF), that order's row map, every
     // group's record {0, first row, rows} and box, and every finest cluster's record

@@ -5,6 +5,7 @@
 #include <limits>
 
 #include "knn.cuh"
+#include "knnsweep.cuh"
 
 #include <algorithm>
 
@@ -36,8 +37,13 @@ void BatchEngine::resetWorkspace() noexcept {
                          &candD2_, &excl_, &probeK_, &resIds_, &resVals_, &resQ_, &resDist_, &zeroBlock_, &cmpCnt_,
                          &cmpKids_, &cmpEntryOff_, &cmpKidOff_, &offsets_, &boxF_, &tau_, &candOff_, &knnCount_,
                          &knnOff_, &knnIds_, &knnD2_, &lbE_, &scoreE_, &sel_, &offF_, &waveM_, &selCount_, &selOff_,
-                         &selIds_, &selD2_, &candOffB_, &candOffS_, &resIdsB_, &resQB_, &resDistB_})
+                         &selIds_, &selD2_, &candOffB_, &candOffS_, &resIdsB_, &resQB_, &resDistB_, &swQuery_, &swBits_,
+                         &swLive_, &swCand_, &swEnt_})
         m->release();
+    swQcap_ = 0;
+    swLast_ = false;
+    swCandCap_ = swEntCap_ = 0;
+    swFactor_ = 1;
     caps_ = EngineCaps{};
     qcap_ = 0;
     haveVals_ = false;
@@ -182,7 +188,7 @@ void BatchEngine::levelCounts(std::vector<uint64_t>& entries, std::vector<uint64
 
 uint64_t BatchEngine::lastTotal(uint32_t nq) {
     uint64_t total = 0;
-    const uint64_t* off = lastKnn_ ? knnOff_.as<uint64_t>() : offsets_.as<uint64_t>();
+    const uint64_t* off = lastKnn_ ? (swLast_ ? swOff_ : knnOff_.as<uint64_t>()) : offsets_.as<uint64_t>();
     TBLAEQ_CUDA(cudaMemcpyAsync(&total, off + nq, 8, cudaMemcpyDeviceToHost, stream_));
     TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
     return total;
@@ -678,7 +684,7 @@ BatchOutput BatchEngine::output(uint32_t nq, unsigned flags) const {
     BatchOutput o;
     o.nq = nq;
     if (lastKnn_) {
-        o.offsets = knnOff_.as<uint64_t>();
+        o.offsets = swLast_ ? swOff_ : knnOff_.as<uint64_t>();
         o.ids = knnIds_.as<uint64_t>();
         o.dist2 = knnD2_.as<double>();
         o.levelItems = (flags & kWantLevels)
@@ -1079,7 +1085,7 @@ void BatchEngine::enqueueKnn(const double* dPoints, uint32_t nq, const uint32_t*
         c.decoded = di_.pointsD.bytes() ? di_.pointsD.as<double>() : nullptr;
         if (c.decoded && di_.pointPerm.bytes()) {  // decoded points in point-group order
             c.perm = di_.pointPerm.as<uint32_t>();
-            if (knnGroups_) {
+            if (knnGroups_ && paddedDims(di_.D) == di_.D) {  // this kernel reads unpadded boxes
                 c.clusterGroups = di_.clusterGroups.as<NodeRec>();
                 c.groupRec = di_.groupRec.as<NodeRec>();
                 c.groupBox = di_.groupBox.as<float>();
@@ -1276,10 +1282,191 @@ bool BatchEngine::growKnnMajor() {
     return grew;
 }
 
+bool BatchEngine::useKnnSweep(unsigned flags) const {
+    // Per-level counts and the scorer's training traces describe the level-synchronous walk, and so do
+    // the options that change it; a streamed last interval has no decoded points on the device.
+    return twoWave_ && knnNodeMajor_ && probeBeam_ > 0 && knnGroups_ && !knnTrace_ && !(flags & kWantLevels) &&
+           di_.height >= 2 && di_.height <= kSweepMaxHeight && di_.pointsD.bytes() && di_.pointsF.bytes() &&
+           di_.maxAbs <= kSweepMaxAbs;
+}
+
+// Queries per block of the sweep: the bits of a block take at most 512 MiB.
+uint32_t BatchEngine::knnSweepBlock(uint32_t nq) const {
+    const uint64_t rows = std::max<uint64_t>(1, di_.meshCount[di_.height - 2]);
+    const uint64_t words = std::max<uint64_t>(8, (512ull << 20) / (rows * 4) / 8 * 8);
+    return static_cast<uint32_t>(std::min<uint64_t>(nq, words * 32));
+}
+
+void BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK) {
+    const uint64_t D = di_.D, DP = paddedDims(D), nC = di_.meshCount[di_.height - 2];
+    if (swQcap_ < nq) {
+        swQcap_ = nq;
+        // tau, result offsets, candidate offsets (8 bytes); float rows; margin, tauF, thrF, counts,
+        // entry offsets and counts (4 bytes)
+        swQuery_.alloc((static_cast<uint64_t>(nq) + 1) * (3 * 8 + DP * 4 + 6 * 4) + 1024);
+    }
+    const uint32_t block = knnSweepBlock(nq);
+    const uint64_t words = block <= 32 ? 1 : (((static_cast<uint64_t>(block) + 31) / 32 + 3) / 4 * 4);
+    if (swBits_.bytes() < nC * words * 4) swBits_.alloc(nC * words * 4);
+    if (swLive_.bytes() < nC * 4 + 256) swLive_.alloc(nC * 4 + 256);
+    const uint64_t cand = swFactor_ * (4 * sumK + 64ull * nq);
+    if (swCandCap_ < cand) {
+        swCand_.alloc(cand * 16);
+        swCandCap_ = cand;
+    }
+    if (scorer_) {
+        // The clusters under the beam: probeBeam_ nodes' children per query, grown on overflow.
+        const uint64_t up = di_.height > 2 ? std::max<uint64_t>(1, di_.meshCount[di_.height - 3]) : 0;
+        const uint64_t each = std::min<uint64_t>(nC, up ? probeBeam_ * ((nC + up - 1) / up) : nC);
+        const uint64_t want = std::max<uint64_t>(swEntCap_, nq * each * 5 / 4 + 1024);
+        if (swEnt_.bytes() < want * (4 + 4 + 8 * D + 8)) swEnt_.alloc(want * (4 + 4 + 8 * D + 8));
+        swEntCap_ = want;
+    }
+    if (knnCap_ < std::max<uint64_t>(sumK, 1)) {
+        knnCap_ = std::max<uint64_t>(sumK, 1);
+        knnIds_.alloc(knnCap_ * 8);
+        knnD2_.alloc(knnCap_ * 8);
+    }
+}
+
+void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK) {
+    lastKnn_ = true;
+    lastCompletion_ = true;
+    const int H = static_cast<int>(di_.height);
+    const uint64_t D = di_.D, DP = paddedDims(D);
+    char* z = zeroBlock_.as<char>();
+    if (timing_) record(0);
+    // Tickets, status, headers and the work counters (neighbours in the block).
+    TBLAEQ_CUDA(cudaMemsetAsync(z + offTickets_, 0, offQcount_ - offTickets_, stream_));
+    TBLAEQ_CUDA(cudaMemsetAsync(z + offWork_, 0, 16, stream_));
+    KnnSweepArgs a{};
+    a.D = static_cast<int>(D);
+    a.height = H;
+    a.nq = nq;
+    a.points = dPoints;
+    a.K = dK;
+    a.maxAbs = di_.maxAbs;
+    a.nPoints = di_.meshCount[H - 1];
+    for (int m = 0; m + 1 < H; ++m)
+        a.level[m] = KnnSweepLevel{di_.nodeXF[m].as<float>(), di_.radF[m].as<float>(),
+                                   di_.nodeSub[m].as<NodeRec>(), di_.leaf[m].as<uint32_t>(), static_cast<uint32_t>(di_.meshCount[m])};
+    a.pointsF = di_.pointsF.as<float>();
+    a.pointsD = di_.pointsD.as<double>();
+    a.perm = di_.pointPerm.as<uint32_t>();
+    a.map = di_.mapPtr[H - 1];
+    a.clusterGroups = di_.clusterGroups.as<NodeRec>();
+    a.groupRec = di_.groupRec.as<NodeRec>();
+    a.groupBox = di_.groupBox.as<float>();
+    const size_t q1 = static_cast<size_t>(swQcap_) + 1;
+    char* b = swQuery_.as<char>();
+    a.qF = reinterpret_cast<float*>(b);  // 16-byte rows first
+    b += align256(q1 * DP * 4);
+    a.tau = reinterpret_cast<double*>(b);
+    a.outOff = reinterpret_cast<uint64_t*>(a.tau + q1);
+    a.candOff = a.outOff + q1;
+    a.margin = reinterpret_cast<float*>(a.candOff + q1);
+    a.tauF = a.margin + q1;
+    a.thrF = a.tauF + q1;
+    a.candCnt = reinterpret_cast<uint32_t*>(a.thrF + q1);
+    a.entOff = a.candCnt + q1;
+    a.entCnt = a.entOff + q1;
+    swOff_ = a.outOff;
+    a.candFactor = static_cast<uint32_t>(swFactor_);
+    a.candCap = swCandCap_;
+    a.candId = swCand_.as<uint64_t>();
+    a.candD2 = reinterpret_cast<double*>(a.candId + swCandCap_);
+    a.beam = probeBeam_;
+    a.waveFactor = waveScale_ * static_cast<double>(di_.meshCount[H - 2]) / static_cast<double>(di_.meshCount[H - 1]);
+    a.liveCnt = swLive_.as<uint32_t>();
+    a.ticket = a.liveCnt + 1;
+    a.live = a.liveCnt + 64;
+    a.bits = swBits_.as<uint32_t>();
+    a.hdr = hdrPtr(0);
+    a.work = reinterpret_cast<unsigned long long*>(z + offWork_);
+    a.status = reinterpret_cast<uint32_t*>(z + offStatus_);
+    launchKnnSweepPrepare(a, stream_);
+    if (timing_) record(1);
+    if (scorer_) {
+        a.entCap = static_cast<uint32_t>(std::min<uint64_t>(swEntCap_, 0xffffffffull));
+        a.entX = swEnt_.as<double>();
+        double* score = a.entX + swEntCap_ * D;
+        a.score = score;
+        a.entQ = reinterpret_cast<uint32_t*>(score + swEntCap_);
+        a.entNode = a.entQ + swEntCap_;
+        a.nodeX = di_.nodeX[H - 2].as<double>();
+        launchKnnProbe(a, kProbeEntries, stream_);
+        FrontierIn f{};
+        f.q = a.entQ;
+        f.x = a.entX;
+        f.hdr = hdrPtr(H - 1);
+        f.cap = a.entCap;
+        scorer_(scorerCtx_, f, a.entNode, a.entCap, dPoints, score, stream_);
+        launchKnnProbe(a, kProbeBound, stream_);
+    } else {
+        launchKnnProbe(a, kProbeWhole, stream_);
+    }
+    if (timing_)
+        for (int m = 0; m + 1 < H; ++m) record(2 + m);
+    const uint32_t block = knnSweepBlock(nq);
+    for (uint32_t q0 = 0; q0 < nq; q0 += block) {
+        a.qBegin = q0;
+        a.qEnd = std::min(nq, q0 + block);
+        const uint32_t n = a.qEnd - q0;
+        a.words = n <= 32 ? 1 : ((n + 31) / 32 + 3) / 4 * 4;
+        if (q0) TBLAEQ_CUDA(cudaMemsetAsync(a.liveCnt, 0, 8, stream_));  // live clusters and the ticket
+        launchKnnSweepBound(a, stream_);
+        launchKnnSweepPoints(a, stream_);
+    }
+    if (timing_) record(1 + H);
+    launchTopK(a.candOff, a.candId, a.candD2, a.candCap, nullptr, nullptr, nullptr, 0, dK, nq, a.outOff,
+               knnIds_.as<uint64_t>(), knnD2_.as<double>(), nullptr, a.status, stream_, a.candCnt);
+    if (timing_) record(2 + H);
+}
+
+bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o) {
+    // Candidate slots start at 4 K + 64 a query (the bound is within a few percent of the K-th
+    // distance, so about 1.5 K pass); ties and bounds that stayed loose grow them, at most 256-fold.
+    const uint64_t cap = std::min<uint64_t>(sumK, nq * di_.meshCount[di_.height - 1]);
+    for (int attempt = 0; attempt < 8; ++attempt) {
+        lastRuns_ = static_cast<uint32_t>(attempt + 1);
+        reserveKnnSweep(nq, cap);
+        enqueueKnnSweep(dPoints, nq, dK);
+        uint32_t st = 0;
+        uint32_t entries = 0;
+        uint64_t total = 0;
+        TBLAEQ_CUDA(cudaMemcpyAsync(&st, zeroBlock_.as<char>() + offStatus_, 4, cudaMemcpyDeviceToHost, stream_));
+        TBLAEQ_CUDA(cudaMemcpyAsync(&total, swOff_ + nq, 8, cudaMemcpyDeviceToHost, stream_));
+        TBLAEQ_CUDA(cudaMemcpyAsync(&entries, hdrPtr(static_cast<int>(di_.height) - 1), 4, cudaMemcpyDeviceToHost, stream_));
+        TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+        if (st & kStatusKnnFallback) return false;
+        if (st == 0) {
+            if (splitLimit_ < 0xffffffffull) checkSplitLimit();
+            swLast_ = true;
+            o = output(nq, 0);
+            o.total = total;
+            return true;
+        }
+        if (scorer_ && entries > swEntCap_) {
+            swEntCap_ = entries + entries / 4;
+        } else if (swFactor_ >= 256) {
+            swFactor_ = 1;
+            return false;
+        } else {
+            swFactor_ *= 4;
+        }
+    }
+    return false;
+}
+
 BatchOutput BatchEngine::runKnn(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK,
                                 unsigned flags) {
     WorkspaceGuard guard(*this);
     reserve(caps_, nq, flags);
+    swLast_ = false;
+    if (nq > 0 && useKnnSweep(flags)) {
+        BatchOutput o;
+        if (runKnnSweep(dPoints, nq, dK, sumK, o)) return o;
+    }
     reserveKnn(nq);
     if (knnCap_ < std::max<uint64_t>(sumK, 1)) {
         knnCap_ = std::max<uint64_t>(sumK, 1);

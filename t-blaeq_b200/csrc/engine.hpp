@@ -121,6 +121,8 @@ public:
     uint64_t graphKernels() const { return graphExec_ ? graphKernels_ : 0; }
     uint64_t graphNodes() const { return graphExec_ ? graphNodes_ : 0; }
     bool twoWave() const { return twoWave_; }
+    // Keep the last KNN batch's final frontier (lastKnnFrontier): batches run the level-synchronous walk.
+    void setKnnTrace(bool on) { knnTrace_ = on; }
     // Optional device scorer of the last frontier's entries (higher = expand earlier); when unset
     // the entries are ranked by their lower bound. Called with (frontier, hdr, cap, points, out scores).
     using EntryScorer = void (*)(void* ctx, const FrontierIn& f, const uint32_t* node, uint32_t cap,
@@ -251,6 +253,19 @@ private:
     // offsets into zeroBlock_
     size_t offDesc_ = 0, offTickets_ = 0, offStatus_ = 0, offHdr_ = 0, offQcount_ = 0, offLevels_ = 0;
     uint64_t tileCap_ = 0;
+
+    // Exact KNN as a probe and one sweep (knnsweep.cuh): workspace, and whether the last batch ran it.
+    // runKnnSweep returns false when the batch needs the level-synchronous path instead.
+    DeviceMem swQuery_, swBits_, swLive_, swCand_, swEnt_;
+    uint32_t swQcap_ = 0;
+    uint64_t swCandCap_ = 0, swEntCap_ = 0, swFactor_ = 1;
+    uint64_t* swOff_ = nullptr;
+    bool swLast_ = false, knnTrace_ = false;
+    bool useKnnSweep(unsigned flags) const;
+    uint32_t knnSweepBlock(uint32_t nq) const;
+    void reserveKnnSweep(uint32_t nq, uint64_t sumK);
+    void enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK);
+    bool runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o);
 
     void growFromHeaders();
     void checkSplitLimit();  // throws SplitBatch when the last batch's levels exceed splitLimit_

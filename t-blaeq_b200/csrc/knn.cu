@@ -187,24 +187,32 @@ __global__ void __launch_bounds__(1024) stepKernel(const uint64_t* keys, const u
 }
 
 constexpr int kTopKStage = 4096;  // candidates a CTA sorts in shared memory
+constexpr uint64_t kTopKCount = 512;  // candidates a CTA places by counting (one per thread)
+
+// The double of an orderKey.
+__device__ __forceinline__ double keyValue(uint64_t b) {
+    b = (b & 0x8000000000000000ull) ? (b & 0x7fffffffffffffffull) : ~b;
+    return __longlong_as_double(static_cast<long long>(b));
+}
 
 __global__ void __launch_bounds__(512) topKKernel(const uint64_t* offA, const uint64_t* idsA, const double* d2A,
                                                   uint64_t capA, const uint64_t* offB, const uint64_t* idsB,
                                                   const double* d2B, uint64_t capB, const uint32_t* Kq,
                                                   const uint64_t* outOff, uint64_t* outIds, double* outD2,
-                                                  uint32_t* outCount, uint32_t* status) {
+                                                  uint32_t* outCount, uint32_t* status, const uint32_t* cntA) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* sk = reinterpret_cast<uint64_t*>(smem);
     uint64_t* sv = sk + kTopKStage;
     const uint32_t q = blockIdx.x;
-    const uint64_t a0 = offA[q], na = offA[q + 1] - a0;
+    const uint64_t a0 = offA[q], slots = offA[q + 1] - a0;
+    const uint64_t na = cntA ? std::min<uint64_t>(cntA[q], slots) : slots;
     const uint64_t b0 = offB ? offB[q] : 0, nb = offB ? offB[q + 1] - b0 : 0;
     const uint64_t n = na + nb;
     const uint32_t K = Kq[q];
     // Candidates beyond the arrays mean the producer overflowed: never read them.
     if (a0 + na > capA || (offB && b0 + nb > capB)) {
         if (threadIdx.x == 0) {
-            outCount[q] = 0;
+            if (outCount) outCount[q] = 0;
             atomicOr(status, kStatusOverflowEntries);
         }
         return;
@@ -215,9 +223,34 @@ __global__ void __launch_bounds__(512) topKKernel(const uint64_t* offA, const ui
         if (i < na) return idsA ? idsA[a0 + i] : a0 + i;  // no id array: the candidate's position
         return idsB ? idsB[b0 + i - na] : b0 + i - na;
     };
-    if (threadIdx.x == 0) outCount[q] = static_cast<uint32_t>(keep);
+    if (threadIdx.x == 0 && outCount) outCount[q] = static_cast<uint32_t>(keep);
     if (keep == 0) return;
     const uint64_t o = outOff[q];
+    if (n <= kTopKCount) {
+        // One candidate per thread: its place is the number of smaller ones, counted over the staged
+        // keys (broadcast reads), instead of the sort's log^2 rounds with a barrier each. 4,096 queries
+        // of about 70 candidates take 68 us this way (about 60: 79 us sorted).
+        const uint32_t t = threadIdx.x;
+        uint64_t k = ~0ull, v = ~0ull;
+        if (t < n) {
+            k = keyAt(t);
+            v = idAt(t);
+            sk[2 * t] = k;
+            sk[2 * t + 1] = v;
+        }
+        __syncthreads();
+        if (t >= n) return;
+        uint32_t place = 0;
+        for (uint32_t i = 0; i < static_cast<uint32_t>(n); ++i) {
+            const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(sk + 2 * i);
+            place += (c.x < k || (c.x == k && (c.y < v || (c.y == v && i < t)))) ? 1u : 0u;
+        }
+        if (place < keep) {
+            outIds[o + place] = v;
+            outD2[o + place] = keyValue(k);
+        }
+        return;
+    }
     // Sorts sk/sv[0, count) by (key, id) with a bitonic network and writes the first `keep`.
     auto sortAndWrite = [&](uint32_t count) {
         int size = 1;
@@ -555,7 +588,7 @@ void launchStep(const uint64_t* keys, const uint32_t* labels, const uint32_t* cn
 void launchTopK(const uint64_t* offA, const uint64_t* idsA, const double* d2A, uint64_t capA, const uint64_t* offB,
                 const uint64_t* idsB, const double* d2B, uint64_t capB, const uint32_t* K, uint32_t nq,
                 const uint64_t* outOff, uint64_t* outIds, double* outD2, uint32_t* outCount, uint32_t* status,
-                cudaStream_t s) {
+                cudaStream_t s, const uint32_t* cntA) {
     if (nq == 0) return;
     const size_t smem = static_cast<size_t>(kTopKStage) * 16;
     static bool attr = false;
@@ -565,7 +598,7 @@ void launchTopK(const uint64_t* offA, const uint64_t* idsA, const double* d2A, u
         attr = true;
     }
     topKKernel<<<nq, 512, smem, s>>>(offA, idsA, d2A, capA, offB, idsB, d2B, capB, K, outOff, outIds, outD2, outCount,
-                                     status);
+                                     status, cntA);
     TBLAEQ_LAUNCHED();
 }
 

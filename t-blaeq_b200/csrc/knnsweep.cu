@@ -1,0 +1,745 @@
+// Exact KNN: probe, dense cluster bound and point sweep (see knnsweep.cuh).
+#include "knnsweep.cuh"
+
+#include <algorithm>
+#include <type_traits>
+
+namespace tblaeq {
+
+namespace {
+
+constexpr uint32_t FULL = 0xffffffffu;
+constexpr float kRel = 1.00001f;  // the float sums' relative error: (D + 3) 2^-24 < 2.1e-6 for D <= 32
+
+__device__ __forceinline__ uint32_t floatKey(float f) {  // order-preserving bits
+    const uint32_t u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// ---- prepare: float queries, result and candidate slots ------------------------------------------
+// One block scans K (results are min(K, points) per query, known before any search); all blocks convert
+// the queries. margin[q] bounds the distance error of rounding the query's and a data point's
+// coordinates to float: sqrt(D) 2^-24 (|q| + |x|) each way, doubled.
+__global__ void __launch_bounds__(1024) sweepPrepareKernel(KnnSweepArgs a, uint32_t DP) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (uint32_t q = blockIdx.x * blockDim.x + tid; q < a.nq; q += gridDim.x * blockDim.x) {
+        double m = 0.0;
+        bool ok = true;
+        const uint32_t K = a.K[q];
+        for (int d = 0; d < a.D; ++d) {
+            const double p = a.points[static_cast<size_t>(q) * a.D + d];
+            ok = ok && fabs(p) <= kSweepMaxAbs;  // false for NaN
+            m = fmax(m, fabs(p));
+        }
+        if (!ok || K > kProbePoints / 2) atomicOr(a.status, kStatusKnnFallback);
+        for (uint32_t d = 0; d < DP; ++d)
+            a.qF[static_cast<size_t>(q) * DP + d] =
+                d >= static_cast<uint32_t>(a.D) ? 0.f
+                : K == 0                        ? static_cast<float>(kSweepMaxAbs)
+                                                : static_cast<float>(a.points[static_cast<size_t>(q) * a.D + d]);
+        a.margin[q] = __double2float_ru(sqrt(static_cast<double>(a.D)) * (m + a.maxAbs) * 1.2e-7);
+        a.candCnt[q] = 0;
+    }
+    if (blockIdx.x) return;
+    __shared__ unsigned long long sCarryR, sCarryC, sR[32], sC[32];
+    if (tid == 0) {
+        sCarryR = sCarryC = 0;
+        *a.liveCnt = 0;
+        *a.ticket = 0;
+    }
+    __syncthreads();
+    for (uint32_t base = 0; base < a.nq; base += blockDim.x) {
+        const uint32_t q = base + tid;
+        const uint32_t K = q < a.nq ? a.K[q] : 0u;
+        const unsigned long long r = min(static_cast<unsigned long long>(K), static_cast<unsigned long long>(a.nPoints));
+        const unsigned long long c = q < a.nq ? static_cast<unsigned long long>(a.candFactor) * (4ull * r + 64ull) : 0ull;
+        unsigned long long ir = r, ic = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(FULL, ir, o), u = __shfl_up_sync(FULL, ic, o);
+            if (lane >= static_cast<uint32_t>(o)) {
+                ir += t;
+                ic += u;
+            }
+        }
+        if (lane == 31) {
+            sR[warp] = ir;
+            sC[warp] = ic;
+        }
+        __syncthreads();
+        unsigned long long br = sCarryR, bc = sCarryC;
+        for (uint32_t w = 0; w < warp; ++w) {
+            br += sR[w];
+            bc += sC[w];
+        }
+        if (q < a.nq) {
+            a.outOff[q] = br + ir - r;
+            a.candOff[q] = bc + ic - c;
+        }
+        __syncthreads();
+        if (tid == blockDim.x - 1) {
+            sCarryR = br + ir;
+            sCarryC = bc + ic;
+        }
+        __syncthreads();
+    }
+    if (tid == 0) {
+        a.outOff[a.nq] = sCarryR;
+        a.candOff[a.nq] = sCarryC;
+        a.hdr[0] = a.nq;
+        a.hdr[1] = a.nq * a.level[0].count;
+    }
+}
+
+// ---- probe ----------------------------------------------------------------------------------------
+constexpr int kProbeThreads = 256;
+constexpr int kProbeWarps = kProbeThreads / 32;
+
+__device__ __forceinline__ uint64_t shflXor64(uint64_t v, int o) { return __shfl_xor_sync(FULL, v, o); }
+
+// The warp's 32 smallest keys so far, ascending over the lanes.
+struct WarpBest {
+    uint64_t best = ~0ull;
+    // Sorts v over the lanes and keeps the 32 smallest of both (bitonic networks).
+    __device__ __forceinline__ void add(uint64_t v, int lane) {
+        const uint64_t worst = __shfl_sync(FULL, best, 31);
+        if (__ballot_sync(FULL, v < worst) == 0) return;
+#pragma unroll
+        for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                const uint64_t o = shflXor64(v, stride);
+                const bool up = ((lane & size) == 0) == ((lane & stride) == 0);
+                v = (up == (o < v)) ? o : v;
+            }
+        }
+        merge(v, lane);
+    }
+    // v ascending over the lanes.
+    __device__ __forceinline__ void merge(uint64_t v, int lane) {
+        const uint64_t r = __shfl_sync(FULL, v, 31 - lane);
+        best = min(best, r);
+#pragma unroll
+        for (int stride = 16; stride > 0; stride >>= 1) {
+            const uint64_t o = shflXor64(best, stride);
+            const bool low = (lane & stride) == 0;
+            best = (low == (o < best)) ? o : best;
+        }
+    }
+};
+
+// Distance between two padded float rows; b may lie in global memory.
+template <int DP>
+__device__ __forceinline__ float rowDist2(const float (&p)[DP], const float* x) {
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int d = 0; d < DP; d += 4) {
+        const float4 c = __ldg(reinterpret_cast<const float4*>(x + d));
+        const float2 e = __fadd2_rn(make_float2(p[d], p[d + 1]), make_float2(-c.x, -c.y));
+        const float2 f = __fadd2_rn(make_float2(p[d + 2], p[d + 3]), make_float2(-c.z, -c.w));
+        s = __ffma2_rn(e, e, s);
+        s = __ffma2_rn(f, f, s);
+    }
+    return s.x + s.y;
+}
+
+// FP64 squared distance of a decoded point (the products the traversal rebuilds), fma in dimension
+// order: the value KNN results report.
+__device__ __forceinline__ double pointDist2(const double* p, const double* y, int D) {
+    double s = 0.0;
+    if ((D & 1) == 0) {  // rows start on 16-byte boundaries
+        for (int d = 0; d < D; d += 2) {
+            const double2 v = __ldg(reinterpret_cast<const double2*>(y + d));
+            const double e = p[d] - v.x;
+            s = __fma_rn(e, e, s);
+            const double f = p[d + 1] - v.y;
+            s = __fma_rn(f, f, s);
+        }
+    } else {
+        for (int d = 0; d < D; ++d) {
+            const double e = p[d] - __ldg(y + d);
+            s = __fma_rn(e, e, s);
+        }
+    }
+    return s;
+}
+
+// One CTA per query. Every warp keeps the 32 best of the nodes it ranked in registers; the eight lists
+// merge through shared memory once per level. The chain of levels is what bounds it (a few thousand
+// nodes and points per query, latency between the levels), so each CTA is small and several share
+// an SM: 252 us for 4,096 queries (N = 10M, D = 8), 39 us for one.
+template <int DP>
+__global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(KnnSweepArgs a, int phase) {
+    __shared__ uint64_t sMerge[kProbeWarps][32];
+    __shared__ uint32_t sBeg[32], sPre[33];
+    __shared__ float sKeys[kProbePoints];
+    __shared__ uint32_t sHist[256];
+    __shared__ uint32_t sSel[2], sTauUb;
+    __shared__ uint64_t sScored[32];
+    const uint32_t q = blockIdx.x;
+    const uint32_t K = a.K[q];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int H = a.height;
+    if (*a.status & kStatusKnnFallback) return;
+    if (K == 0) {
+        if (tid == 0) {
+            a.tau[q] = -1.0;
+            a.tauF[q] = 0.f;
+            a.thrF[q] = -1.f;
+            if (phase != kProbeBound && a.entCnt) a.entCnt[q] = 0;
+        }
+        return;
+    }
+    float p[DP];
+#pragma unroll
+    for (int d = 0; d < DP; ++d) p[d] = a.qF[static_cast<size_t>(q) * DP + d];
+    const float margin = a.margin[q];
+    if (tid == 0) sTauUb = __float_as_uint(INFINITY);
+    __syncthreads();
+
+    const uint32_t M = static_cast<uint32_t>(
+        fmin(32.0, fmax(2.0, ceil(a.waveFactor * static_cast<double>(K)) + 1.0)));
+    uint32_t nList = 0;  // ranges in sBeg / sPre
+    auto itemOf = [&](uint32_t i) {  // row i of the ranges laid end to end
+        uint32_t lo = 0, hi = nList - 1;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1) >> 1;
+            if (sPre[mid] <= i) lo = mid; else hi = mid - 1;
+        }
+        return sBeg[lo] + (i - sPre[lo]);
+    };
+    // Leaves the 32 best of the items 0 .. total-1 in sMerge[0], ascending; keyOf(i) returns the
+    // item's order key and node, and may lower the bound `ub`.
+    auto rank = [&](uint32_t total, auto&& keyOf) {
+        WarpBest best;
+        for (uint32_t i0 = warp * 32; i0 < total; i0 += kProbeThreads) {
+            const uint32_t i = i0 + lane;
+            uint64_t key = ~0ull;
+            uint32_t ub = 0xffffffffu;
+            if (i < total) key = keyOf(i, ub);
+            ub = __reduce_min_sync(FULL, ub);
+            if (lane == 0 && ub != 0xffffffffu) atomicMin(&sTauUb, ub);
+            best.add(key, lane);
+        }
+        sMerge[warp][lane] = best.best;
+        __syncthreads();
+        if (warp == 0) {
+            for (int w = 1; w < kProbeWarps; ++w) best.merge(sMerge[w][lane], lane);
+            sMerge[0][lane] = best.best;
+        }
+        __syncthreads();
+    };
+    // Node j of mesh m: its centre's distance, less the subtree radius (the sphere's lower bound) when
+    // bySphere. A node with K points below it bounds the K-th distance by its far side.
+    auto nodeKey = [&](int m, uint32_t j, bool bySphere, uint32_t& ub) -> uint64_t {
+        const KnnSweepLevel& L = a.level[m];
+        const float d = sqrtf(rowDist2<DP>(p, L.x + static_cast<size_t>(j) * DP));
+        const float r = __ldg(L.rad + j);
+        if (__ldg(L.leaf + j) >= K) ub = __float_as_uint((d + r) * kRel + margin);
+        if (L.nodes[j].cnt == 0) return ~0ull;
+        return (static_cast<uint64_t>(floatKey(bySphere ? d - r : d)) << 32) | j;
+    };
+    // The ranges recs[] of the first `keep` nodes of sMerge[0] become the list; returns their rows.
+    auto expand = [&](const NodeRec* recs, uint32_t keep, int headerLevel) {
+        if (warp == 0) {
+            const uint64_t key = sMerge[0][lane];
+            const bool v = static_cast<uint32_t>(lane) < keep && key != ~0ull;
+            const NodeRec nr = v ? recs[static_cast<uint32_t>(key)] : NodeRec{0.0, 0u, 0u};
+            uint32_t inc = nr.cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += t;
+            }
+            sBeg[lane] = nr.cbeg;
+            sPre[lane] = inc - nr.cnt;
+            if (lane == 31) sPre[32] = inc;
+            const uint32_t n = __popc(__ballot_sync(FULL, v));
+            if (lane == 31) {
+                sSel[0] = n;
+                if (headerLevel > 0) {  // entries kept and their children
+                    atomicAdd(a.hdr + 2 * headerLevel, n);
+                    atomicAdd(a.hdr + 2 * headerLevel + 1, inc);
+                }
+            }
+        }
+        __syncthreads();
+        nList = sSel[0];
+        const uint32_t rows = sPre[32];
+        __syncthreads();
+        return rows;
+    };
+
+    uint32_t total = a.level[0].count;
+    if (phase != kProbeBound) {
+        for (int m = 0; m + 2 < H; ++m) {
+            rank(total, [&](uint32_t i, uint32_t& ub) { return nodeKey(m, m ? itemOf(i) : i, true, ub); });
+            total = expand(a.level[m].nodes, a.beam, m + 1);
+        }
+    }
+    if (phase == kProbeEntries) {
+        // Hand the clusters under the beam to the scorer.
+        __shared__ uint32_t sBase;
+        if (tid == 0) {
+            sBase = atomicAdd(a.hdr + 2 * (H - 1), total);
+            a.entOff[q] = sBase;
+            a.entCnt[q] = total;
+            if (static_cast<uint64_t>(sBase) + total > a.entCap) atomicOr(a.status, kStatusOverflowEntries);
+            a.tau[q] = static_cast<double>(__uint_as_float(sTauUb));
+        }
+        __syncthreads();
+        // Every slot the scorer reads (those below the capacity) is written, also when the entries
+        // outgrow the capacity and the batch will rerun.
+        const uint32_t base = sBase;
+        const uint32_t room = base < a.entCap ? min(total, a.entCap - base) : 0u;
+        for (uint32_t i = tid; i < room; i += kProbeThreads) {
+            const uint32_t j = H > 2 ? itemOf(i) : i;
+            a.entQ[base + i] = q;
+            a.entNode[base + i] = j;
+            for (int d = 0; d < a.D; ++d)
+                a.entX[static_cast<size_t>(base + i) * a.D + d] = a.nodeX[static_cast<size_t>(j) * a.D + d];
+        }
+        return;
+    }
+    uint32_t rows;
+    if (phase == kProbeBound) {
+        if (tid == 0) sTauUb = __float_as_uint(__double2float_ru(a.tau[q]));
+        __syncthreads();
+        // The M best-scored clusters (smaller = read earlier), filled up to 32 with the nearest centres
+        // of the others, so that a scorer that ranks badly cannot leave the bound loose; of their point
+        // groups the 32 whose boxes' centres lie nearest are read (all of them when K asks for more).
+        const uint32_t base = a.entOff[q];
+        const uint32_t n = static_cast<uint64_t>(base) + a.entCnt[q] <= a.entCap ? a.entCnt[q] : 0u;
+        rank(n, [&](uint32_t i, uint32_t&) -> uint64_t {
+            const uint32_t j = a.entNode[base + i];
+            if (a.level[H - 2].nodes[j].cnt == 0) return ~0ull;
+            return (static_cast<uint64_t>(floatKey(static_cast<float>(a.score[base + i]))) << 32) | j;
+        });
+        if (warp == 0) sScored[lane] = static_cast<uint32_t>(lane) < M ? sMerge[0][lane] : ~0ull;
+        __syncthreads();
+        rank(n, [&](uint32_t i, uint32_t& ub) -> uint64_t {
+            const uint32_t j = a.entNode[base + i];
+            const uint64_t key = nodeKey(H - 2, j, false, ub);
+            for (uint32_t t = 0; t < M; ++t)
+                if (sScored[t] != ~0ull && static_cast<uint32_t>(sScored[t]) == j) return ~0ull;
+            return key;
+        });
+        if (warp == 0) {
+            const uint64_t own = sScored[lane];
+            const uint32_t nS = __popc(__ballot_sync(FULL, own != ~0ull));
+            const uint64_t fill = sMerge[0][static_cast<uint32_t>(lane) >= nS ? lane - nS : 0];
+            __syncwarp();
+            sMerge[0][lane] = static_cast<uint32_t>(lane) < nS ? own : fill;
+        }
+        __syncthreads();
+        const uint64_t mine = sMerge[0][lane];
+        const uint32_t groups = expand(a.clusterGroups, 32, 0);
+        rank(groups, [&](uint32_t i, uint32_t&) -> uint64_t {
+            const uint32_t g = itemOf(i);
+            const float* b = a.groupBox + static_cast<size_t>(g) * 2 * DP;
+            float s = 0.f;
+#pragma unroll
+            for (int d = 0; d < DP; ++d) {
+                const float e = 0.5f * (__ldg(b + d) + __ldg(b + DP + d)) - p[d];
+                s = fmaf(e, e, s);
+            }
+            return (static_cast<uint64_t>(floatKey(s)) << 32) | g;
+        });
+        rows = expand(a.groupRec, 32, 0);
+        if (rows < 2 * K) {
+            if (warp == 0) sMerge[0][lane] = mine;
+            __syncthreads();
+            rows = expand(a.level[H - 2].nodes, 32, 0);
+        }
+    } else {
+        rank(total, [&](uint32_t i, uint32_t& ub) { return nodeKey(H - 2, H > 2 ? itemOf(i) : i, false, ub); });
+        if (tid == 0) atomicAdd(a.hdr + 2 * (H - 1), total);
+        // A wide read: twelve times the clusters the scored one takes (float tests of points that lie
+        // near the query anyway are cheap, and the bound they give is what the sweep costs by).
+        const uint32_t wide = static_cast<uint32_t>(
+            fmin(32.0, fmax(2.0, ceil(12.0 * a.waveFactor * static_cast<double>(K)) + 1.0)));
+        rows = expand(a.level[H - 2].nodes, wide, 0);
+    }
+    // The K-th smallest distance among the points read.
+    const uint32_t n = min(rows, kProbePoints);
+    if (tid == 0) {
+        atomicAdd(a.hdr + 2 * (H - 1) + 1, rows);
+        atomicAdd(a.hdr + 2 * H, n);
+        atomicAdd(a.work, static_cast<unsigned long long>(n));
+    }
+    for (uint32_t i = tid; i < n; i += kProbeThreads)
+        sKeys[i] = rowDist2<DP>(p, a.pointsF + static_cast<size_t>(itemOf(i)) * DP);
+    if (tid == 0) {
+        sSel[0] = 0;  // prefix chosen so far
+        sSel[1] = K;  // rank within it
+    }
+    __syncthreads();
+    if (n >= K) {
+        // Radix selection over the keys' bits (non-negative floats order like integers).
+        for (int shift = 24; shift >= 0; shift -= 8) {
+            sHist[tid] = 0;
+            __syncthreads();
+            const uint32_t prefix = sSel[0], mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
+            for (uint32_t i = tid; i < n; i += kProbeThreads) {
+                const uint32_t key = __float_as_uint(sKeys[i]);
+                if ((key & mask) == prefix) atomicAdd(&sHist[(key >> shift) & 255u], 1u);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                uint32_t c[8], sum = 0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    c[i] = sHist[lane * 8 + i];
+                    sum += c[i];
+                }
+                uint32_t inc = sum;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                    if (lane >= o) inc += t;
+                }
+                const uint32_t need = sSel[1];
+                __syncwarp();
+                uint32_t before = inc - sum;
+                if (before < need && need <= inc) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        if (before < need && need <= before + c[i]) {
+                            sSel[0] = prefix | (static_cast<uint32_t>(lane * 8 + i) << shift);
+                            sSel[1] = need - before;
+                        }
+                        before += c[i];
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+    if (tid == 0) {
+        double tau = static_cast<double>(__uint_as_float(sTauUb));
+        if (n >= K)
+            tau = fmin(tau, sqrt(static_cast<double>(__uint_as_float(sSel[0]))) * static_cast<double>(kRel) +
+                                static_cast<double>(margin));
+        const double t = (tau + static_cast<double>(margin)) * (1.0 + 1e-7);
+        a.tau[q] = tau;
+        a.tauF[q] = __double2float_ru(t);
+        const double s = t * static_cast<double>(kRel);
+        a.thrF[q] = __double2float_ru(s * s);
+    }
+}
+
+// ---- dense bound ----------------------------------------------------------------------------------
+constexpr int kBoundThreads = 256;
+constexpr int kBoundWords = 8;  // query words of one CTA
+
+// One thread per cluster, its centre in registers; the block's queries (negated) come from shared
+// memory as broadcasts. Bound by the float pipe: D additions and multiply-adds per pair, packed two
+// to an instruction. 4,096 queries x 100,000 clusters, D = 8: 367 us (1.1e12 pairs/s); the walk's
+// bound levels, filters and transposes for the same queries took 3.4 ms.
+template <int DP>
+__global__ void __launch_bounds__(kBoundThreads) knnBoundBitsKernel(KnnSweepArgs a) {
+    __shared__ __align__(16) float sQ[kBoundWords * 32][DP];
+    __shared__ float sTau[kBoundWords * 32];
+    if (*a.status) return;
+    const KnnSweepLevel& L = a.level[a.height - 2];
+    const uint32_t w0 = blockIdx.y * kBoundWords, w1 = min(a.words, w0 + kBoundWords);
+    const uint32_t nQ = (w1 - w0) * 32;
+    for (uint32_t i = threadIdx.x; i < nQ; i += kBoundThreads) {
+        const uint32_t q = a.qBegin + w0 * 32 + i;
+        const bool v = q < a.qEnd;
+#pragma unroll
+        for (int d = 0; d < DP; ++d)
+            sQ[i][d] = v ? -a.qF[static_cast<size_t>(q) * DP + d] : -static_cast<float>(kSweepMaxAbs);
+        sTau[i] = v ? a.tauF[q] : 0.f;
+    }
+    __syncthreads();
+    const uint32_t c = blockIdx.x * kBoundThreads + threadIdx.x;
+    const bool valid = c < L.count && L.nodes[c].cnt > 0;
+    float2 x[DP / 2];
+#pragma unroll
+    for (int d = 0; d < DP / 2; ++d)
+        x[d] = valid ? __ldg(reinterpret_cast<const float2*>(L.x + static_cast<size_t>(c) * DP) + d) : make_float2(0.f, 0.f);
+    const float r = valid ? __ldg(L.rad + c) : -3e38f;
+    const uint32_t left = a.qEnd - a.qBegin > w0 * 32 ? a.qEnd - a.qBegin - w0 * 32 : 0u;  // queries of this CTA's words
+    uint32_t word[kBoundWords], any = 0;
+#pragma unroll
+    for (int w = 0; w < kBoundWords; ++w) {
+        word[w] = 0;
+        if (static_cast<uint32_t>(w) * 32 >= left) continue;
+        const uint32_t n = min(32u, left - w * 32);
+#pragma unroll 4
+        for (uint32_t j = 0; j < n; ++j) {
+            const uint32_t i = w * 32 + j;
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int d = 0; d < DP / 2; d += 2) {
+                const float4 nq = *reinterpret_cast<const float4*>(&sQ[i][2 * d]);
+                const float2 e = __fadd2_rn(x[d], make_float2(nq.x, nq.y));
+                const float2 f = __fadd2_rn(x[d + 1], make_float2(nq.z, nq.w));
+                s = __ffma2_rn(e, e, s);
+                s = __ffma2_rn(f, f, s);
+            }
+            const float t = (sTau[i] + r) * kRel;
+            if (s.x + s.y <= t * t) word[w] |= 1u << j;
+        }
+        if (!valid) word[w] = 0;
+        any |= word[w];
+    }
+    if (c < L.count) {
+        uint32_t* out = a.bits + static_cast<size_t>(c) * a.words + w0;
+        if (a.words == 1) {
+            out[0] = word[0];
+        } else {  // rows of a multiple of four words
+            *reinterpret_cast<uint4*>(out) = make_uint4(word[0], word[1], word[2], word[3]);
+            if (w0 + 4 < a.words) *reinterpret_cast<uint4*>(out + 4) = make_uint4(word[4], word[5], word[6], word[7]);
+        }
+    }
+    if (gridDim.y == 1) {
+        const uint32_t b = __ballot_sync(FULL, any != 0);
+        if (b) {
+            const int lane = threadIdx.x & 31;
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(a.liveCnt, __popc(b));
+            base = __shfl_sync(FULL, base, 0);
+            if (any) a.live[base + __popc(b & ((1u << lane) - 1u))] = c;
+        }
+    }
+}
+
+// ---- sweep ----------------------------------------------------------------------------------------
+constexpr int kSweepThreads = 128;
+constexpr int kSweepWarps = kSweepThreads / 32;
+constexpr uint32_t kSweepList = 1024 + 32;
+constexpr uint32_t kSweepGroups = 8;  // group boxes staged at once
+
+// One warp per cluster. Lanes are queries while boxes are tested and points while distances are: a
+// group's points stay in registers and every query whose box test passed is broadcast from shared
+// memory, so no lane idles for another query's sake. Bound by the float pipe and the latency of a
+// cluster's first loads. 84M (query, point) tests of 4,096 queries, D = 8: 422 us (the walk's point
+// passes: 2.9 ms for 187M); 811M of 1,000 queries, D = 16: 2.6 ms (26 ms for 1,760M).
+template <int DP>
+__global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(KnnSweepArgs a) {
+    __shared__ uint32_t sList[kSweepWarps][kSweepList];
+    __shared__ __align__(16) float sP[kSweepWarps][32][DP];
+    __shared__ float sThr[kSweepWarps][32];
+    __shared__ uint32_t sId[kSweepWarps][32];
+    __shared__ __align__(16) float sBox[kSweepWarps][kSweepGroups][2 * DP];
+    if (*a.status) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const KnnSweepLevel& L = a.level[a.height - 2];
+    const bool listed = a.qEnd - a.qBegin <= kBoundWords * 32;
+    const uint32_t nClusters = listed ? *a.liveCnt : L.count;
+    unsigned long long tested = 0;
+    uint32_t kept = 0;              // this lane's candidates
+    uint32_t staged = 0xffffffffu;  // first group whose box is in sBox
+
+    // A batch of n <= 32 queries of the list against the cluster's groups.
+    auto batch = [&](const NodeRec& cg, uint32_t from, uint32_t n) {
+        const bool v = static_cast<uint32_t>(lane) < n;
+        const uint32_t q = v ? sList[w][from + lane] : 0u;
+        float p[DP];
+#pragma unroll
+        for (int d = 0; d < DP; d += 4) {
+            const float4 t = v ? __ldg(reinterpret_cast<const float4*>(a.qF + static_cast<size_t>(q) * DP + d))
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+            p[d] = t.x;
+            p[d + 1] = t.y;
+            p[d + 2] = t.z;
+            p[d + 3] = t.w;
+        }
+        const float thr = v ? a.thrF[q] : -1.f;
+        __syncwarp();
+#pragma unroll
+        for (int d = 0; d < DP; d += 4)
+            *reinterpret_cast<float4*>(&sP[w][lane][d]) = make_float4(p[d], p[d + 1], p[d + 2], p[d + 3]);
+        sThr[w][lane] = thr;
+        sId[w][lane] = q;
+        for (uint32_t g0 = 0; g0 < cg.cnt; g0 += kSweepGroups) {
+            const uint32_t ng = min(kSweepGroups, cg.cnt - g0);
+            __syncwarp();
+            if (staged != cg.cbeg + g0) {
+                staged = cg.cbeg + g0;
+                const float4* src = reinterpret_cast<const float4*>(a.groupBox + static_cast<size_t>(staged) * 2 * DP);
+                for (uint32_t i = lane; i < ng * (2 * DP / 4); i += 32)
+                    reinterpret_cast<float4*>(&sBox[w][0][0])[i] = __ldg(src + i);
+            }
+            __syncwarp();
+            for (uint32_t g = 0; g < ng; ++g) {
+                const float* b = sBox[w][g];
+                float gap = 0.f;
+#pragma unroll
+                for (int d = 0; d < DP; d += 4) {
+                    const float4 lo = *reinterpret_cast<const float4*>(b + d);
+                    const float4 hi = *reinterpret_cast<const float4*>(b + DP + d);
+                    const float e0 = fmaxf(fmaxf(lo.x - p[d], p[d] - hi.x), 0.f);
+                    const float e1 = fmaxf(fmaxf(lo.y - p[d + 1], p[d + 1] - hi.y), 0.f);
+                    const float e2 = fmaxf(fmaxf(lo.z - p[d + 2], p[d + 2] - hi.z), 0.f);
+                    const float e3 = fmaxf(fmaxf(lo.w - p[d + 3], p[d + 3] - hi.w), 0.f);
+                    gap = fmaf(e0, e0, gap);
+                    gap = fmaf(e1, e1, gap);
+                    gap = fmaf(e2, e2, gap);
+                    gap = fmaf(e3, e3, gap);
+                }
+                uint32_t mask = __ballot_sync(FULL, gap <= thr);
+                if (mask == 0) continue;
+                const NodeRec gr = a.groupRec[cg.cbeg + g0 + g];
+                const bool pv = static_cast<uint32_t>(lane) < gr.cnt;
+                const uint32_t row = gr.cbeg + (pv ? lane : 0u);
+                tested += static_cast<unsigned long long>(__popc(mask)) * gr.cnt;
+                float2 x[DP / 2];
+#pragma unroll
+                for (int d = 0; d < DP / 2; d += 2) {
+                    const float4 t = __ldg(reinterpret_cast<const float4*>(a.pointsF + static_cast<size_t>(row) * DP) + d / 2);
+                    x[d] = make_float2(-t.x, -t.y);
+                    x[d + 1] = make_float2(-t.z, -t.w);
+                }
+                while (mask) {
+                    const int s = __ffs(mask) - 1;
+                    mask &= mask - 1;
+                    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int d = 0; d < DP / 2; d += 2) {
+                        const float4 t = *reinterpret_cast<const float4*>(&sP[w][s][2 * d]);
+                        const float2 e = __fadd2_rn(x[d], make_float2(t.x, t.y));
+                        const float2 f = __fadd2_rn(x[d + 1], make_float2(t.z, t.w));
+                        acc = __ffma2_rn(e, e, acc);
+                        acc = __ffma2_rn(f, f, acc);
+                    }
+                    const bool hit = pv && acc.x + acc.y <= sThr[w][s];
+                    if (__ballot_sync(FULL, hit) == 0) continue;
+                    if (hit) {
+                        const uint32_t qq = sId[w][s];
+                        const double* pd = a.points + static_cast<size_t>(qq) * a.D;
+                        const double d2 = pointDist2(pd, a.pointsD + static_cast<size_t>(row) * a.D, a.D);
+                        const double tau = a.tau[qq];
+                        if (d2 <= tau * tau * (1.0 + 1e-9)) {
+                            const uint32_t slot = atomicAdd(&a.candCnt[qq], 1u);
+                            const uint64_t pos = a.candOff[qq] + slot;
+                            if (pos < a.candOff[qq + 1] && pos < a.candCap) {
+                                a.candId[pos] = a.map[__ldg(a.perm + row)];
+                                a.candD2[pos] = d2;
+                                ++kept;
+                            } else {
+                                atomicOr(a.status, kStatusOverflowEntries);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    };
+
+    // Clusters per ticket: several where there are many, so the ticket's atomic does not bound the sweep.
+    const uint32_t chunk = max(1u, min(8u, nClusters / (gridDim.x * kSweepWarps * 8u)));
+    uint32_t k = 0, kEnd = 0;
+    while (true) {
+        if (k == kEnd) {
+            if (lane == 0) k = atomicAdd(a.ticket, chunk);
+            k = __shfl_sync(FULL, k, 0);
+            if (k >= nClusters) break;
+            kEnd = min(nClusters, k + chunk);
+        }
+        const uint32_t c = listed ? a.live[k] : k;
+        ++k;
+        const NodeRec cg = a.clusterGroups[c];
+        const uint32_t* row = a.bits + static_cast<size_t>(c) * a.words;
+        uint32_t n = 0;
+        for (uint32_t w0 = 0; w0 < a.words; w0 += 32) {
+            uint32_t word = (w0 + lane < a.words) ? row[w0 + lane] : 0u;
+            uint32_t inc = __popc(word);
+            const uint32_t own = inc;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += t;
+            }
+            const uint32_t add = __shfl_sync(FULL, inc, 31);
+            if (add == 0) continue;
+            uint32_t at = n + inc - own;
+            const uint32_t q0 = a.qBegin + (w0 + lane) * 32;
+            while (word) {
+                sList[w][at++] = q0 + __ffs(word) - 1;
+                word &= word - 1;
+            }
+            __syncwarp();
+            n += add;
+            uint32_t from = 0;
+            const bool last = w0 + 32 >= a.words;
+            for (; from + 32 <= n; from += 32) batch(cg, from, 32);
+            if (last) break;
+            // The rest waits for the next words.
+            const uint32_t rest = n - from;
+            const uint32_t keep = static_cast<uint32_t>(lane) < rest ? sList[w][from + lane] : 0u;
+            __syncwarp();
+            if (static_cast<uint32_t>(lane) < rest) sList[w][lane] = keep;
+            __syncwarp();
+            n = rest;
+        }
+        const uint32_t full = n / 32 * 32;
+        if (n > full) batch(cg, full, n - full);
+        __syncwarp();
+    }
+    if (lane == 0 && tested) atomicAdd(a.work + 1, tested);
+    kept = __reduce_add_sync(FULL, kept);
+    if (lane == 0 && kept) atomicAdd(a.hdr + 2 * (a.height + 1), kept);
+}
+
+int residentBlocks(const void* kern, int threads) {
+    int dev = 0, sms = 0, perSm = 0;
+    TBLAEQ_CUDA(cudaGetDevice(&dev));
+    TBLAEQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    TBLAEQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kern, threads, 0));
+    return std::max(1, sms * std::max(1, perSm));
+}
+
+// Calls f with the padded dimension as a compile-time constant.
+template <class F>
+void withPadded(int D, F&& f) {
+    switch (paddedDims(static_cast<uint64_t>(D))) {
+        case 4: return f(std::integral_constant<int, 4>{});
+        case 8: return f(std::integral_constant<int, 8>{});
+        case 12: return f(std::integral_constant<int, 12>{});
+        case 16: return f(std::integral_constant<int, 16>{});
+        case 20: return f(std::integral_constant<int, 20>{});
+        case 24: return f(std::integral_constant<int, 24>{});
+        case 28: return f(std::integral_constant<int, 28>{});
+        case 32: return f(std::integral_constant<int, 32>{});
+        default: throw std::invalid_argument("KNN sweep: D must be in [1, 32]");
+    }
+}
+
+}  // namespace
+
+void launchKnnSweepPrepare(const KnnSweepArgs& a, cudaStream_t s) {
+    const unsigned blocks = std::min<unsigned>(148u, (a.nq + 1023u) / 1024u);
+    sweepPrepareKernel<<<std::max(1u, blocks), 1024, 0, s>>>(a, paddedDims(static_cast<uint64_t>(a.D)));
+    TBLAEQ_LAUNCHED();
+}
+
+void launchKnnProbe(const KnnSweepArgs& a, KnnProbePhase phase, cudaStream_t s) {
+    if (a.nq == 0) return;
+    withPadded(a.D, [&](auto dp) {
+        knnProbeKernel<decltype(dp)::value><<<a.nq, kProbeThreads, 0, s>>>(a, static_cast<int>(phase));
+        TBLAEQ_LAUNCHED();
+    });
+}
+
+void launchKnnSweepBound(const KnnSweepArgs& a, cudaStream_t s) {
+    const dim3 grid((a.level[a.height - 2].count + kBoundThreads - 1) / kBoundThreads,
+                    (a.words + kBoundWords - 1) / kBoundWords);
+    withPadded(a.D, [&](auto dp) {
+        knnBoundBitsKernel<decltype(dp)::value><<<grid, kBoundThreads, 0, s>>>(a);
+        TBLAEQ_LAUNCHED();
+    });
+}
+
+void launchKnnSweepPoints(const KnnSweepArgs& a, cudaStream_t s) {
+    withPadded(a.D, [&](auto dp) {
+        constexpr int DP = decltype(dp)::value;
+        static const int grid = residentBlocks(reinterpret_cast<const void*>(knnSweepKernel<DP>), kSweepThreads);
+        knnSweepKernel<DP><<<grid, kSweepThreads, 0, s>>>(a);
+        TBLAEQ_LAUNCHED();
+    });
+}
+
+}  // namespace tblaeq

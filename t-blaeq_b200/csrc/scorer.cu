@@ -114,6 +114,11 @@ std::vector<float> trainScorer(Runtime& rt, const double* hostPoints, uint32_t n
     eng.setScorer(nullptr, nullptr);  // traces come from the lower-bound ranking
     const bool wasTwoWave = eng.twoWave();
     eng.setTwoWave(true);
+    eng.setKnnTrace(true);
+    struct TraceOff {
+        BatchEngine& e;
+        ~TraceOff() { e.setKnnTrace(false); }
+    } traceOff{eng};
     std::mt19937_64 rng(cfg.seed);
     std::vector<float> hostX, hostY;
     uint64_t positives = 0;
