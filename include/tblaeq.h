@@ -237,6 +237,10 @@ int tblaeq_group_counts(tblaeq_handle* h, uint64_t* out3);
 /* ---- Launch shapes and the tuning cache (no counterpart in the reference, whose kernel shapes are
  * compile-time constants: kCompact* in src/core/strategies/L0Strategy.cu:18-21, UNROLL_FACTOR in
  * src/Kernel/SpMSpV.cuh:24) ----
+ * Exact range batches whose shapes are all at their defaults (variant 0, 100%) run as one sweep over the
+ * hierarchy instead of one launch per mesh (same results in the same order, same per-level counts); any
+ * other shape asks for the level-synchronous launches. tblaeq_autotune leaves the defaults where the
+ * sweep is the faster.
  * A launch shape per expand launch (one per mesh, `height` of them): the kernel variant (0 = direct,
  * 1 = staged) and the persistent grid as a percentage (1..100) of the kernel's full occupancy.
  * tblaeq_autotune searches variant x grid {100, 75, 50, 25}% per level on the live batch. */

@@ -112,6 +112,54 @@ DerivedArrays computeDerived(const HostIndex& idx) {
 
     out.nodeX.resize(H - 1);
     for (uint64_t m = 0; m + 1 < H; ++m) out.nodeX[m] = dec[m];
+    out.parent.assign(parent.begin(), parent.begin() + static_cast<ptrdiff_t>(H - 1));
+    // Units of the range sweep: every last upper node's clusters, nodes in depth-first order, split
+    // evenly into at most kRangeUnit.
+    {
+        auto split = [&](uint32_t node, uint32_t first, uint32_t n) {
+            const uint32_t parts = (n + kRangeUnit - 1) / kRangeUnit;
+            for (uint32_t i = 0; i < parts; ++i) {
+                const uint32_t a = static_cast<uint32_t>(static_cast<uint64_t>(n) * i / parts);
+                const uint32_t b = static_cast<uint32_t>(static_cast<uint64_t>(n) * (i + 1) / parts);
+                out.units.push_back(RangeUnit{node, first + a, b - a, 0});
+            }
+        };
+        if (H == 2) {
+            split(0, 0, static_cast<uint32_t>(idx.meshCount(0)));
+        } else if (H > 2) {
+            std::vector<uint32_t> order(idx.meshCount(0)), next;
+            for (size_t i = 0; i < order.size(); ++i) order[i] = static_cast<uint32_t>(i);
+            for (uint64_t m = 0; m + 3 < H; ++m) {
+                next.clear();
+                for (uint32_t s : order)
+                    for (uint32_t j = 0; j < out.ccnt[m][s]; ++j) next.push_back(out.cbeg[m][s] + j);
+                order.swap(next);
+            }
+            for (uint32_t s : order) split(s, out.cbeg[H - 3][s], out.ccnt[H - 3][s]);
+            // Upper units: runs of siblings of mesh H-3, parents in position order.
+            auto upper = [&](uint32_t node, uint32_t first, uint32_t n) {
+                for (uint32_t i = 0; i < n; i += kRangeUpperUnit) {
+                    uint32_t flags = 0;
+                    if (i == 0 && H > 3) {  // first below the parent, and below those whose first child it is
+                        uint32_t k = node;
+                        for (uint64_t t = H - 4;; --t) {
+                            flags |= 1u << t;
+                            if (t == 0) break;
+                            const uint32_t up = parent[t][k];
+                            if (out.cbeg[t - 1][up] != k) break;
+                            k = up;
+                        }
+                    }
+                    out.upperUnits.push_back(RangeUnit{node, first + i, std::min(kRangeUpperUnit, n - i), flags});
+                }
+            };
+            if (H == 3) {
+                upper(0, 0, static_cast<uint32_t>(idx.meshCount(0)));
+            } else {
+                for (uint32_t s = 0; s < out.cbeg[H - 4].size(); ++s) upper(s, out.cbeg[H - 4][s], out.ccnt[H - 4][s]);
+            }
+        }
+    }
     // Rows of the float copies and boxes are padded to 16 bytes with zeros.
     const uint64_t DP = paddedDims(D);
     for (const auto& mesh : dec)
@@ -329,7 +377,7 @@ DerivedArrays computeDerived(const HostIndex& idx) {
             out.leaf[m][s] = static_cast<uint32_t>(C[m][s]);
         }
     }
-    if (!out.pointPerm.empty()) {
+    if (!out.pointPerm.empty() && floatPointsSupported(D)) {
         // In point-group order, like the float copy (the KNN point kernel walks the groups).
         const std::vector<double>& pts = dec[H - 1];
         out.pointsD.resize(pts.size());
@@ -434,7 +482,44 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
     di->nodeX.resize(idx.height - 1);
     di->nodeXF.resize(idx.height - 1);
     di->radF.resize(idx.height - 1);
+    di->aabbP.resize(idx.height - 1);
     di->maxAbs = der.maxAbs;
+    di->parent.resize(idx.height - 1);
+    for (uint64_t m = 1; m + 1 < idx.height; ++m) di->parent[m] = upload(der.parent[m], s);
+    di->units = upload(der.units, s);
+    di->unitCount = static_cast<uint32_t>(der.units.size());
+    di->upperUnits = upload(der.upperUnits, s);
+    if (idx.D <= 32) {
+        const uint64_t D = idx.D, DP = paddedDims(D), n = idx.meshCount(idx.height - 2), n0 = idx.meshCount(0);
+        for (uint64_t d = 0; d < D; ++d) {
+            double lo = std::numeric_limits<double>::infinity(), hi = -lo;
+            for (uint64_t i = 0; i < n0; ++i) {
+                if (der.ccnt[0][i] == 0) continue;
+                lo = std::min(lo, static_cast<double>(der.aabb[0][i * 2 * D + d]));
+                hi = std::max(hi, static_cast<double>(der.aabb[0][i * 2 * D + D + d]));
+            }
+            const double ext = hi - lo;
+            di->gridMin[d] = ext > 0.0 && std::isfinite(ext) ? lo : 0.0;
+            di->gridScale[d] = ext > 0.0 && std::isfinite(ext) ? kRangeGrid / ext : 0.0;
+        }
+        std::vector<uint32_t> grid(n * DP, 0u);
+        for (uint64_t i = 0; i < n; ++i) {
+            for (uint64_t d = 0; d < DP; ++d) {
+                uint32_t l = 0, h = 0;
+                if (d < D) {
+                    const float* b = &der.aabb[idx.height - 2][i * 2 * D];
+                    l = rangeGridLower(b[d], di->gridMin[d], di->gridScale[d]);
+                    h = rangeGridUpper(b[D + d], di->gridMin[d], di->gridScale[d]);
+                }
+                grid[i * DP + d / 2] |= l << (16 * (d & 1));
+                grid[i * DP + DP / 2 + d / 2] |= (h | 0x8000u) << (16 * (d & 1));
+            }
+        }
+        di->clusterGrid = upload(grid, s);
+        TBLAEQ_CUDA(cudaStreamSynchronize(s));
+    }
+    di->upperUnitCount = static_cast<uint32_t>(der.upperUnits.size());
+    for (uint32_t n : der.ccnt[idx.height - 2]) di->maxCluster = std::max(di->maxCluster, n);
     for (uint64_t m = 0; m + 1 < idx.height; ++m) {
         const size_t n = der.cbeg[m].size();
         std::vector<NodeRec> ref(n), sub(n);
@@ -458,6 +543,16 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
         }
         di->nodeXF[m] = upload(xf, s);
         di->radF[m] = upload(rf, s);
+        std::vector<float> bp;
+        if (DP != idx.D) {
+            bp.assign(n * 2 * DP, 0.f);
+            for (size_t i = 0; i < n; ++i)
+                for (uint64_t d = 0; d < idx.D; ++d) {
+                    bp[i * 2 * DP + d] = der.aabb[m][i * 2 * idx.D + d];
+                    bp[i * 2 * DP + DP + d] = der.aabb[m][i * 2 * idx.D + idx.D + d];
+                }
+            di->aabbP[m] = upload(bp, s);
+        }
         TBLAEQ_CUDA(cudaStreamSynchronize(s));
     }
     if (!der.pointsD.empty() && idx.intervals > 0 && res(idx.intervals - 1) == kResident) {
@@ -496,9 +591,10 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
 
 size_t DeviceIndex::deviceBytes() const {
     size_t t = coarseVals.bytes() + coarseIds.bytes();
-    for (auto* v : {&pvals, &nodeRef, &nodeSub, &leaf, &aabb, &nodeX, &nodeXF, &radF, &nodeOrig, &maps})
+    for (auto* v : {&pvals, &nodeRef, &nodeSub, &leaf, &aabb, &nodeX, &nodeXF, &radF, &aabbP, &parent, &nodeOrig, &maps})
         for (auto& m : *v) t += m.bytes();
-    return t + pointsD.bytes() + pointsF.bytes() + pointPerm.bytes() + groupRec.bytes() + groupBox.bytes() + clusterGroups.bytes();
+    return t + pointsD.bytes() + pointsF.bytes() + pointPerm.bytes() + groupRec.bytes() + groupBox.bytes() + clusterGroups.bytes() +
+           units.bytes() + upperUnits.bytes() + clusterGrid.bytes();
 }
 
 }  // namespace tblaeq

@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "index.hpp"
+#include "rangesweep.cuh"
 #include "traverse.cuh"
 
 namespace tblaeq {
@@ -94,9 +95,13 @@ struct DerivedArrays {
     std::vector<float> groupBox;         // per group: lo[D] hi[D] of its points, rounded outward
     std::vector<uint32_t> clusterGroup;  // per finest cluster (mesh H-2 position): first group; one more at the end
     // Decoded finest points (y = P[j] * x_parent, one rounded multiply per dimension), in
-    // point-group order when the groups exist (pointPerm maps back to rows), else in row order.
+    // point-group order where floatPointsSupported(D) (pointPerm maps back to rows), else in row order.
     std::vector<double> pointsD;
     double maxAbs = 0.0;                 // largest |coordinate| of any mesh
+    // Parent position of every node (mesh m: position in mesh m-1; mesh 0 empty), meshes 0 .. height-2.
+    std::vector<std::vector<uint32_t>> parent;
+    std::vector<RangeUnit> units;        // the finest clusters in traversal order, see rangesweep.cuh
+    std::vector<RangeUnit> upperUnits;   // the nodes of the mesh above them
 };
 
 // Most points of one point group.
@@ -153,6 +158,13 @@ struct DeviceIndex {
     std::vector<DeviceMem> nodeX;            // mesh m < height-1: decoded coordinates (D doubles per node)
     std::vector<DeviceMem> nodeXF, radF;     // mesh m < height-1: the same as padded floats; subtree radius, rounded up
     double maxAbs = 0.0;                     // largest |coordinate| of any mesh
+    std::vector<DeviceMem> parent;           // mesh 1 <= m < height-1: position of each node's parent (uint32)
+    DeviceMem units;                         // RangeUnit: the finest clusters in traversal order
+    DeviceMem upperUnits;                    // RangeUnit: the nodes of the mesh above them
+    uint32_t unitCount = 0, upperUnitCount = 0;
+    uint32_t maxCluster = 0;                 // points of the largest finest cluster
+    DeviceMem clusterGrid;                   // the finest clusters' boxes on the grid of the data's extent (rangesweep.cu)
+    double gridMin[32] = {}, gridScale[32] = {};
     // Finest exact range level, when the last interval's rows are device-resident (else empty): the
     // points as floats in point-group order (DerivedArrays::pointsF), that order's row map, every
     // group's record {0, first row, rows} and box, and every finest cluster's record
@@ -166,6 +178,9 @@ struct DeviceIndex {
     DeviceMem coarseIds;                     // uint64
     std::vector<DeviceMem> nodeOrig;         // interval l, NodeRec by original column id
     std::vector<DeviceMem> maps;             // mesh m >= 1 (uint64); maps[0] empty
+
+    std::vector<DeviceMem> aabbP;            // aabb with rows padded to paddedDims(D), where D is not a multiple of 4
+    const float* aabbPadded(uint64_t m) const { return aabbP[m].bytes() ? aabbP[m].as<float>() : aabb[m].as<float>(); }
 
     size_t deviceBytes() const;
 };

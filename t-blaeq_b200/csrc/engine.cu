@@ -1,11 +1,13 @@
 // Batched traversal engine (range queries; see engine.hpp).
 #include "engine.hpp"
 
+#include <cmath>
 #include <exception>
 #include <limits>
 
 #include "knn.cuh"
 #include "knnsweep.cuh"
+#include "rangesweep.cuh"
 
 #include <algorithm>
 
@@ -38,8 +40,10 @@ void BatchEngine::resetWorkspace() noexcept {
                          &cmpKids_, &cmpEntryOff_, &cmpKidOff_, &offsets_, &boxF_, &tau_, &candOff_, &knnCount_,
                          &knnOff_, &knnIds_, &knnD2_, &lbE_, &scoreE_, &sel_, &offF_, &waveM_, &selCount_, &selOff_,
                          &selIds_, &selD2_, &candOffB_, &candOffS_, &resIdsB_, &resQB_, &resDistB_, &swQuery_, &swBits_,
-                         &swLive_, &swCand_, &swEnt_})
+                         &swLive_, &swCand_, &swEnt_, &rsBits_, &rsBoxF_, &rsRaw_, &rsSegs_})
         m->release();
+    rsRawCap_ = 0;
+    rsSegFactor_ = 1;
     swQcap_ = 0;
     swLast_ = false;
     swCandCap_ = swEntCap_ = 0;
@@ -89,7 +93,28 @@ std::vector<float> BatchEngine::autotuneRange(const double* dBoxes, uint32_t nq,
     const int H = static_cast<int>(di_.height);
     const bool wasTiming = timing_;
     setTiming(true);
-    runRange(dBoxes, nq, mode, flags & ~kUseGraph);  // sizes the workspace
+    setLaunchShapes(std::vector<int>(H, kVariantDirect), std::vector<int>(H, 100));
+    // The sweep (all launch shapes at their defaults) against the best level-synchronous launches.
+    runRange(dBoxes, nq, mode, flags & ~kUseGraph);
+    float sweepMs = std::numeric_limits<float>::infinity();
+    if (lastSweep_) {
+        std::vector<float> samples;
+        for (int r = 0; r < std::max(1, reps); ++r) {
+            enqueueRange(dBoxes, nq, mode, flags & ~kUseGraph);
+            if (status() != 0) throw CudaError(cudaErrorLaunchFailure, "autotune batch reported a device status");
+            float t = 0.f;
+            for (float x : stageTimes()) t += x;
+            samples.push_back(t);
+        }
+        std::sort(samples.begin(), samples.end());
+        sweepMs = samples[samples.size() / 2];
+    }
+    struct SweepOff {
+        bool& off;
+        ~SweepOff() { off = false; }
+    } sweepOff{rsOff_};
+    rsOff_ = true;
+    runRange(dBoxes, nq, mode, flags & ~kUseGraph);  // sizes the level-synchronous workspace
     struct Shape {
         int variant, grid;
     };
@@ -126,7 +151,16 @@ std::vector<float> BatchEngine::autotuneRange(const double* dBoxes, uint32_t nq,
         bestG[m] = candidates[bi].grid;
         bestT[m] = med[bi][m];
     }
+    float sum = 0.f;
+    for (float t : bestT) sum += t;
+    if (sweepMs <= sum) {
+        best.assign(H, kVariantDirect);
+        bestG.assign(H, 100);
+        bestT.assign(H, 0.f);
+        bestT[H - 1] = sweepMs;  // one launch sequence, not a time per level
+    }
     setLaunchShapes(best, bestG);
+    dropGraph();
     setTiming(wasTiming);
     return bestT;
 }
@@ -276,12 +310,14 @@ void BatchEngine::reserve(const EngineCaps& want, uint32_t nq, unsigned flags) {
         offDesc_ = off;
         off = align256(off + (H + 1) * tileCap_ * 8);
         offTickets_ = off;
-        off = align256(off + (H + 1) * 4);
+        off = align256(off + (H + 2) * 4);
         offStatus_ = off;
         off = align256(off + 4);
         offHdr_ = off;
         off = align256(off + (H + 4) * 2 * 4);  // levels 0..H-1, results, wave 2, compaction, point groups
         offQcount_ = off;
+        off = align256(off + static_cast<size_t>(qcap_) * 4);
+        offQsegs_ = off;
         off = align256(off + static_cast<size_t>(qcap_) * 4);
         offLevels_ = off;
         off = align256(off + static_cast<size_t>(di_.intervals) * qcap_ * 4);
@@ -481,9 +517,119 @@ void BatchEngine::enqueueNodeMajorLevel(int m, int buf, const double* dBoxes, ui
     launchFrontierHeader(n.counter, hdrPtr(m + 1), n.out.cap, n.out.tileCap, status, stream_);
 }
 
+bool BatchEngine::useRangeSweep(uint32_t nq, int mode, unsigned flags) const {
+    // Per-level counts per query, chosen launch shapes and the tests switched off all ask for the
+    // level-synchronous launches, and so does a streamed last interval (no decoded points on the device).
+    if (mode != kModeExact || (flags & kWantLevels) || nq == 0 || rsOff_ || rsSkip_ || !floatPoints_ || !pointGroups_ ||
+        lookbackTestHookSet() || di_.height < 2 || di_.height > kRangeMaxHeight || !di_.pointsF.bytes() ||
+        !di_.pointsD.bytes() || di_.unitCount == 0 ||
+        (!floatPointsSupported(di_.D) && di_.maxCluster > kRangeRowsCluster))
+        return false;
+    for (size_t m = 0; m < variants_.size(); ++m)
+        if (variants_[m] != kVariantDirect || grids_[m] != 100) return false;
+    const uint64_t upper = di_.height > 2 ? di_.meshCount[di_.height - 3] : 1;
+    return rangeSweepBitBytes(upper, nq) <= (1ull << 30) && nq <= (1u << 21);  // grid rows of 32 queries
+}
+
+// Segments a query may have: 262,144 over the batch at first, at most what the gather can order.
+uint32_t BatchEngine::rangeSweepSlots(uint32_t nq) const {
+    const uint64_t each = std::max<uint64_t>(64, 262144 / nq) * rsSegFactor_;
+    return static_cast<uint32_t>(std::min<uint64_t>(kRangeSegments, each));
+}
+
+void BatchEngine::reserveRangeSweep(uint32_t nq) {
+    const uint64_t DP = paddedDims(di_.D), upper = di_.height > 2 ? di_.meshCount[di_.height - 3] : 1;
+    const uint64_t bits = rangeSweepBitBytes(upper, nq), segs = static_cast<uint64_t>(nq) * rangeSweepSlots(nq) * sizeof(RangeSegment);
+    if (rsBits_.bytes() < bits || rsBoxF_.bytes() < nq * (5 * DP + 1) * 4 || rsSegs_.bytes() < segs || rsRawCap_ < caps_.results) {
+        dropGraph();
+        if (rsBits_.bytes() < bits) rsBits_.alloc(bits);
+        if (rsBoxF_.bytes() < nq * (5 * DP + 1) * 4) rsBoxF_.alloc(nq * (5 * DP + 1) * 4);
+        if (rsSegs_.bytes() < segs) rsSegs_.alloc(segs);
+        if (rsRawCap_ < caps_.results) {
+            rsRaw_.alloc(caps_.results * 4);
+            rsRawCap_ = caps_.results;
+        }
+    }
+}
+
+bool BatchEngine::rangeSweepReady(uint32_t nq, unsigned flags) const {
+    const uint64_t DP = paddedDims(di_.D), upper = di_.height > 2 ? di_.meshCount[di_.height - 3] : 1;
+    return rsBits_.bytes() >= rangeSweepBitBytes(upper, nq) && rsBoxF_.bytes() >= nq * (5 * DP + 1) * 4 &&
+           rsSegs_.bytes() >= static_cast<uint64_t>(nq) * rangeSweepSlots(nq) * sizeof(RangeSegment) &&
+           rsRawCap_ >= caps_.results && nq <= qcap_ && (!(flags & kWantVals) || haveVals_);
+}
+
+void BatchEngine::enqueueRangeSweep(const double* dBoxes, uint32_t nq, unsigned flags) {
+    lastKnn_ = false;
+    lastCompletion_ = false;
+    lastSweep_ = true;
+    groupsThisBatch_ = floatPointsSupported(di_.D);
+    const int H = static_cast<int>(di_.height);
+    char* z = zeroBlock_.as<char>();
+    if (timing_) record(0);
+    // Tickets, status, headers, result counts and segment counts lie together.
+    TBLAEQ_CUDA(cudaMemsetAsync(z + offTickets_, 0, offQsegs_ + static_cast<size_t>(nq) * 4 - offTickets_, stream_));
+    if (timing_) record(1);
+    RangeSweepArgs a{};
+    a.D = static_cast<int>(di_.D);
+    a.height = H;
+    a.nq = nq;
+    a.words = (nq + 31) / 32;
+    a.boxes = dBoxes;
+    a.boxF = rsBoxF_.as<float>();
+    a.boxGrid = reinterpret_cast<uint32_t*>(a.boxF + static_cast<size_t>(nq) * 4 * paddedDims(di_.D));
+    a.margin = reinterpret_cast<float*>(a.boxGrid + static_cast<size_t>(nq) * paddedDims(di_.D));
+    a.clusterGrid = di_.clusterGrid.as<uint32_t>();
+    std::copy(di_.gridMin, di_.gridMin + 32, a.gridMin);
+    std::copy(di_.gridScale, di_.gridScale + 32, a.gridScale);
+    a.maxAbs = static_cast<float>(di_.maxAbs * (1.0 + 1e-6));
+    a.marginScale = static_cast<float>(std::sqrt(static_cast<double>(di_.D)) * 2.5e-7);  // two float ulps a dimension, doubled
+    for (int m = 0; m + 1 < H; ++m)
+        a.level[m] = RangeSweepLevel{di_.aabbPadded(m), di_.nodeX[m].as<double>(), di_.nodeXF[m].as<float>(),
+                                     di_.radF[m].as<float>(), di_.nodeSub[m].as<NodeRec>(),
+                                     m ? di_.parent[m].as<uint32_t>() : nullptr, static_cast<uint32_t>(di_.meshCount[m])};
+    a.units = di_.units.as<RangeUnit>();
+    a.nUnits = di_.unitCount;
+    a.upper = di_.upperUnits.as<RangeUnit>();
+    a.nUpper = di_.upperUnitCount;
+    a.rowOrder = floatPointsSupported(di_.D) ? 0 : 1;
+    a.clusterGroups = di_.clusterGroups.as<NodeRec>();
+    a.groupRec = di_.groupRec.as<NodeRec>();
+    a.groupBox = di_.groupBox.as<float>();
+    a.countRec = innerRecords(H - 2);
+    a.pointsF = di_.pointsF.as<float>();
+    a.pointsD = di_.pointsD.as<double>();
+    a.perm = di_.pointPerm.as<uint32_t>();
+    a.map = di_.mapPtr[H - 1];
+    a.bits = rsBits_.as<uint32_t>();
+    a.raw = rsRaw_.as<uint32_t>();
+    a.rawCap = static_cast<uint32_t>(rsRawCap_);
+    a.segs = rsSegs_.as<RangeSegment>();
+    a.segSlots = rangeSweepSlots(nq);
+    auto* tickets = reinterpret_cast<uint32_t*>(z + offTickets_);
+    a.ticket = tickets;
+    a.rawCnt = tickets + 1;
+    a.qsegs = reinterpret_cast<uint32_t*>(z + offQsegs_);
+    a.qcount = reinterpret_cast<uint32_t*>(z + offQcount_);
+    a.hdr = hdrPtr(0);
+    a.status = reinterpret_cast<uint32_t*>(z + offStatus_);
+    a.offsets = offsets_.as<uint64_t>();
+    a.ids = resIds_.as<uint64_t>();
+    a.vals = (flags & kWantVals) ? resVals_.as<double>() : nullptr;
+    a.resultCap = static_cast<uint32_t>(caps_.results);
+    launchRangeSweep(a, stream_);
+    if (timing_)
+        for (int m = 0; m <= H; ++m) record(2 + m);
+}
+
 void BatchEngine::enqueueLaunches(const double* dBoxes, uint32_t nq, int mode, unsigned flags) {
     lastKnn_ = false;
     lastCompletion_ = false;
+    lastSweep_ = false;
+    if (useRangeSweep(nq, mode, flags) && rangeSweepReady(nq, flags)) {
+        enqueueRangeSweep(dBoxes, nq, flags);
+        return;
+    }
     const int H = static_cast<int>(di_.height);
     const int D = static_cast<int>(di_.D);
     char* z = zeroBlock_.as<char>();
@@ -700,12 +846,37 @@ BatchOutput BatchEngine::output(uint32_t nq, unsigned flags) const {
     return o;
 }
 
+// After an overflow of the sweep: room for all hits it counted, or more segments per query. A batch
+// whose queries have more segments than the gather orders (each of at least one result) runs level by
+// level, and so do the next ones for a while.
+void BatchEngine::growRangeSweep(uint32_t nq, uint32_t st, unsigned flags) {
+    uint32_t hits = 0;
+    TBLAEQ_CUDA(cudaMemcpyAsync(&hits, zeroBlock_.as<char>() + offTickets_ + 4, 4, cudaMemcpyDeviceToHost, stream_));
+    TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+    dropGraph();
+    if (hits > caps_.results) {
+        EngineCaps want = caps_;
+        want.results = static_cast<uint64_t>(hits) + hits / 4 + 4096;
+        reserve(want, qcap_, haveVals_ || (flags & kWantVals) ? kWantVals : 0);
+    }
+    if (st & kStatusOverflowItems) {
+        if (rangeSweepSlots(nq) >= kRangeSegments)
+            rsSkip_ = 16;
+        else
+            rsSegFactor_ *= 4;
+    }
+}
+
 BatchOutput BatchEngine::runRange(const double* dBoxes, uint32_t nq, int mode, unsigned flags) {
     WorkspaceGuard guard(*this);
     reserve(caps_, nq, flags);
     for (int attempt = 0; attempt < 16; ++attempt) {
         lastRuns_ = static_cast<uint32_t>(attempt + 1);
-        if (useNodeMajor(mode)) reserveNodeMajor(flags);
+        const bool sweep = useRangeSweep(nq, mode, flags);
+        if (sweep)
+            reserveRangeSweep(nq);
+        else if (useNodeMajor(mode))
+            reserveNodeMajor(flags);
         enqueueRange(dBoxes, nq, mode, flags);
         // The status word and the result total come back together: one host synchronisation.
         uint32_t st = 0;
@@ -723,11 +894,15 @@ BatchOutput BatchEngine::runRange(const double* dBoxes, uint32_t nq, int mode, u
         if (st & kStatusOverflowSum)
             throw SplitBatch("a level generates more than 2^32 items; split the batch");
         if (st == 0) {
+            if (!sweep && mode == kModeExact && rsSkip_ && --rsSkip_ == 0) dropGraph();
             BatchOutput o = output(nq, flags);
             o.total = total;
             return o;
         }
-        growFromHeaders();
+        if (sweep)
+            growRangeSweep(nq, st, flags);
+        else
+            growFromHeaders();
     }
     throw CudaError(cudaErrorMemoryAllocation, "traversal workspace did not converge after 16 growth steps");
 }
@@ -1083,9 +1258,9 @@ void BatchEngine::enqueueKnn(const double* dPoints, uint32_t nq, const uint32_t*
         c.rows = di_.rows[H - 2];
         c.rowsOnHost = di_.rowsOnHost[H - 2];
         c.decoded = di_.pointsD.bytes() ? di_.pointsD.as<double>() : nullptr;
-        if (c.decoded && di_.pointPerm.bytes()) {  // decoded points in point-group order
+        if (c.decoded && di_.pointPerm.bytes() && floatPointsSupported(di_.D)) {  // decoded points in point-group order
             c.perm = di_.pointPerm.as<uint32_t>();
-            if (knnGroups_ && paddedDims(di_.D) == di_.D) {  // this kernel reads unpadded boxes
+            if (knnGroups_) {
                 c.clusterGroups = di_.clusterGroups.as<NodeRec>();
                 c.groupRec = di_.groupRec.as<NodeRec>();
                 c.groupBox = di_.groupBox.as<float>();
@@ -1353,6 +1528,7 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
     a.pointsF = di_.pointsF.as<float>();
     a.pointsD = di_.pointsD.as<double>();
     a.perm = di_.pointPerm.as<uint32_t>();
+    a.rowOrder = floatPointsSupported(di_.D) ? 0 : 1;
     a.map = di_.mapPtr[H - 1];
     a.clusterGroups = di_.clusterGroups.as<NodeRec>();
     a.groupRec = di_.groupRec.as<NodeRec>();

@@ -254,6 +254,18 @@ private:
     size_t offDesc_ = 0, offTickets_ = 0, offStatus_ = 0, offHdr_ = 0, offQcount_ = 0, offLevels_ = 0;
     uint64_t tileCap_ = 0;
 
+    // Exact range batches as one sweep (rangesweep.cuh): workspace, and whether the last range batch ran it.
+    DeviceMem rsBits_, rsBoxF_, rsRaw_, rsSegs_;
+    uint32_t rsSegFactor_ = 1, rsSkip_ = 0;
+    uint64_t rsRawCap_ = 0;
+    size_t offQsegs_ = 0;
+    bool rsOff_ = false, lastSweep_ = false;
+    bool useRangeSweep(uint32_t nq, int mode, unsigned flags) const;
+    uint32_t rangeSweepSlots(uint32_t nq) const;
+    void reserveRangeSweep(uint32_t nq);
+    bool rangeSweepReady(uint32_t nq, unsigned flags) const;
+    void enqueueRangeSweep(const double* dBoxes, uint32_t nq, unsigned flags);
+    void growRangeSweep(uint32_t nq, uint32_t st, unsigned flags);
     // Exact KNN as a probe and one sweep (knnsweep.cuh): workspace, and whether the last batch ran it.
     // runKnnSweep returns false when the batch needs the level-synchronous path instead.
     DeviceMem swQuery_, swBits_, swLive_, swCand_, swEnt_;

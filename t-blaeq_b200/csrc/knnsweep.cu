@@ -610,13 +610,14 @@ __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(KnnSweepArgs a) 
                     if (hit) {
                         const uint32_t qq = sId[w][s];
                         const double* pd = a.points + static_cast<size_t>(qq) * a.D;
-                        const double d2 = pointDist2(pd, a.pointsD + static_cast<size_t>(row) * a.D, a.D);
+                        const uint32_t pr = __ldg(a.perm + row);
+                        const double d2 = pointDist2(pd, a.pointsD + static_cast<size_t>(a.rowOrder ? pr : row) * a.D, a.D);
                         const double tau = a.tau[qq];
                         if (d2 <= tau * tau * (1.0 + 1e-9)) {
                             const uint32_t slot = atomicAdd(&a.candCnt[qq], 1u);
                             const uint64_t pos = a.candOff[qq] + slot;
                             if (pos < a.candOff[qq + 1] && pos < a.candCap) {
-                                a.candId[pos] = a.map[__ldg(a.perm + row)];
+                                a.candId[pos] = a.map[pr];
                                 a.candD2[pos] = d2;
                                 ++kept;
                             } else {

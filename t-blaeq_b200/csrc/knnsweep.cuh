@@ -63,6 +63,7 @@ struct KnnSweepArgs {
     const float* pointsF;
     const double* pointsD;
     const uint32_t* perm;
+    int rowOrder;           // pointsD is in row order (row perm[i] holds point i), not in point-group order
     const uint64_t* map;
     const NodeRec* clusterGroups;
     const NodeRec* groupRec;

@@ -1,0 +1,131 @@
+// Exact range batches in three launches: upper test, sweep, gather.
+//
+//   upper   one thread per (node, 32 queries) over the meshes above the finest clusters: bit (node,
+//           query) of the last of them = the node and its ancestors survive for the query;
+//   sweep   one warp per (unit, 1,024 queries), a unit being at most 32 sibling clusters: lanes are
+//           clusters while their boxes are tested against the queries whose bit is set, then
+//           (query, cluster) pairs, then (query, group) pairs, then points. Hits go out as segments:
+//           runs of points of one query and one unit, in traversal order;
+//   gather  per query, its segments in the order of their units, as ids (and coordinates).
+//
+// Against one launch per level this keeps nothing between the levels in memory: no frontier with its
+// coordinates, no look-back, no per-level tail. Every (query, node) pair is decided by the same
+// tests as there -- float box, FP64 radius, float point with the FP64 test near a face -- so the same
+// nodes survive at every level, the counts per level are the same, and so are the results and their
+// order (depth-first: queries, then the clusters in traversal order, then the points: in point-group
+// order at D = 4, 8 and 16, in row order elsewhere).
+//
+// Measured on B200 against the level-synchronous launches, device time of one batch: 4,096 boxes, N = 10M,
+// D = 8: 620 -> 220 us; 37 boxes there: 105 -> 46 us; 100 boxes, N = 500k, D = 5: 110 -> 60 us; one box:
+// 60 -> 28 us; 301 boxes with 1.0M results and their coordinates, N = 1.5M, D = 3: 180 -> 146 us.
+#pragma once
+
+#include <cstdint>
+
+#include "common.cuh"
+#include "traverse.cuh"
+
+namespace tblaeq {
+
+constexpr uint32_t kRangeUnit = 32;        // clusters per unit
+constexpr uint32_t kRangeSegments = 2048;  // segments of a query the gather can order
+constexpr uint32_t kRangeMaxHeight = 16;
+// Most points of a cluster at dimensions whose hits leave in row order (sorted per cluster on chip).
+constexpr uint32_t kRangeRowsCluster = 512;
+
+// At most kRangeUnit consecutive children (finest clusters) of one node of the mesh above.
+struct RangeUnit {
+    uint32_t node, first, count;
+    uint32_t pad;  // upper units: bit t = the first unit below its ancestor of mesh t
+};
+constexpr uint32_t kRangeUpperUnit = 8;    // nodes of an upper unit
+
+// Steps of a box coordinate on the grid of the data's extent (see rangesweep.cu); the host lays out the
+// clusters' boxes with the same functions.
+constexpr double kRangeGrid = 32767.0;
+__host__ __device__ inline double rangeGridStep(double v, double lo, double scale) {
+#ifdef __CUDA_ARCH__
+    return __dmul_rn(__dsub_rn(v, lo), scale);
+#else
+    return (v - lo) * scale;
+#endif
+}
+__host__ __device__ inline uint32_t rangeGridLower(double v, double lo, double scale) {
+    const double s = rangeGridStep(v, lo, scale);  // not a number: 0, which every cluster's box meets
+    return s >= kRangeGrid ? static_cast<uint32_t>(kRangeGrid) : s > 0.0 ? static_cast<uint32_t>(s) : 0u;
+}
+__host__ __device__ inline uint32_t rangeGridUpper(double v, double lo, double scale) {
+    const double s = rangeGridStep(v, lo, scale);
+    if (!(s < kRangeGrid)) return static_cast<uint32_t>(kRangeGrid);
+    if (!(s > 0.0)) return 0u;
+    const uint32_t f = static_cast<uint32_t>(s);
+    return f + (static_cast<double>(f) < s ? 1u : 0u);
+}
+
+struct RangeSegment {
+    uint64_t key;  // unit, then the run's number within it
+    uint32_t pos;  // first hit
+    uint32_t len;
+};
+
+struct RangeSweepLevel {
+    const float* box;       // two padded rows: lo, hi, rounded outward
+    const double* x;        // decoded centres
+    const float* xF;        // the same, padded float rows
+    const float* radF;      // subtree radius, rounded up
+    const NodeRec* nodes;   // subtree radius, first child, child count
+    const uint32_t* parent; // position in the mesh above (null for mesh 0)
+    uint32_t count;
+};
+
+struct RangeSweepArgs {
+    int D, height;
+    uint32_t nq, words;
+    const double* boxes;    // nq x (lo[D] hi[D])
+    float* boxF;            // nq x 4 padded rows: outward lo, hi, inward lo, hi
+    float* margin;          // nq: see radiusQuick
+    uint32_t* boxGrid;      // nq x paddedDims: upper corners (guard bits set), lower corners, two to a word
+    const uint32_t* clusterGrid;  // per finest cluster: lower corners, upper corners (guard bits set)
+    double gridMin[32], gridScale[32];
+    float maxAbs;           // largest |coordinate| of the data, rounded up
+    float marginScale;      // margin = (largest |box coordinate| + maxAbs) * marginScale
+    RangeSweepLevel level[kRangeMaxHeight];  // meshes 0 .. height-2
+    const RangeUnit* units; // in traversal order
+    uint32_t nUnits;
+    const RangeUnit* upper; // siblings of mesh height-3 (node: their parent)
+    uint32_t nUpper;
+    int rowOrder;           // pointsD (and the hits) are in row order, not in point-group order
+    const NodeRec* clusterGroups;
+    const NodeRec* groupRec;
+    const float* groupBox;
+    const NodeRec* countRec;  // what a surviving cluster adds to the finest level's count
+    const float* pointsF;
+    const double* pointsD;
+    const uint32_t* perm;
+    const uint64_t* map;
+    uint32_t* bits;         // last upper mesh (or one virtual root) x words
+    uint32_t* raw;          // hits: rows of the points
+    uint32_t rawCap;
+    RangeSegment* segs;     // nq x segSlots
+    uint32_t segSlots;
+    // Zeroed before the launch:
+    uint32_t* ticket;
+    uint32_t* rawCnt;
+    uint32_t* qsegs;        // segments per query
+    uint32_t* qcount;       // hits per query
+    uint32_t* hdr;          // the engine's level headers
+    uint32_t* status;
+    // Results
+    uint64_t* offsets;
+    uint64_t* ids;
+    double* vals;
+    uint32_t resultCap;
+};
+
+// kStatusOverflowItems here: a query has more segments than segSlots (rawCnt and the headers tell the
+// other capacities).
+void launchRangeSweep(const RangeSweepArgs& a, cudaStream_t s);
+// (query, unit block) tasks etc. are sized inside; bytes of `bits` for nq queries:
+uint64_t rangeSweepBitBytes(uint64_t lastUpper, uint64_t nq);
+
+}  // namespace tblaeq

@@ -1217,6 +1217,8 @@ void setLookbackTestHook(uint32_t withholdTile, uint32_t spinLimit) {
     gHookSpins.store(off ? 0u : spinLimit);
 }
 
+bool lookbackTestHookSet() { return gHookSpins.load() != 0; }
+
 void launchExpand(const ExpandArgs& in, int pred, bool toResult, int gridBlocks, cudaStream_t stream) {
     ExpandArgs a = in;
     a.withholdTile = 0xffffffffu;

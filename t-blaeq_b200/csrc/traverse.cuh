@@ -178,6 +178,7 @@ void launchExpand(const ExpandArgs& a, int pred, bool toResult, int gridBlocks, 
 // restores normal operation. Process-wide; launches captured in a CUDA graph keep the values they
 // were captured with.
 void setLookbackTestHook(uint32_t withholdTile, uint32_t spinLimit);
+bool lookbackTestHookSet();
 
 // Tile size (work items per tile) used by every expand instantiation.
 inline int expandTile(int) { return kWarpTile; }
