@@ -20,6 +20,7 @@ std::atomic<uint64_t> tblaeq::gKernelLaunches{0};
 struct tblaeq_handle {
     std::unique_ptr<QueryHandler> qh;
     DeviceMem stage;                            // device staging for host-side query batches
+    PinnedMem pinIn, pinOut;                    // page-locked staging of small host batches (kPinned bytes a part)
     std::vector<std::vector<uint32_t>> parent;  // parent position per mesh (lazy, decode_points)
     std::vector<std::vector<uint64_t>> posOf;   // position of each original id per mesh (lazy)
     DeviceMem kStage;                           // per-query K of KNN batches
@@ -219,6 +220,20 @@ int tblaeq_coarsest_grid(tblaeq_handle* h, tblaeq_grid* out) {
     return TBLAEQ_OK;
 }
 
+// Host batches whose queries, K, offsets and first results are small go through page-locked staging, so
+// that their copies are plain DMA in the stream: a pageable copy of a few bytes costs the driver's own
+// staging, and back to the host a wait each. Larger copies go straight to the caller's memory.
+constexpr size_t kPinned = 64 << 10;
+
+static void copyIn(tblaeq_handle* h, void* dst, const void* src, size_t bytes, size_t part) {
+    const void* from = src;
+    if (bytes <= kPinned) {
+        if (!h->pinIn.bytes()) h->pinIn.alloc(2 * kPinned);
+        from = std::memcpy(h->pinIn.as<char>() + part * kPinned, src, bytes);
+    }
+    TBLAEQ_CUDA(cudaMemcpyAsync(dst, from, bytes, cudaMemcpyHostToDevice, h->qh->runtime().stream));
+}
+
 // A KNN batch too large for one traversal (high dimensions keep most clusters alive, so the
 // frontier outgrows the 32-bit item space or the free device memory) runs as consecutive chunks,
 // halved until each fits; the
@@ -226,6 +241,7 @@ int tblaeq_coarsest_grid(tblaeq_handle* h, tblaeq_grid* out) {
 // kept for chunked batches.
 static BatchOutput runKnnChunked(tblaeq_handle* h, const double* dQueries, uint64_t nq, const std::vector<uint32_t>& k,
                                  unsigned flags, uint64_t firstChunk) {
+    h->qh->runtime().engine->setAfterEnqueue(nullptr, nullptr);  // a chunk's output is not the batch's
     Runtime& rt = h->qh->runtime();
     const uint64_t D = rt.dev->D;
     uint64_t sumK = 0;
@@ -303,8 +319,7 @@ static int runBatch(tblaeq_handle* h, const tblaeq_batch* b, const double* dQuer
             sumK += v;
         }
         if (h->kStage.bytes() < std::max<size_t>(b->nq, 1) * 4) h->kStage.alloc(std::max<size_t>(b->nq, 1) * 4);
-        if (b->nq)
-            TBLAEQ_CUDA(cudaMemcpyAsync(h->kStage.get(), k.data(), b->nq * 4, cudaMemcpyHostToDevice, rt.stream));
+        if (b->nq) copyIn(h, h->kStage.get(), k.data(), b->nq * 4, 1);
         h->knnSum.clear();
         // A size learnt under the other finest-level mode (one pass or two waves) does not apply.
         const uint64_t hint = (h->knnHintTwoWave == rt.engine->twoWave()) ? h->knnChunkHint : 0;
@@ -360,9 +375,10 @@ int tblaeq_query_batch(tblaeq_handle* h, const tblaeq_batch* b, tblaeq_batch_res
             const uint64_t D = rt.dev->D;
             const size_t bytes = b->nq * (b->qtype == TBLAEQ_RANGE ? 2 * D : D) * 8;
             if (h->stage.bytes() < bytes) h->stage.alloc(bytes);
-            TBLAEQ_CUDA(cudaMemcpyAsync(h->stage.get(), b->queries, bytes,
-                                        b->queriesOnDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                                        rt.stream));
+            if (b->queriesOnDevice)
+                TBLAEQ_CUDA(cudaMemcpyAsync(h->stage.get(), b->queries, bytes, cudaMemcpyDeviceToDevice, rt.stream));
+            else
+                copyIn(h, h->stage.get(), b->queries, bytes, 0);
             dq = h->stage.as<double>();
         }
         return runBatch(h, b, dq, out);
@@ -376,15 +392,59 @@ int tblaeq_query_batch_host(tblaeq_handle* h, const tblaeq_batch* b, uint64_t* o
     return guarded([&]() -> int {
         tblaeq_batch hb = *b;
         tblaeq_batch_result r{};
+        Runtime& rt = h->qh->runtime();
+        // Offsets and the first results come back with the batch's own wait where they are few.
+        struct Fetch {
+            char* to;
+            size_t offBytes, n;
+            bool dist;
+            cudaStream_t stream;
+        } f{nullptr, (b->nq + 1) * 8, 0, false, rt.stream};
+        uint64_t most = 1024 + 4 * b->nq;  // range: a guess; KNN: the neighbours asked for
+        if (b->qtype == TBLAEQ_POINT) {
+            most = 0;
+            for (uint64_t i = 0; i < b->nq && most <= kPinned; ++i) most += b->kPerQuery ? b->kPerQuery[i] : b->K;
+        }
+        f.n = std::min<uint64_t>({most, ids_cap, kPinned / 8, b->nq * rt.host->N});
+        f.dist = dist2_out != nullptr && b->qtype == TBLAEQ_POINT;
+        struct Detach {
+            BatchEngine* e;
+            ~Detach() {
+                if (e) e->setAfterEnqueue(nullptr, nullptr);
+            }
+        } detach{nullptr};
+        if (f.offBytes <= kPinned) {
+            if (!h->pinOut.bytes()) h->pinOut.alloc(3 * kPinned);
+            f.to = h->pinOut.as<char>();
+            detach.e = rt.engine.get();
+            rt.engine->setAfterEnqueue(
+                [](void* ctx, const BatchOutput& o) {
+                    const Fetch& g = *static_cast<Fetch*>(ctx);
+                    TBLAEQ_CUDA(cudaMemcpyAsync(g.to, o.offsets, g.offBytes, cudaMemcpyDeviceToHost, g.stream));
+                    if (!g.n) return;
+                    TBLAEQ_CUDA(cudaMemcpyAsync(g.to + kPinned, o.ids, g.n * 8, cudaMemcpyDeviceToHost, g.stream));
+                    if (g.dist)
+                        TBLAEQ_CUDA(cudaMemcpyAsync(g.to + 2 * kPinned, o.dist2, g.n * 8, cudaMemcpyDeviceToHost, g.stream));
+                },
+                &f);
+        }
         int c = tblaeq_query_batch(h, &hb, &r);
         if (c) return c;
-        Runtime& rt = h->qh->runtime();
-        TBLAEQ_CUDA(cudaMemcpyAsync(offsets_out, r.offsets, (b->nq + 1) * 8, cudaMemcpyDeviceToHost, rt.stream));
         const uint64_t n = std::min<uint64_t>(r.total, ids_cap);
-        if (n) TBLAEQ_CUDA(cudaMemcpyAsync(ids_out, r.ids, n * 8, cudaMemcpyDeviceToHost, rt.stream));
-        if (n && dist2_out && r.dist2)
-            TBLAEQ_CUDA(cudaMemcpyAsync(dist2_out, r.dist2, n * 8, cudaMemcpyDeviceToHost, rt.stream));
-        TBLAEQ_CUDA(cudaStreamSynchronize(rt.stream));
+        const bool fetched = f.to && rt.engine->fetched();
+        if (fetched)
+            std::memcpy(offsets_out, f.to, f.offBytes);
+        else
+            TBLAEQ_CUDA(cudaMemcpyAsync(offsets_out, r.offsets, f.offBytes, cudaMemcpyDeviceToHost, rt.stream));
+        const bool dist = n && dist2_out && r.dist2;
+        if (fetched && n <= f.n) {
+            if (n) std::memcpy(ids_out, f.to + kPinned, n * 8);
+            if (dist) std::memcpy(dist2_out, f.to + 2 * kPinned, n * 8);
+        } else {
+            if (n) TBLAEQ_CUDA(cudaMemcpyAsync(ids_out, r.ids, n * 8, cudaMemcpyDeviceToHost, rt.stream));
+            if (dist) TBLAEQ_CUDA(cudaMemcpyAsync(dist2_out, r.dist2, n * 8, cudaMemcpyDeviceToHost, rt.stream));
+            TBLAEQ_CUDA(cudaStreamSynchronize(rt.stream));
+        }
         if (total) *total = r.total;
         if (r.total > ids_cap) return fail(TBLAEQ_ERR_OVERFLOW, "result ids exceed ids_cap");
         return TBLAEQ_OK;

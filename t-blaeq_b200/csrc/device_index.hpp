@@ -63,6 +63,32 @@ private:
     size_t n_ = 0;
 };
 
+// Page-locked host memory (grown by the caller, freed with the object).
+class PinnedMem {
+public:
+    PinnedMem() = default;
+    ~PinnedMem() { release(); }
+    PinnedMem(const PinnedMem&) = delete;
+    PinnedMem& operator=(const PinnedMem&) = delete;
+    void alloc(size_t bytes) {
+        release();
+        TBLAEQ_CUDA(cudaMallocHost(&p_, bytes));
+        n_ = bytes;
+    }
+    void release() {
+        if (p_) cudaFreeHost(p_);
+        p_ = nullptr;
+        n_ = 0;
+    }
+    size_t bytes() const { return n_; }
+    template <class T>
+    T* as() const { return static_cast<T*>(p_); }
+
+private:
+    void* p_ = nullptr;
+    size_t n_ = 0;
+};
+
 template <class T>
 DeviceMem upload(const std::vector<T>& v, cudaStream_t s = nullptr) {
     DeviceMem m(std::max<size_t>(v.size() * sizeof(T), 16));

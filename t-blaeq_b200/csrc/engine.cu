@@ -270,8 +270,10 @@ void BatchEngine::reserve(const EngineCaps& want, uint32_t nq, unsigned flags) {
     if (c.entries > 0xffffffffull || c.items > 0xffffffffull || c.results > 0xffffffffull)
         throw SplitBatch("batch exceeds 32-bit traversal capacities; split the batch");
     // Frontier and result buffers that would not fit in device memory (beside what this engine
-    // already holds and will release) also call for a smaller batch, not an allocation failure.
-    {
+    // already holds and will release) also call for a smaller batch, not an allocation failure. Asked
+    // only when something grows: the driver takes about 70 us for the answer, and milliseconds while
+    // others ask, on every batch of a handle whose workspace already fits.
+    if (growF || growR) {
         const uint64_t needF = growF ? 2 * (c.entries * (16 + 8 * D) + (c.items / tile_ + 2) * 4) : 0;
         const uint64_t needR = growR ? c.results * (20 + ((wantVals || haveVals_) ? 8 * D : 0)) : 0;
         size_t freeB = 0, totalB = 0;
@@ -763,6 +765,13 @@ std::vector<uint64_t> BatchEngine::groupCounts() {
     return out;
 }
 
+void BatchEngine::fetchControl() {
+    const size_t bytes = offHdr_ + (di_.height + 4) * 8 - offTickets_;
+    if (control_.bytes() < bytes) control_.alloc(bytes);
+    TBLAEQ_CUDA(cudaMemcpyAsync(control_.as<void>(), zeroBlock_.as<char>() + offTickets_, bytes, cudaMemcpyDeviceToHost, stream_));
+    TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+}
+
 uint32_t BatchEngine::status() {
     uint32_t st = 0;
     TBLAEQ_CUDA(cudaMemcpyAsync(&st, zeroBlock_.as<char>() + offStatus_, 4, cudaMemcpyDeviceToHost, stream_));
@@ -850,9 +859,7 @@ BatchOutput BatchEngine::output(uint32_t nq, unsigned flags) const {
 // whose queries have more segments than the gather orders (each of at least one result) runs level by
 // level, and so do the next ones for a while.
 void BatchEngine::growRangeSweep(uint32_t nq, uint32_t st, unsigned flags) {
-    uint32_t hits = 0;
-    TBLAEQ_CUDA(cudaMemcpyAsync(&hits, zeroBlock_.as<char>() + offTickets_ + 4, 4, cudaMemcpyDeviceToHost, stream_));
-    TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+    const uint32_t hits = controlWord(offTickets_ + 4);
     dropGraph();
     if (hits > caps_.results) {
         EngineCaps want = caps_;
@@ -878,12 +885,12 @@ BatchOutput BatchEngine::runRange(const double* dBoxes, uint32_t nq, int mode, u
         else if (useNodeMajor(mode))
             reserveNodeMajor(flags);
         enqueueRange(dBoxes, nq, mode, flags);
-        // The status word and the result total come back together: one host synchronisation.
-        uint32_t st = 0;
-        uint64_t total = 0;
-        TBLAEQ_CUDA(cudaMemcpyAsync(&st, zeroBlock_.as<char>() + offStatus_, 4, cudaMemcpyDeviceToHost, stream_));
-        TBLAEQ_CUDA(cudaMemcpyAsync(&total, offsets_.as<uint64_t>() + nq, 8, cudaMemcpyDeviceToHost, stream_));
-        TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+        // The status word and the result total (the results' header) come back in one copy, and the
+        // caller's copies with them: one host synchronisation.
+        if (after_) after_(afterCtx_, output(nq, flags));
+        fetchControl();
+        const uint32_t st = controlStatus();
+        const uint64_t total = nq ? controlHeader(static_cast<int>(di_.height), 0) : 0;
         // A 32-bit prefix overflow leaves the next frontier's item mapping meaningless, so the
         // launches after it may report window overflows and look-back timeouts of their own: those
         // count as failures only when no overflow explains them.
@@ -897,6 +904,7 @@ BatchOutput BatchEngine::runRange(const double* dBoxes, uint32_t nq, int mode, u
             if (!sweep && mode == kModeExact && rsSkip_ && --rsSkip_ == 0) dropGraph();
             BatchOutput o = output(nq, flags);
             o.total = total;
+            fetched_ = after_ != nullptr;
             return o;
         }
         if (sweep)
@@ -1560,6 +1568,7 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
     a.hdr = hdrPtr(0);
     a.work = reinterpret_cast<unsigned long long*>(z + offWork_);
     a.status = reinterpret_cast<uint32_t*>(z + offStatus_);
+    a.total = reinterpret_cast<unsigned long long*>(z + offTickets_);  // the level-synchronous launches' tickets
     launchKnnSweepPrepare(a, stream_);
     if (timing_) record(1);
     if (scorer_) {
@@ -1607,19 +1616,19 @@ bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t
         lastRuns_ = static_cast<uint32_t>(attempt + 1);
         reserveKnnSweep(nq, cap);
         enqueueKnnSweep(dPoints, nq, dK);
-        uint32_t st = 0;
-        uint32_t entries = 0;
-        uint64_t total = 0;
-        TBLAEQ_CUDA(cudaMemcpyAsync(&st, zeroBlock_.as<char>() + offStatus_, 4, cudaMemcpyDeviceToHost, stream_));
-        TBLAEQ_CUDA(cudaMemcpyAsync(&total, swOff_ + nq, 8, cudaMemcpyDeviceToHost, stream_));
-        TBLAEQ_CUDA(cudaMemcpyAsync(&entries, hdrPtr(static_cast<int>(di_.height) - 1), 4, cudaMemcpyDeviceToHost, stream_));
-        TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+        swLast_ = true;  // output() names the sweep's offsets
+        if (after_) after_(afterCtx_, output(nq, 0));
+        fetchControl();
+        swLast_ = false;
+        const uint32_t st = controlStatus(), entries = controlHeader(static_cast<int>(di_.height) - 1, 0);
+        const uint64_t total = controlWord(offTickets_) | static_cast<uint64_t>(controlWord(offTickets_ + 4)) << 32;
         if (st & kStatusKnnFallback) return false;
         if (st == 0) {
             if (splitLimit_ < 0xffffffffull) checkSplitLimit();
             swLast_ = true;
             o = output(nq, 0);
             o.total = total;
+            fetched_ = after_ != nullptr;
             return true;
         }
         if (scorer_ && entries > swEntCap_) {

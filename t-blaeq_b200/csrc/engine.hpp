@@ -115,6 +115,16 @@ public:
         pointGroups_ = on;
     }
     std::vector<uint64_t> groupCounts();
+    // Called by the synchronous batches after each enqueue, before their wait, with the batch's output
+    // (total not yet known): the caller's own copies then share that wait. `fetched` tells whether the
+    // last batch called it for the run it returned.
+    using AfterEnqueue = void (*)(void* ctx, const BatchOutput& o);
+    void setAfterEnqueue(AfterEnqueue fn, void* ctx) {
+        after_ = fn;
+        afterCtx_ = ctx;
+        fetched_ = false;
+    }
+    bool fetched() const { return fetched_; }
     // Enqueues of the last synchronous batch: 1, plus one rerun per workspace growth.
     uint32_t lastRuns() const { return lastRuns_; }
     // Kernel nodes and all nodes of the captured range graph (0, 0 when none is held).
@@ -254,6 +264,15 @@ private:
     size_t offDesc_ = 0, offTickets_ = 0, offStatus_ = 0, offHdr_ = 0, offQcount_ = 0, offLevels_ = 0;
     uint64_t tileCap_ = 0;
 
+    AfterEnqueue after_ = nullptr;
+    void* afterCtx_ = nullptr;
+    bool fetched_ = false;
+    // The control words of a batch (tickets, status, headers), read back in one copy.
+    PinnedMem control_;
+    void fetchControl();  // enqueues the copy and waits for the stream
+    uint32_t controlWord(size_t offset) const { return control_.as<uint32_t>()[(offset - offTickets_) / 4]; }
+    uint32_t controlStatus() const { return controlWord(offStatus_); }
+    uint32_t controlHeader(int level, int which) const { return controlWord(offHdr_ + (2 * level + which) * 4); }
     // Exact range batches as one sweep (rangesweep.cuh): workspace, and whether the last range batch ran it.
     DeviceMem rsBits_, rsBoxF_, rsRaw_, rsSegs_;
     uint32_t rsSegFactor_ = 1, rsSkip_ = 0;

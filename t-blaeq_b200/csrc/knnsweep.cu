@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(1024) sweepPrepareKernel(KnnSweepArgs a, uint3
     }
     if (tid == 0) {
         a.outOff[a.nq] = sCarryR;
+        *a.total = sCarryR;
         a.candOff[a.nq] = sCarryC;
         a.hdr[0] = a.nq;
         a.hdr[1] = a.nq * a.level[0].count;

@@ -100,6 +100,7 @@ struct KnnSweepArgs {
     uint32_t* liveCnt;
     uint32_t* ticket;
     uint32_t* hdr;          // the engine's level headers: (entries, items) of levels 0 .. height + 1
+    unsigned long long* total; // results of the batch
     unsigned long long* work;  // [0] points the probe measured, [1] points the sweep tested
     uint32_t* status;
 };
