@@ -1,6 +1,7 @@
 // C++ host facade: QueryHandler, PolicyScheduler and the B200 per-level strategy.
 #include "handler.hpp"
 
+#include "gridlevel.cuh"
 #include "knn.cuh"
 
 #include <algorithm>
@@ -98,6 +99,7 @@ Runtime::~Runtime() {
     knnCnt.release();
     knnRr.release();
     scratchQuery.release();
+    gridScratch.release();
     dev.reset();
     if (stream) cudaStreamDestroy(stream);
 }
@@ -178,7 +180,36 @@ LevelResult B200Strategy::runLevel(size_t l, SparseGrid* curGrid, QueryType qTyp
         out.cap = cap;
     }
     uint64_t n = 0;
-    if (qType == QueryType::RANGE) {
+    if (cur.nnz > 0 && cur.nnz <= kGridLevelMax && D <= 32 && !lookbackTestHookSet()) {
+        GridLevelArgs a{};
+        a.ids = cur.ids;
+        a.vals = cur.vals;
+        a.p = static_cast<uint32_t>(cur.nnz);
+        a.D = static_cast<int>(D);
+        a.knn = qType == QueryType::RANGE ? 0 : 1;
+        if (a.knn) {
+            std::copy(queryPoint, queryPoint + D, a.q);
+        } else {
+            std::copy(lo, lo + D, a.q);
+            std::copy(hi, hi + D, a.q + D);
+        }
+        a.K = K;
+        a.nodes = rt_.dev->nodeOrig[l].as<NodeRec>();
+        a.rows = rt_.dev->rows[l];
+        a.rowsOnHost = rt_.dev->rowsOnHost[l];
+        a.map = rt_.dev->mapPtr[l + 1];
+        if (rt_.gridScratch.bytes() < gridLevelScratchBytes(a.p)) rt_.gridScratch.alloc(gridLevelScratchBytes(kGridLevelMax));
+        if (!rt_.gridCount.bytes()) rt_.gridCount.alloc(64);
+        gridLevelScratch(a, rt_.gridScratch.get());
+        a.outIds = out.ids.as<uint64_t>();
+        a.outVals = out.vals.as<double>();
+        a.outCap = static_cast<uint32_t>(std::min<uint64_t>(cap, 0xffffffffull));
+        launchGridLevel(a, rt_.stream);
+        TBLAEQ_CUDA(cudaMemcpyAsync(rt_.gridCount.as<void>(), a.bound + 1, 8, cudaMemcpyDeviceToHost, rt_.stream));
+        TBLAEQ_CUDA(cudaStreamSynchronize(rt_.stream));
+        n = *rt_.gridCount.as<uint64_t>();
+        if (n > cap) throw CudaError(cudaErrorMemoryAllocation, "level output exceeds its buffer");
+    } else if (qType == QueryType::RANGE) {
         TBLAEQ_CUDA(cudaMemcpyAsync(rt_.scratchQuery.as<double>(), lo, D * 8, cudaMemcpyHostToDevice, rt_.stream));
         TBLAEQ_CUDA(cudaMemcpyAsync(rt_.scratchQuery.as<double>() + D, hi, D * 8, cudaMemcpyHostToDevice, rt_.stream));
         n = rt_.pluginEngine->runGridLevel(static_cast<int>(l), cur.ids, cur.vals, cur.nnz, true,

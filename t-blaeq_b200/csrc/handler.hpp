@@ -204,6 +204,8 @@ struct Runtime {
     // Per-level KNN plugin scratch: bound keys, labels (+ sort scratch), child counts, STEP bounds, mask.
     DeviceMem knnKeys, knnKeys2, knnLabels, knnLabels2, knnCnt, knnRr, pluginMask;
     uint64_t knnCap = 0;
+    DeviceMem gridScratch;   // plugin levels without a sort (gridlevel.cuh)
+    PinnedMem gridCount;
     DeviceMem scratchQuery;  // lo|hi or point staged on the device
     // Learned frontier scorer and the maps its training labels need.
     std::unique_ptr<Mlp> scorer;
