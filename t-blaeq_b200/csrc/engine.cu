@@ -1502,7 +1502,7 @@ void BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK) {
         const uint64_t up = di_.height > 2 ? std::max<uint64_t>(1, di_.meshCount[di_.height - 3]) : 0;
         const uint64_t each = std::min<uint64_t>(nC, up ? probeBeam_ * ((nC + up - 1) / up) : nC);
         const uint64_t want = std::max<uint64_t>(swEntCap_, nq * each * 5 / 4 + 1024);
-        if (swEnt_.bytes() < want * (4 + 4 + 8 * D + 8)) swEnt_.alloc(want * (4 + 4 + 8 * D + 8));
+        if (swEnt_.bytes() < want * (4 + 4 + 8)) swEnt_.alloc(want * (4 + 4 + 8));
         swEntCap_ = want;
     }
     if (knnCap_ < std::max<uint64_t>(sumK, 1)) {
@@ -1573,16 +1573,13 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
     if (timing_) record(1);
     if (scorer_) {
         a.entCap = static_cast<uint32_t>(std::min<uint64_t>(swEntCap_, 0xffffffffull));
-        a.entX = swEnt_.as<double>();
-        double* score = a.entX + swEntCap_ * D;
+        double* score = swEnt_.as<double>();
         a.score = score;
         a.entQ = reinterpret_cast<uint32_t*>(score + swEntCap_);
         a.entNode = a.entQ + swEntCap_;
-        a.nodeX = di_.nodeX[H - 2].as<double>();
         launchKnnProbe(a, kProbeEntries, stream_);
         FrontierIn f{};
         f.q = a.entQ;
-        f.x = a.entX;
         f.hdr = hdrPtr(H - 1);
         f.cap = a.entCap;
         scorer_(scorerCtx_, f, a.entNode, a.entCap, dPoints, score, stream_);

@@ -297,8 +297,6 @@ __global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(KnnSweepArgs a, 
             const uint32_t j = H > 2 ? itemOf(i) : i;
             a.entQ[base + i] = q;
             a.entNode[base + i] = j;
-            for (int d = 0; d < a.D; ++d)
-                a.entX[static_cast<size_t>(base + i) * a.D + d] = a.nodeX[static_cast<size_t>(j) * a.D + d];
         }
         return;
     }
@@ -513,13 +511,125 @@ constexpr int kSweepWarps = kSweepThreads / 32;
 constexpr uint32_t kSweepList = 1024 + 32;
 constexpr uint32_t kSweepGroups = 8;  // group boxes staged at once
 
+// A point that passed the float filter: measured in FP64, and a candidate when it lies within the bound.
+__device__ __forceinline__ bool measureInline(const KnnSweepArgs& a, uint32_t row, uint32_t q) {
+    const uint32_t pr = __ldg(a.perm + row);
+    const double d2 = pointDist2(a.points + static_cast<size_t>(q) * a.D,
+                                 a.pointsD + static_cast<size_t>(a.rowOrder ? pr : row) * a.D, a.D);
+    const double tau = a.tau[q];
+    if (!(d2 <= tau * tau * (1.0 + 1e-9))) return false;
+    const uint64_t pos = a.candOff[q] + atomicAdd(&a.candCnt[q], 1u);
+    if (pos < a.candOff[q + 1] && pos < a.candCap) {
+        a.candId[pos] = a.map[pr];
+        a.candD2[pos] = d2;
+        return true;
+    }
+    atomicOr(a.status, kStatusOverflowEntries);
+    return false;
+}
+
+// Out of line where the registers around it are short (a few in ten thousand tested points come here).
+__device__ __noinline__ bool measure(const KnnSweepArgs& a, uint32_t row, uint32_t q) { return measureInline(a, row, q); }
+
+// Deals the clusters to the warps and hands each cluster's queries (the set bits of its row) to
+// batch(cluster, first list entry, n <= 32).
+template <class Batch>
+__device__ __forceinline__ void sweepClusters(const KnnSweepArgs& a, uint32_t* list, Batch&& batch) {
+    const int lane = threadIdx.x & 31;
+    const bool listed = a.qEnd - a.qBegin <= kBoundWords * 32;
+    const uint32_t nClusters = listed ? *a.liveCnt : a.level[a.height - 2].count;
+    // Clusters per ticket: several where there are many, so the ticket's atomic does not bound the sweep.
+    const uint32_t chunk = max(1u, min(8u, nClusters / (gridDim.x * kSweepWarps * 8u)));
+    uint32_t k = 0, kEnd = 0;
+    while (true) {
+        if (k == kEnd) {
+            if (lane == 0) k = atomicAdd(a.ticket, chunk);
+            k = __shfl_sync(FULL, k, 0);
+            if (k >= nClusters) break;
+            kEnd = min(nClusters, k + chunk);
+        }
+        const uint32_t c = listed ? a.live[k] : k;
+        ++k;
+        const uint32_t* row = a.bits + static_cast<size_t>(c) * a.words;
+        uint32_t n = 0;
+        for (uint32_t w0 = 0; w0 < a.words; w0 += 32) {
+            uint32_t word = (w0 + lane < a.words) ? row[w0 + lane] : 0u;
+            uint32_t inc = __popc(word);
+            const uint32_t own = inc;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += t;
+            }
+            const uint32_t add = __shfl_sync(FULL, inc, 31);
+            if (add == 0) continue;
+            uint32_t at = n + inc - own;
+            const uint32_t q0 = a.qBegin + (w0 + lane) * 32;
+            while (word) {
+                list[at++] = q0 + __ffs(word) - 1;
+                word &= word - 1;
+            }
+            __syncwarp();
+            n += add;
+            uint32_t from = 0;
+            const bool last = w0 + 32 >= a.words;
+            for (; from + 32 <= n; from += 32) batch(c, from, 32);
+            if (last) break;
+            // The rest waits for the next words.
+            const uint32_t rest = n - from;
+            const uint32_t keep = static_cast<uint32_t>(lane) < rest ? list[from + lane] : 0u;
+            __syncwarp();
+            if (static_cast<uint32_t>(lane) < rest) list[lane] = keep;
+            __syncwarp();
+            n = rest;
+        }
+        const uint32_t full = n / 32 * 32;
+        if (n > full) batch(c, full, n - full);
+        __syncwarp();
+    }
+}
+
+// Copies the boxes of ng groups from g on to shared memory.
+template <int DP>
+__device__ __forceinline__ void stageBoxes(const KnnSweepArgs& a, float (*box)[2 * DP], uint32_t g, uint32_t ng) {
+    const float4* src = reinterpret_cast<const float4*>(a.groupBox + static_cast<size_t>(g) * 2 * DP);
+    for (uint32_t i = threadIdx.x & 31; i < ng * (2 * DP / 4); i += 32) reinterpret_cast<float4*>(&box[0][0])[i] = __ldg(src + i);
+}
+
+// max(a, b, c) in one instruction (sm_100 three-input max.f32).
+__device__ __forceinline__ float max3f(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// Squared distance from p to a staged box, two dimensions an instruction where there is one.
+template <int DP>
+__device__ __forceinline__ float boxGap2(const float* b, const float (&p)[DP]) {
+    float2 gap = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int d = 0; d < DP; d += 4) {
+        const float4 lo = *reinterpret_cast<const float4*>(b + d);
+        const float4 hi = *reinterpret_cast<const float4*>(b + DP + d);
+        const float2 q0 = make_float2(p[d], p[d + 1]), q1 = make_float2(p[d + 2], p[d + 3]);
+        const float2 m0 = make_float2(-p[d], -p[d + 1]), m1 = make_float2(-p[d + 2], -p[d + 3]);
+        const float2 l0 = __fadd2_rn(make_float2(lo.x, lo.y), m0), h0 = __fadd2_rn(q0, make_float2(-hi.x, -hi.y));
+        const float2 l1 = __fadd2_rn(make_float2(lo.z, lo.w), m1), h1 = __fadd2_rn(q1, make_float2(-hi.z, -hi.w));
+        const float2 e0 = make_float2(max3f(l0.x, h0.x, 0.f), max3f(l0.y, h0.y, 0.f));
+        const float2 e1 = make_float2(max3f(l1.x, h1.x, 0.f), max3f(l1.y, h1.y, 0.f));
+        gap = __ffma2_rn(e0, e0, gap);
+        gap = __ffma2_rn(e1, e1, gap);
+    }
+    return gap.x + gap.y;
+}
+
 // One warp per cluster. Lanes are queries while boxes are tested and points while distances are: a
 // group's points stay in registers and every query whose box test passed is broadcast from shared
 // memory, so no lane idles for another query's sake. Bound by the float pipe and the latency of a
-// cluster's first loads. 84M (query, point) tests of 4,096 queries, D = 8: 422 us (the walk's point
-// passes: 2.9 ms for 187M); 811M of 1,000 queries, D = 16: 2.6 ms (26 ms for 1,760M).
+// cluster's first loads. 84M (query, point) tests of 4,096 queries, N = 10M, D = 8: 383 us (422 us before
+// the box test took three-input maxima and packed pairs; the walk's point passes: 2.9 ms for 187M).
 template <int DP>
-__global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(KnnSweepArgs a) {
+__global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(const __grid_constant__ KnnSweepArgs a) {
     __shared__ uint32_t sList[kSweepWarps][kSweepList];
     __shared__ __align__(16) float sP[kSweepWarps][32][DP];
     __shared__ float sThr[kSweepWarps][32];
@@ -527,15 +637,13 @@ __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(KnnSweepArgs a) 
     __shared__ __align__(16) float sBox[kSweepWarps][kSweepGroups][2 * DP];
     if (*a.status) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const KnnSweepLevel& L = a.level[a.height - 2];
-    const bool listed = a.qEnd - a.qBegin <= kBoundWords * 32;
-    const uint32_t nClusters = listed ? *a.liveCnt : L.count;
     unsigned long long tested = 0;
     uint32_t kept = 0;              // this lane's candidates
     uint32_t staged = 0xffffffffu;  // first group whose box is in sBox
 
     // A batch of n <= 32 queries of the list against the cluster's groups.
-    auto batch = [&](const NodeRec& cg, uint32_t from, uint32_t n) {
+    auto batch = [&](uint32_t c, uint32_t from, uint32_t n) {
+        const NodeRec cg = a.clusterGroups[c];
         const bool v = static_cast<uint32_t>(lane) < n;
         const uint32_t q = v ? sList[w][from + lane] : 0u;
         float p[DP];
@@ -560,28 +668,11 @@ __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(KnnSweepArgs a) 
             __syncwarp();
             if (staged != cg.cbeg + g0) {
                 staged = cg.cbeg + g0;
-                const float4* src = reinterpret_cast<const float4*>(a.groupBox + static_cast<size_t>(staged) * 2 * DP);
-                for (uint32_t i = lane; i < ng * (2 * DP / 4); i += 32)
-                    reinterpret_cast<float4*>(&sBox[w][0][0])[i] = __ldg(src + i);
+                stageBoxes<DP>(a, sBox[w], staged, ng);
             }
             __syncwarp();
             for (uint32_t g = 0; g < ng; ++g) {
-                const float* b = sBox[w][g];
-                float gap = 0.f;
-#pragma unroll
-                for (int d = 0; d < DP; d += 4) {
-                    const float4 lo = *reinterpret_cast<const float4*>(b + d);
-                    const float4 hi = *reinterpret_cast<const float4*>(b + DP + d);
-                    const float e0 = fmaxf(fmaxf(lo.x - p[d], p[d] - hi.x), 0.f);
-                    const float e1 = fmaxf(fmaxf(lo.y - p[d + 1], p[d + 1] - hi.y), 0.f);
-                    const float e2 = fmaxf(fmaxf(lo.z - p[d + 2], p[d + 2] - hi.z), 0.f);
-                    const float e3 = fmaxf(fmaxf(lo.w - p[d + 3], p[d + 3] - hi.w), 0.f);
-                    gap = fmaf(e0, e0, gap);
-                    gap = fmaf(e1, e1, gap);
-                    gap = fmaf(e2, e2, gap);
-                    gap = fmaf(e3, e3, gap);
-                }
-                uint32_t mask = __ballot_sync(FULL, gap <= thr);
+                uint32_t mask = __ballot_sync(FULL, boxGap2<DP>(sBox[w][g], p) <= thr);
                 if (mask == 0) continue;
                 const NodeRec gr = a.groupRec[cg.cbeg + g0 + g];
                 const bool pv = static_cast<uint32_t>(lane) < gr.cnt;
@@ -608,79 +699,203 @@ __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(KnnSweepArgs a) 
                     }
                     const bool hit = pv && acc.x + acc.y <= sThr[w][s];
                     if (__ballot_sync(FULL, hit) == 0) continue;
-                    if (hit) {
-                        const uint32_t qq = sId[w][s];
-                        const double* pd = a.points + static_cast<size_t>(qq) * a.D;
-                        const uint32_t pr = __ldg(a.perm + row);
-                        const double d2 = pointDist2(pd, a.pointsD + static_cast<size_t>(a.rowOrder ? pr : row) * a.D, a.D);
-                        const double tau = a.tau[qq];
-                        if (d2 <= tau * tau * (1.0 + 1e-9)) {
-                            const uint32_t slot = atomicAdd(&a.candCnt[qq], 1u);
-                            const uint64_t pos = a.candOff[qq] + slot;
-                            if (pos < a.candOff[qq + 1] && pos < a.candCap) {
-                                a.candId[pos] = a.map[pr];
-                                a.candD2[pos] = d2;
-                                ++kept;
-                            } else {
-                                atomicOr(a.status, kStatusOverflowEntries);
-                            }
-                        }
-                    }
+                    if (hit && measureInline(a, row, sId[w][s])) ++kept;
                 }
             }
         }
     };
 
-    // Clusters per ticket: several where there are many, so the ticket's atomic does not bound the sweep.
-    const uint32_t chunk = max(1u, min(8u, nClusters / (gridDim.x * kSweepWarps * 8u)));
-    uint32_t k = 0, kEnd = 0;
-    while (true) {
-        if (k == kEnd) {
-            if (lane == 0) k = atomicAdd(a.ticket, chunk);
-            k = __shfl_sync(FULL, k, 0);
-            if (k >= nClusters) break;
-            kEnd = min(nClusters, k + chunk);
-        }
-        const uint32_t c = listed ? a.live[k] : k;
-        ++k;
-        const NodeRec cg = a.clusterGroups[c];
-        const uint32_t* row = a.bits + static_cast<size_t>(c) * a.words;
-        uint32_t n = 0;
-        for (uint32_t w0 = 0; w0 < a.words; w0 += 32) {
-            uint32_t word = (w0 + lane < a.words) ? row[w0 + lane] : 0u;
-            uint32_t inc = __popc(word);
-            const uint32_t own = inc;
+    sweepClusters(a, sList[w], batch);
+    if (lane == 0 && tested) atomicAdd(a.work + 1, tested);
+    kept = __reduce_add_sync(FULL, kept);
+    if (lane == 0 && kept) atomicAdd(a.hdr + 2 * (a.height + 1), kept);
+}
+
+// d = a (16 x 8) * b (8 x 8) + c, TF32 operands (the low 13 bits of a float are not read), FP32 sums.
+__device__ __forceinline__ void mmaTf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1,
+                                       float c2, float c3) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+// One warp per cluster: its queries, 32 at a time, against its points, 16 at a time, as a product on the
+// matrix units. With y and p relative to the cluster's centre, |y - p|^2 <= thr is
+//     y.p >= |y|^2 / 2 + (|p|^2 - thr) / 2,
+// so the query's side seeds the accumulator and a comparison per pair remains. TF32 drops 13 bits of
+// each factor: y.p is off by at most 2^-9 |y| |p|, and the query's side is lowered by that (with the
+// cluster's radius for |y|), so the filter only lets too much through; measure() decides. The boxes of
+// the cluster's point groups are tested first, a query a lane: a group no query of the batch reaches
+// is not read.
+//
+// Taken above eight (padded) dimensions. On the float pipe (a point per lane, queries broadcast from shared
+// memory) the broadcasts bound it there: 1,000 queries, N = 5M, D = 16, 811M needed pairs: 2.53 ms at 85%
+// of the shared-memory pipe and 1,681M instructions, here 1.73 ms and 762M, bound by latency: four
+// blocks an SM (128 registers), an instruction in 40% of the issue slots. At D = 8, where a box test
+// leaves about four of a batch's queries, the product does eight times the needed pairs and is slower
+// (868 against 422 us).
+template <int DP>
+__global__ void __launch_bounds__(kSweepThreads, DP <= 16 ? 4 : 2) knnSweepMmaKernel(const __grid_constant__ KnnSweepArgs a) {
+    constexpr int STEPS = (DP + 7) / 8;
+    __shared__ uint32_t sList[kSweepWarps][kSweepList];
+    __shared__ __align__(16) float sBox[kSweepWarps][kSweepGroups][2 * DP];
+    if (*a.status) return;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int quad = lane >> 2, kc = 2 * (lane & 3);  // fragment row, first of the lane's two dimensions in a step
+    const KnnSweepLevel& L = a.level[a.height - 2];
+    unsigned long long tested = 0;
+    uint32_t kept = 0;               // this lane's candidates
+    uint32_t staged = 0xffffffffu;  // first group whose box is in sBox
+
+    // The lane's pair of dimensions of a padded float row, step s (zero past the row).
+    auto pairAt = [&](const float* row, int s) {
+        return (8 * s + kc < DP) ? __ldg(reinterpret_cast<const float2*>(row + 8 * s + kc)) : make_float2(0.f, 0.f);
+    };
+
+    // A batch of n <= 32 queries of the list against cluster c.
+    auto batch = [&](uint32_t c, uint32_t from, uint32_t n) {
+        const float* centre = L.x + static_cast<size_t>(c) * DP;
+        const float rad = __ldg(L.rad + c);
+        const uint32_t nt = (n + 7) / 8;
+        float2 ctr[STEPS];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(FULL, inc, o);
-                if (lane >= o) inc += t;
+        for (int s = 0; s < STEPS; ++s) ctr[s] = pairAt(centre, s);
+        // Queries: fragments (tile t, column quad), and what seeds the accumulators.
+        uint32_t b[4][STEPS][2];
+        float seed[4][2];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            seed[t][0] = seed[t][1] = -INFINITY;
+            if (static_cast<uint32_t>(t) >= nt) continue;  // warp-uniform
+            const uint32_t i = t * 8 + quad;
+            const bool v = i < n;
+            const uint32_t q = sList[w][from + (v ? i : 0)];
+            const float* row = a.qF + static_cast<size_t>(q) * DP;
+            float n2 = 0.f;
+#pragma unroll
+            for (int s = 0; s < STEPS; ++s) {
+                const float2 p = pairAt(row, s);
+                const float x = p.x - ctr[s].x, y = p.y - ctr[s].y;
+                n2 = fmaf(x, x, fmaf(y, y, n2));
+                b[t][s][0] = __float_as_uint(x);
+                b[t][s][1] = __float_as_uint(y);
             }
-            const uint32_t add = __shfl_sync(FULL, inc, 31);
-            if (add == 0) continue;
-            uint32_t at = n + inc - own;
-            const uint32_t q0 = a.qBegin + (w0 + lane) * 32;
-            while (word) {
-                sList[w][at++] = q0 + __ffs(word) - 1;
-                word &= word - 1;
-            }
-            __syncwarp();
-            n += add;
-            uint32_t from = 0;
-            const bool last = w0 + 32 >= a.words;
-            for (; from + 32 <= n; from += 32) batch(cg, from, 32);
-            if (last) break;
-            // The rest waits for the next words.
-            const uint32_t rest = n - from;
-            const uint32_t keep = static_cast<uint32_t>(lane) < rest ? sList[w][from + lane] : 0u;
-            __syncwarp();
-            if (static_cast<uint32_t>(lane) < rest) sList[w][lane] = keep;
-            __syncwarp();
-            n = rest;
+            n2 += __shfl_xor_sync(FULL, n2, 1);
+            n2 += __shfl_xor_sync(FULL, n2, 2);
+            const float thr = a.thrF[q];
+            const float slack = 0.0021f * rad * sqrtf(n2) + 4e-6f * (n2 + rad * rad);
+            const float mine = v ? 0.5f * (thr * kRel - n2) + slack : -INFINITY;
+            seed[t][0] = __shfl_sync(FULL, mine, kc * 4);
+            seed[t][1] = __shfl_sync(FULL, mine, kc * 4 + 4);
         }
-        const uint32_t full = n / 32 * 32;
-        if (n > full) batch(cg, full, n - full);
-        __syncwarp();
-    }
+        // A group's points, all loaded at once (two tiles of sixteen rows) while the group before is tested.
+        float2 y[4][STEPS];
+        auto fetch = [&](uint32_t first, uint32_t cnt) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const uint32_t r = quad + 8 * h;
+                const float* row = a.pointsF + static_cast<size_t>(first + (r < cnt ? r : 0)) * DP;
+#pragma unroll
+                for (int s = 0; s < STEPS; ++s) y[h][s] = pairAt(row, s);
+            }
+        };
+        // Tests the fetched group; fetches the next (cnt2 points from first2 on) once its own are in use.
+        auto points = [&](uint32_t first, uint32_t cnt, uint32_t first2, uint32_t cnt2) {
+            const uint32_t end = first + cnt;
+            uint32_t f[2][STEPS][4];
+            float h[2][2];
+#pragma unroll
+            for (int tile = 0; tile < 2; ++tile)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float n2 = 0.f;
+#pragma unroll
+                    for (int s = 0; s < STEPS; ++s) {
+                        const float x0 = y[2 * tile + half][s].x - ctr[s].x, x1 = y[2 * tile + half][s].y - ctr[s].y;
+                        n2 = fmaf(x0, x0, fmaf(x1, x1, n2));
+                        f[tile][s][half] = __float_as_uint(x0);
+                        f[tile][s][2 + half] = __float_as_uint(x1);
+                    }
+                    n2 += __shfl_xor_sync(FULL, n2, 1);
+                    n2 += __shfl_xor_sync(FULL, n2, 2);
+                    h[tile][half] = 0.5f * n2;
+                }
+            if (cnt2) fetch(first2, cnt2);
+#pragma unroll
+            for (int tile = 0; tile < 2; ++tile) {
+                if (static_cast<uint32_t>(tile) * 16 >= cnt) break;  // warp-uniform
+                bool any = false;
+                float d[4][4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    if (static_cast<uint32_t>(t) >= nt) continue;  // warp-uniform
+                    mmaTf32(d[t], f[tile][0], b[t][0][0], b[t][0][1], seed[t][0], seed[t][1], seed[t][0], seed[t][1]);
+#pragma unroll
+                    for (int s = 1; s < STEPS; ++s)
+                        mmaTf32(d[t], f[tile][s], b[t][s][0], b[t][s][1], d[t][0], d[t][1], d[t][2], d[t][3]);
+                    any = any || d[t][0] >= h[tile][0] || d[t][1] >= h[tile][0] || d[t][2] >= h[tile][1] || d[t][3] >= h[tile][1];
+                }
+                if (__ballot_sync(FULL, any) == 0) continue;
+                if (any) {
+#pragma unroll
+                    for (int t = 0; t < 4; ++t)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint32_t r = first + 16 * tile + quad + (j & 2) * 4, i = t * 8 + kc + (j & 1);
+                            if (i < n && r < end && d[t][j] >= h[tile][j >> 1] && measure(a, r, sList[w][from + i])) ++kept;
+                        }
+                }
+                __syncwarp();
+            }
+        };
+        // Lanes are queries while the groups' boxes are tested.
+        const NodeRec cg = a.clusterGroups[c];
+        const bool v = static_cast<uint32_t>(lane) < n;
+        const uint32_t q = sList[w][from + (v ? lane : 0)];
+        const float thr = v ? a.thrF[q] : -1.f;
+        for (uint32_t g0 = 0; g0 < cg.cnt; g0 += kSweepGroups) {
+            const uint32_t ng = min(kSweepGroups, cg.cnt - g0);
+            __syncwarp();
+            if (staged != cg.cbeg + g0) {
+                staged = cg.cbeg + g0;
+                stageBoxes<DP>(a, sBox[w], staged, ng);
+            }
+            const NodeRec gr = a.groupRec[cg.cbeg + g0 + min(static_cast<uint32_t>(lane), ng - 1)];
+            __syncwarp();
+            uint32_t mine = 0;  // lane g: group g's queries
+            {
+                float p[DP];
+#pragma unroll
+                for (int d = 0; d < DP; d += 4) {
+                    const float4 t = __ldg(reinterpret_cast<const float4*>(a.qF + static_cast<size_t>(q) * DP + d));
+                    p[d] = t.x;
+                    p[d + 1] = t.y;
+                    p[d + 2] = t.z;
+                    p[d + 3] = t.w;
+                }
+                for (uint32_t g = 0; g < ng; ++g) {
+                    const uint32_t m = __ballot_sync(FULL, boxGap2<DP>(sBox[w][g], p) <= thr);
+                    if (static_cast<uint32_t>(lane) == g) mine = m;
+                }
+            }
+            uint32_t some = __ballot_sync(FULL, mine != 0);
+            if (some == 0) continue;
+            tested += static_cast<unsigned long long>(__reduce_add_sync(FULL, __popc(mine) * gr.cnt));
+            int g = __ffs(some) - 1;
+            uint32_t first = __shfl_sync(FULL, gr.cbeg, g), cnt = __shfl_sync(FULL, gr.cnt, g);
+            fetch(first, cnt);
+            while (some) {
+                some &= some - 1;
+                g = some ? __ffs(some) - 1 : 0;
+                const uint32_t first2 = __shfl_sync(FULL, gr.cbeg, g), cnt2 = some ? __shfl_sync(FULL, gr.cnt, g) : 0u;
+                points(first, cnt, first2, cnt2);
+                first = first2;
+                cnt = cnt2;
+            }
+        }
+    };
+
+    sweepClusters(a, sList[w], batch);
     if (lane == 0 && tested) atomicAdd(a.work + 1, tested);
     kept = __reduce_add_sync(FULL, kept);
     if (lane == 0 && kept) atomicAdd(a.hdr + 2 * (a.height + 1), kept);
@@ -738,8 +953,13 @@ void launchKnnSweepBound(const KnnSweepArgs& a, cudaStream_t s) {
 void launchKnnSweepPoints(const KnnSweepArgs& a, cudaStream_t s) {
     withPadded(a.D, [&](auto dp) {
         constexpr int DP = decltype(dp)::value;
-        static const int grid = residentBlocks(reinterpret_cast<const void*>(knnSweepKernel<DP>), kSweepThreads);
-        knnSweepKernel<DP><<<grid, kSweepThreads, 0, s>>>(a);
+        void (*kern)(const KnnSweepArgs);
+        if constexpr (DP > 8)
+            kern = knnSweepMmaKernel<DP>;
+        else
+            kern = knnSweepKernel<DP>;
+        static const int grid = residentBlocks(reinterpret_cast<const void*>(kern), kSweepThreads);
+        kern<<<grid, kSweepThreads, 0, s>>>(a);
         TBLAEQ_LAUNCHED();
     });
 }

@@ -23,8 +23,8 @@
 //
 // Measured on B200 against the level-synchronous walk (beam, wave 1, node-major completion in two
 // refinement stages; about 90 launches), device time of one batch: 4,096 queries, K = 20 / 100, N = 10M,
-// D = 8: 11.4 -> 1.2 ms; 300 queries there: 3.0 -> 0.25 ms; one query: 0.38 -> 0.08 ms; 1,000 queries,
-// N = 5M, D = 16, scored: 40 -> 3.4 ms.
+// D = 8: 11.4 -> 1.09 ms; 300 queries there: 3.0 -> 0.23 ms; one query: 0.38 -> 0.08 ms; 1,000 queries,
+// N = 5M, D = 16, scored: 40 -> 2.2 ms.
 #pragma once
 
 #include <cstdint>
@@ -83,13 +83,11 @@ struct KnnSweepArgs {
     double* candD2;
     uint32_t beam;
     double waveFactor;      // wave scale / points per cluster (see BatchEngine::setWaveScale)
-    // Cluster-level probe entries for a scorer: entries [entOff[q], + entCnt[q]) of q, node and x.
+    // Cluster-level probe entries for a scorer: entries [entOff[q], + entCnt[q]) of query and node.
     uint32_t* entOff;
     uint32_t* entCnt;
     uint32_t* entQ;
     uint32_t* entNode;
-    double* entX;
-    const double* nodeX;    // FP64 centres of the finest clusters
     const double* score;
     uint32_t entCap;
     // Bit per (cluster, query of the block), `words` words a cluster.

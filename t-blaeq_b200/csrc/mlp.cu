@@ -246,19 +246,24 @@ struct FeatureSrc {
     // Frontier features: query point, cluster centre, subtree radius, level one-hot.
     const uint32_t* q;
     const uint32_t* node;
-    const double* x;
+    const double* x;            // centres: a row per entry, or per node (xByNode)
     const double* points;
     const NodeRec* nodes;
     uint32_t level;
     double inv;
+    bool xByNode;
     // Plain features: X[n][in].
     const float* X;
 };
 
+__device__ __forceinline__ const double* centreRow(const FeatureSrc& s, uint32_t e, int D) {
+    return s.x + static_cast<size_t>(s.xByNode ? s.node[e] : e) * D;
+}
+
 // Feature k (< in) of frontier entry e, as frontierFeaturesKernel builds it.
 __device__ __forceinline__ float frontierFeature(const FeatureSrc& s, uint32_t e, int k, int D) {
     if (k < D) return static_cast<float>(s.points[static_cast<size_t>(s.q[e]) * D + k] * s.inv);
-    if (k < 2 * D) return static_cast<float>(s.x[static_cast<size_t>(e) * D + (k - D)] * s.inv);
+    if (k < 2 * D) return static_cast<float>(centreRow(s, e, D)[k - D] * s.inv);
     if (k == 2 * D) return static_cast<float>(s.nodes[s.node[e]].rad * s.inv);
     return (k - 2 * D - 1 == static_cast<int>(s.level)) ? 1.f : 0.f;
 }
@@ -322,7 +327,7 @@ __global__ void __launch_bounds__(kTcRows) forwardTcKernel(const __nv_bfloat16* 
             // The entry's query point and centre are rows of D doubles: chunks of eight features
             // that lie inside one of them (D even) are read as four 16-byte loads.
             const double* pt = src.points + static_cast<size_t>(live ? src.q[e] : 0u) * D;
-            const double* xr = src.x + static_cast<size_t>(live ? e : 0u) * D;
+            const double* xr = centreRow(src, live ? e : 0u, D);
             const bool even = (D & 1) == 0;
             for (uint32_t k0 = 0; k0 < L.kp; k0 += 8) {
                 const int kb = static_cast<int>(k0);
@@ -580,13 +585,14 @@ void Mlp::launchTc(bool frontier, const void* srcPtr, const uint32_t* hdr, uint3
 }
 
 void Mlp::scoreFrontier(const FrontierIn& f, const uint32_t* node, uint32_t cap, const double* points,
-                        const NodeRec* nodes, uint32_t level, double invScale, double* score, cudaStream_t s) const {
-    FeatureSrc src{f.q, node, f.x, points, nodes, level, invScale, nullptr};
+                        const NodeRec* nodes, uint32_t level, double invScale, double* score, cudaStream_t s,
+                        const double* nodeX) const {
+    FeatureSrc src{f.q, node, f.x ? f.x : nodeX, points, nodes, level, invScale, f.x == nullptr, nullptr};
     launchTc(true, &src, f.hdr, 0, cap, score, s);
 }
 
 void Mlp::logitsTensor(const float* X, uint32_t n, float* z, cudaStream_t s) const {
-    FeatureSrc src{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0.0, X};
+    FeatureSrc src{nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0.0, false, X};
     launchTc(false, &src, nullptr, n, 0, z, s);
 }
 

@@ -66,8 +66,10 @@ public:
     // Scores the entries of a KNN frontier on the tensor cores: score[e] = -logit (ascending order =
     // most promising). Features are built in the kernel; both layers are tcgen05 BF16 MMAs with FP32
     // accumulation in tensor memory, so h1 is rounded to BF16 between the layers.
+    // (A frontier without coordinates of its own takes them from nodeX, the level's centres by node.)
     void scoreFrontier(const FrontierIn& f, const uint32_t* node, uint32_t cap, const double* points,
-                       const NodeRec* nodes, uint32_t level, double invScale, double* score, cudaStream_t s) const;
+                       const NodeRec* nodes, uint32_t level, double invScale, double* score, cudaStream_t s,
+                       const double* nodeX = nullptr) const;
 
     // Logits of n samples through the same tensor-core kernel as scoreFrontier.
     void logitsTensor(const float* X, uint32_t n, float* z, cudaStream_t s) const;

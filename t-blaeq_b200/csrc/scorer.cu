@@ -41,7 +41,7 @@ void scorerHook(void* ctx, const FrontierIn& f, const uint32_t* node, uint32_t c
     auto* rt = static_cast<Runtime*>(ctx);
     const uint32_t level = static_cast<uint32_t>(rt->dev->height - 2);
     rt->scorer->scoreFrontier(f, node, cap, points, rt->dev->nodeSub[level].as<NodeRec>(), level, rt->scorerInvScale,
-                              score, s);
+                              score, s, rt->dev->nodeX[level].as<double>());
 }
 
 // Device arrays that map a point id to its cluster in the finest cluster mesh (for labels).
