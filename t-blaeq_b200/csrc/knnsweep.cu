@@ -423,84 +423,197 @@ __global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(KnnSweepArgs a, 
         a.tau[q] = tau;
         a.tauF[q] = __double2float_ru(t);
         const double s = t * static_cast<double>(kRel);
-        a.thrF[q] = __double2float_ru(s * s);
+        a.thrF[q] = __double2float_ru(s * s + 1e-36);  // the least a float square can miss by underflow
     }
 }
 
 // ---- dense bound ----------------------------------------------------------------------------------
 constexpr int kBoundThreads = 256;
-constexpr int kBoundWords = 8;  // query words of one CTA
+constexpr int kBoundWords = 8;          // query words of one CTA
+constexpr float kFarthest = 1.2e19f;    // above every distance between coordinates of at most kSweepMaxAbs, D <= 32
+constexpr float kBoundSlack = 1.6e-5f;  // error of a bound product relative to |x|^2 + |p|^2 + r^2 + T^2, see below
 
-// One thread per cluster, its centre in registers; the block's queries (negated) come from shared
-// memory as broadcasts. Bound by the float pipe: D additions and multiply-adds per pair, packed two
-// to an instruction. 4,096 queries x 100,000 clusters, D = 8: 367 us (1.1e12 pairs/s); the walk's
-// bound levels, filters and transposes for the same queries took 3.4 ms.
+// d = a (16 x 8) * b (8 x 8) + c, TF32 operands (the low 13 bits of a float are not read), FP32 sums.
+__device__ __forceinline__ void mmaTf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1,
+                                       float c2, float c3) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
+}
+
+// x = hi + lo: TF32 operands whose sum keeps 21 bits of x.
+__device__ __forceinline__ float tf32Hi(float x) { return __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
+
+// 4 x 4 bytes across the four lanes of a quad: lane j gets byte j of lanes 0 .. 3, lane 0's lowest.
+__device__ __forceinline__ uint32_t quadTranspose(uint32_t v, int j) {
+    uint32_t o = __shfl_xor_sync(FULL, v, 1);
+    v = __byte_perm(v, o, (j & 1) ? 0x3715 : 0x6240);
+    o = __shfl_xor_sync(FULL, v, 2);
+    return __byte_perm(v, o, (j & 2) ? 0x3276 : 0x5410);
+}
+
+// Which queries' bounds T reach which clusters (centre x, radius r): |x - p| <= T + r, written as
+//     x.p + T r - (|x|^2 - r^2) / 2 - (|p|^2 - T^2) / 2 >= 0
+// with x and p relative to a centre of the CTA's clusters, so that one product per pair on the matrix
+// units remains, whose sign is the answer. Factors are split in two TF32 parts (hi hi + hi lo + lo hi);
+// an eighth-K step of its own carries T r and the two sums. With 21 bits a factor, products lose less
+// than 2^-18 of |x| |p| and T r, and the at most 13 steps' FP32 sums less than 2^-18 of all terms' sizes
+// (together under 8e-6 of |x|^2 + |p|^2 + r^2 + T^2); kBoundSlack, twice that, is added to the sums, so a
+// bit is only ever set too much (1e-35 covers what underflow loses). A warp holds 32 clusters as fragments and walks the CTA's queries, whose
+// fragments are split once into shared memory, in an order that leaves each lane whole bytes of the words.
+//
+// 4,096 queries x 100,000 clusters, D = 8: 166 us (2.5e12 pairs/s), bound by the rate of the warp-wide
+// products; as differences on the float pipe, a cluster per thread, 366 us, and 97 -> 48 us for 1,000 x
+// 50,000 at D = 16, 42 -> 22 us for 300 x 100,000 at D = 8. (The walk's bound levels,
+// filters and transposes took 3.4 ms for the first.)
 template <int DP>
-__global__ void __launch_bounds__(kBoundThreads) knnBoundBitsKernel(KnnSweepArgs a) {
-    __shared__ __align__(16) float sQ[kBoundWords * 32][DP];
-    __shared__ float sTau[kBoundWords * 32];
+__global__ void __launch_bounds__(kBoundThreads) knnBoundBitsKernel(const __grid_constant__ KnnSweepArgs a, uint32_t iters) {
+    constexpr int STEPS = (DP + 7) / 8;
+    constexpr int W = STEPS <= 2 ? kBoundWords : kBoundWords / 2;  // words staged at once (48 KB of shared memory)
+    __shared__ __align__(16) float4 sB[W][4][STEPS][32];  // hi, hi, lo, lo of a lane's two dimensions
+    __shared__ __align__(8) float2 sE[W][4][32];
     if (*a.status) return;
     const KnnSweepLevel& L = a.level[a.height - 2];
-    const uint32_t w0 = blockIdx.y * kBoundWords, w1 = min(a.words, w0 + kBoundWords);
-    const uint32_t nQ = (w1 - w0) * 32;
-    for (uint32_t i = threadIdx.x; i < nQ; i += kBoundThreads) {
-        const uint32_t q = a.qBegin + w0 * 32 + i;
-        const bool v = q < a.qEnd;
+    const uint32_t w0 = blockIdx.y * kBoundWords;
+    const uint32_t left = a.qEnd - a.qBegin > w0 * 32 ? a.qEnd - a.qBegin - w0 * 32 : 0u;  // queries from w0 on
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int quad = lane >> 2, j = lane & 3;
+    const uint32_t c0 = blockIdx.x * iters * kBoundThreads, c1 = min(L.count, c0 + iters * kBoundThreads);
+    // The CTA's centre: its first cluster's (the origin where an empty cluster has none).
+    auto centre = [&](int d) {
+        const float x = __ldg(L.x + static_cast<size_t>(c0) * DP + d);
+        return fabsf(x) <= static_cast<float>(kSweepMaxAbs) ? x : 0.f;
+    };
+
+    for (uint32_t wb = 0; wb < kBoundWords && wb * 32 < left; wb += W) {
+        if (wb) __syncthreads();
+        if (tid < W * 32) {
+            // Bit b, lane byte j and tile t of query i's place in its word: the accumulators' layout.
+            const uint32_t i = tid & 31, w = tid >> 5, t = (i >> 1) & 3, n = 2 * (i >> 3) + (i & 1);
+            const uint32_t at = (wb + w) * 32 + i;
+            const bool v = at < left;
+            const uint32_t q = a.qBegin + w0 * 32 + (v ? at : 0);
+            float n2 = 0.f;
 #pragma unroll
-        for (int d = 0; d < DP; ++d)
-            sQ[i][d] = v ? -a.qF[static_cast<size_t>(q) * DP + d] : -static_cast<float>(kSweepMaxAbs);
-        sTau[i] = v ? a.tauF[q] : 0.f;
-    }
-    __syncthreads();
-    const uint32_t c = blockIdx.x * kBoundThreads + threadIdx.x;
-    const bool valid = c < L.count && L.nodes[c].cnt > 0;
-    float2 x[DP / 2];
+            for (int s = 0; s < STEPS; ++s)
 #pragma unroll
-    for (int d = 0; d < DP / 2; ++d)
-        x[d] = valid ? __ldg(reinterpret_cast<const float2*>(L.x + static_cast<size_t>(c) * DP) + d) : make_float2(0.f, 0.f);
-    const float r = valid ? __ldg(L.rad + c) : -3e38f;
-    const uint32_t left = a.qEnd - a.qBegin > w0 * 32 ? a.qEnd - a.qBegin - w0 * 32 : 0u;  // queries of this CTA's words
-    uint32_t word[kBoundWords], any = 0;
+                for (int k = 0; k < 4; ++k) {
+                    float2 p = make_float2(0.f, 0.f);
+                    if (v && 8 * s + 2 * k < DP) {
+                        p = __ldg(reinterpret_cast<const float2*>(a.qF + static_cast<size_t>(q) * DP + 8 * s + 2 * k));
+                        p.x -= centre(8 * s + 2 * k);
+                        p.y -= centre(8 * s + 2 * k + 1);
+                    }
+                    n2 = fmaf(p.x, p.x, fmaf(p.y, p.y, n2));
+                    const float hx = tf32Hi(p.x), hy = tf32Hi(p.y);
+                    sB[w][t][s][n * 4 + k] = make_float4(hx, hy, p.x - hx, p.y - hy);
+                }
+            const float T = v ? fminf(a.tauF[q] * kRel, kFarthest) : 0.f;
+            const float sum = v ? 0.5f * (T * T - n2) + kBoundSlack * (T * T + n2) + 1e-35f : -1e38f;
+            const float hT = tf32Hi(T), hS = tf32Hi(sum);
+            sE[w][t][n * 4 + 0] = make_float2(hT, sum - hS);  // against r hi, 1
+            sE[w][t][n * 4 + 1] = make_float2(hT, 1.f);       // r lo, sum hi
+            sE[w][t][n * 4 + 2] = make_float2(T - hT, 1.f);   // r hi, sum lo
+            sE[w][t][n * 4 + 3] = make_float2(hS, 0.f);       // 1, 0
+        }
+        __syncthreads();
+        for (uint32_t it = 0; it < iters; ++it) {
+            const uint32_t base = c0 + it * kBoundThreads + warp * 32;
+            if (base >= c1) break;  // warp-uniform
+            uint32_t hi[2][STEPS][4], lo[2][STEPS][4], ext[2][4];
 #pragma unroll
-    for (int w = 0; w < kBoundWords; ++w) {
-        word[w] = 0;
-        if (static_cast<uint32_t>(w) * 32 >= left) continue;
-        const uint32_t n = min(32u, left - w * 32);
-#pragma unroll 4
-        for (uint32_t j = 0; j < n; ++j) {
-            const uint32_t i = w * 32 + j;
-            float2 s = make_float2(0.f, 0.f);
+            for (int h = 0; h < 4; ++h) {
+                const uint32_t c = base + quad + 8 * h;
+                const bool v = c < c1 && L.nodes[c].cnt > 0;
+                const int m = h >> 1, e = h & 1;
+                float n2 = 0.f;
 #pragma unroll
-            for (int d = 0; d < DP / 2; d += 2) {
-                const float4 nq = *reinterpret_cast<const float4*>(&sQ[i][2 * d]);
-                const float2 e = __fadd2_rn(x[d], make_float2(nq.x, nq.y));
-                const float2 f = __fadd2_rn(x[d + 1], make_float2(nq.z, nq.w));
-                s = __ffma2_rn(e, e, s);
-                s = __ffma2_rn(f, f, s);
+                for (int s = 0; s < STEPS; ++s) {
+                    float2 x = make_float2(0.f, 0.f);
+                    if (v && 8 * s + 2 * j < DP) {
+                        x = __ldg(reinterpret_cast<const float2*>(L.x + static_cast<size_t>(c) * DP + 8 * s + 2 * j));
+                        x.x -= centre(8 * s + 2 * j);
+                        x.y -= centre(8 * s + 2 * j + 1);
+                    }
+                    n2 = fmaf(x.x, x.x, fmaf(x.y, x.y, n2));
+                    const float hx = tf32Hi(x.x), hy = tf32Hi(x.y);
+                    hi[m][s][e] = __float_as_uint(hx);
+                    hi[m][s][2 + e] = __float_as_uint(hy);
+                    lo[m][s][e] = __float_as_uint(x.x - hx);
+                    lo[m][s][2 + e] = __float_as_uint(x.y - hy);
+                }
+                n2 += __shfl_xor_sync(FULL, n2, 1);
+                n2 += __shfl_xor_sync(FULL, n2, 2);
+                const float r = v ? __ldg(L.rad + c) * kRel : 0.f;
+                const float sum = 0.5f * (r * r - n2) + kBoundSlack * (r * r + n2);
+                const float hR = tf32Hi(r), hS = tf32Hi(sum);
+                ext[m][e] = __float_as_uint(j == 1 ? r - hR : j == 3 ? 1.f : hR);
+                ext[m][2 + e] = __float_as_uint(j == 0 ? 1.f : j == 1 ? hS : j == 2 ? sum - hS : 0.f);
             }
-            const float t = (sTau[i] + r) * kRel;
-            if (s.x + s.y <= t * t) word[w] |= 1u << j;
-        }
-        if (!valid) word[w] = 0;
-        any |= word[w];
-    }
-    if (c < L.count) {
-        uint32_t* out = a.bits + static_cast<size_t>(c) * a.words + w0;
-        if (a.words == 1) {
-            out[0] = word[0];
-        } else {  // rows of a multiple of four words
-            *reinterpret_cast<uint4*>(out) = make_uint4(word[0], word[1], word[2], word[3]);
-            if (w0 + 4 < a.words) *reinterpret_cast<uint4*>(out + 4) = make_uint4(word[4], word[5], word[6], word[7]);
-        }
-    }
-    if (gridDim.y == 1) {
-        const uint32_t b = __ballot_sync(FULL, any != 0);
-        if (b) {
-            const int lane = threadIdx.x & 31;
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(a.liveCnt, __popc(b));
-            base = __shfl_sync(FULL, base, 0);
-            if (any) a.live[base + __popc(b & ((1u << lane) - 1u))] = c;
+            const uint32_t c = base + quad + 8 * j;  // the cluster whose words this lane ends up with
+            const bool valid = c < c1 && L.nodes[c].cnt > 0;
+            uint32_t word[W], any = 0;
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                word[w] = 0;
+                if ((wb + w) * 32 >= left) continue;  // uniform
+                uint32_t far[4] = {0u, 0u, 0u, 0u};  // signs, a byte of the word per cluster row
+#pragma unroll
+                for (int t = 3; t >= 0; --t) {
+                    float d[2][4];
+                    const float2 e = sE[w][t][lane];
+#pragma unroll
+                    for (int m = 0; m < 2; ++m)
+                        mmaTf32(d[m], ext[m], __float_as_uint(e.x), __float_as_uint(e.y), 0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int s = 0; s < STEPS; ++s) {
+                        const float4 b = sB[w][t][s][lane];
+                        const uint32_t bx = __float_as_uint(b.x), by = __float_as_uint(b.y);
+                        const uint32_t bz = __float_as_uint(b.z), bw = __float_as_uint(b.w);
+#pragma unroll
+                        for (int m = 0; m < 2; ++m) {
+                            mmaTf32(d[m], lo[m][s], bx, by, d[m][0], d[m][1], d[m][2], d[m][3]);
+                            mmaTf32(d[m], hi[m][s], bz, bw, d[m][0], d[m][1], d[m][2], d[m][3]);
+                            mmaTf32(d[m], hi[m][s], bx, by, d[m][0], d[m][1], d[m][2], d[m][3]);
+                        }
+                    }
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        far[h] = __funnelshift_l(__float_as_uint(d[h >> 1][2 * (h & 1) + 1]), far[h], 1);
+                        far[h] = __funnelshift_l(__float_as_uint(d[h >> 1][2 * (h & 1)]), far[h], 1);
+                    }
+                }
+                const uint32_t bytes = __byte_perm(__byte_perm(far[0], far[1], 0x0040), __byte_perm(far[2], far[3], 0x0040), 0x5410);
+                const uint32_t near = quadTranspose(~bytes, j);
+                word[w] = valid ? near : 0u;
+                any |= word[w];
+            }
+            if (c < c1) {
+                uint32_t* out = a.bits + static_cast<size_t>(c) * a.words + w0 + wb;
+                if (a.words == 1) {
+                    out[0] = word[0];
+                } else {  // rows of a multiple of four words
+#pragma unroll
+                    for (int w = 0; w < W; w += 4)
+                        if (w0 + wb + w < a.words) *reinterpret_cast<uint4*>(out + w) = make_uint4(word[w], word[w + 1], word[w + 2], word[w + 3]);
+                }
+            }
+            if (gridDim.y == 1) {
+                // Listed when the first queries that reach it are found: with the words in two turns, the second
+                // turn lists what the first left out.
+                const bool seen = wb && valid && a.words > 1 &&
+                                  [&] {
+                                      const uint4 f = *reinterpret_cast<const uint4*>(a.bits + static_cast<size_t>(c) * a.words);
+                                      return (f.x | f.y | f.z | f.w) != 0;
+                                  }();
+                const uint32_t b = __ballot_sync(FULL, any != 0 && !seen);
+                if (b) {
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(a.liveCnt, __popc(b));
+                    at = __shfl_sync(FULL, at, 0);
+                    if (any != 0 && !seen) a.live[at + __popc(b & ((1u << lane) - 1u))] = c;
+                }
+            }
         }
     }
 }
@@ -709,14 +822,6 @@ __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(const __grid_con
     if (lane == 0 && tested) atomicAdd(a.work + 1, tested);
     kept = __reduce_add_sync(FULL, kept);
     if (lane == 0 && kept) atomicAdd(a.hdr + 2 * (a.height + 1), kept);
-}
-
-// d = a (16 x 8) * b (8 x 8) + c, TF32 operands (the low 13 bits of a float are not read), FP32 sums.
-__device__ __forceinline__ void mmaTf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c0, float c1,
-                                       float c2, float c3) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 
 // One warp per cluster: its queries, 32 at a time, against its points, 16 at a time, as a product on the
@@ -942,10 +1047,14 @@ void launchKnnProbe(const KnnSweepArgs& a, KnnProbePhase phase, cudaStream_t s) 
 }
 
 void launchKnnSweepBound(const KnnSweepArgs& a, cudaStream_t s) {
-    const dim3 grid((a.level[a.height - 2].count + kBoundThreads - 1) / kBoundThreads,
-                    (a.words + kBoundWords - 1) / kBoundWords);
+    // 256 clusters a turn, and up to eight turns a CTA while a few CTAs per SM remain: a CTA's queries are
+    // split once, which is a fifth of a single turn.
+    const uint32_t turns = (a.level[a.height - 2].count + kBoundThreads - 1) / kBoundThreads;
+    const uint32_t gy = (a.words + kBoundWords - 1) / kBoundWords;
+    const uint32_t iters = std::max<uint32_t>(1, std::min<uint64_t>(8, static_cast<uint64_t>(turns) * gy / (148 * 8)));
+    const dim3 grid((turns + iters - 1) / iters, gy);
     withPadded(a.D, [&](auto dp) {
-        knnBoundBitsKernel<decltype(dp)::value><<<grid, kBoundThreads, 0, s>>>(a);
+        knnBoundBitsKernel<decltype(dp)::value><<<grid, kBoundThreads, 0, s>>>(a, iters);
         TBLAEQ_LAUNCHED();
     });
 }

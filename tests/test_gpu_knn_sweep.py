@@ -81,3 +81,17 @@ def test_equal_distances_grow_the_candidates(tb, oracle_mod, cuda):
     pts, ids = h.decode_points(np.arange(6000))
     P = np.ascontiguousarray(np.repeat(np.array([[7.0, 7.0, 7.0, 7.0]]), 33, axis=0))
     _check(tb, oracle_mod, h, pts, ids, P, 12)
+
+
+@pytest.mark.parametrize("D,nq", [(4, 33), (12, 128), (20, 130), (28, 257)])
+@pytest.mark.parametrize("offset,scale", [(0.0, 1e-12), (3e4, 1.0), (-2e6, 1e3)])
+def test_bound_products_far_from_the_origin(tb, oracle_mod, cuda, D, nq, offset, scale):
+    """Two clouds far apart, both far from the origin or tiny: the bound's products must lose no cluster."""
+    rng = np.random.default_rng(D + nq)
+    X = rng.normal(0, scale, (6000, D)) + offset
+    X[3000:] += 40 * scale
+    h, _ = tb.QueryHandler.build(X.astype(np.float32), height=3, ratios=(20, 10), iters=3, seed=1)
+    h.prepare_for_query(tb.LevelPolicy.L0)
+    pts, ids = h.decode_points(np.arange(6000))
+    P = np.ascontiguousarray(pts[rng.integers(0, 6000, nq)] + rng.normal(0, 0.3 * scale, (nq, D)))
+    _check(tb, oracle_mod, h, pts, ids, P, 9)
