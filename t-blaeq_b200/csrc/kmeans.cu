@@ -120,8 +120,14 @@ __global__ void packCentroidsKernel(const float* C, uint64_t k, uint64_t kPad, i
 // each tile into one of two tensor-memory accumulators. Eight consumer warps reduce: warps w and
 // w+4 read TMEM lane quarter w (point rows 32w..32w+31), each half of the columns, and keep the two
 // smallest ||c||^2 - 2 x.c (the two nearest centroids): per 32-column chunk one fused multiply-add
-// and one min per value, and the top-2 update only when a lane's chunk minimum beats its current
-// second best (rare once the first tiles have passed). Hand-offs are mbarriers: a stage is
+// and one min per value, and the top-2 update only for the eight columns whose minimum beats a lane's
+// current second best. Started from nothing that is nearly every chunk of a warp (a row improves some
+// 15 times over 10,000 centroids in its half, a warp has 32 rows), so from the second iteration on a row starts
+// just above what the pair kept for it in the last iteration reaches against the moved centroids (startBound):
+// the two smallest lie below, and few others do. 1M points x 10,000 centroids, D = 16: 3.50 -> 2.35 ms
+// an iteration (2.6 ms for the first), bound by the updates before and now by the latency of a
+// consumer's tile (tensor-memory load, norms, minima; an instruction in 42% of the issue slots).
+// Hand-offs are mbarriers: a stage is
 // "full" when its copy lands, an accumulator "done" when its MMAs commit, and both are "free"
 // again once all eight consumer warps have arrived; no CTA-wide barrier runs per tile. The two
 // column halves merge through shared memory at the end, and an FP64 step then picks between the
@@ -143,9 +149,31 @@ __device__ __forceinline__ void keepTwo(float v, uint32_t i, float& s1, uint32_t
     }
 }
 
+// A value above both ||c||^2 - 2 x.c of the pair (a, b) as the tensor cores compute them, or infinity where
+// there is none (one centroid, values that are not finite). Three TF32 products leave out at most
+// 2.4e-6 |x| |c|, and their 48 FP32 sums round within 1.2e-5 |x| |c|; 2e-5 (|x|^2 + |c|^2) covers both and
+// the sums here.
+__device__ __forceinline__ float startBound(const float* x, const float* C, int D, uint2 pair) {
+    if (pair.x == pair.y) return INFINITY;
+    const float* a = C + static_cast<uint64_t>(pair.x) * D;
+    const float* b = C + static_cast<uint64_t>(pair.y) * D;
+    float xx = 0.f, aa = 0.f, bb = 0.f, xa = 0.f, xb = 0.f;
+    for (int d = 0; d < D; ++d) {
+        const float v = __ldg(x + d), u = __ldg(a + d), w = __ldg(b + d);
+        xx = fmaf(v, v, xx);
+        aa = fmaf(u, u, aa);
+        bb = fmaf(w, w, bb);
+        xa = fmaf(v, u, xa);
+        xb = fmaf(v, w, xb);
+    }
+    const float bound = fmaxf(aa - 2.f * xa, bb - 2.f * xb) + (2e-5f * (xx + fmaxf(aa, bb)) + 1e-30f);
+    return fabsf(bound) <= 3e38f && xx + aa + bb <= 3e38f ? bound : INFINITY;
+}
+
+// cand is read before it is written when `started` (a row's own pair of the last iteration).
 __global__ void __launch_bounds__(kAssignThreads, 2)
-    assignTcKernel(const uint8_t* points, const uint8_t* cents, uint64_t n, uint32_t nTiles, uint2* cand,
-                   uint32_t* status) {
+    assignTcKernel(const uint8_t* points, const uint8_t* cents, uint64_t n, uint32_t nTiles, const float* X,
+                   const float* C, int D, int started, uint2* cand, uint32_t* status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sA = smem;
     uint8_t* sB = smem + kPointTileBytes;  // kStages stages of kCentTileBytes
@@ -237,6 +265,13 @@ __global__ void __launch_bounds__(kAssignThreads, 2)
         }
     } else {
         const uint32_t rowBase = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        {
+            const uint64_t p = tile * kTileM + static_cast<uint64_t>((warp & 3) * 32 + lane);
+            if (p >= n)
+                s1 = s2 = -INFINITY;  // a row of the tile's padding
+            else if (started)
+                s1 = s2 = startBound(X + p * D, C, D, cand[p]);
+        }
         for (uint32_t t = 0; t < nTiles; ++t) {
             const uint32_t b = t & 1u, st = t % kStages;
             if (!mbarWait(&mmaDone[b], (t >> 1) & 1u) || *sAbort) {
@@ -255,7 +290,7 @@ __global__ void __launch_bounds__(kAssignThreads, 2)
                 uint32_t r[32];
                 tmemLoad32(base + static_cast<uint32_t>(c), r);
                 tmemWaitLoad();
-                float m0 = INFINITY, m1 = INFINITY;
+                float m[4];  // of eight columns each
 #pragma unroll
                 for (int j = 0; j < 32; j += 4) {
                     // ||c||^2 - 2 x.c for four columns: two packed FMAs, two three-input minima
@@ -269,12 +304,17 @@ __global__ void __launch_bounds__(kAssignThreads, 2)
                     r[j + 1] = __float_as_uint(va.y);
                     r[j + 2] = __float_as_uint(vb.x);
                     r[j + 3] = __float_as_uint(vb.y);
-                    m0 = min3f(m0, va.x, va.y);
-                    m1 = min3f(m1, vb.x, vb.y);
+                    const float lo = (j & 4) ? min3f(m[j >> 3], va.x, va.y) : fminf(va.x, va.y);
+                    m[j >> 3] = min3f(lo, vb.x, vb.y);
                 }
-                if (fminf(m0, m1) < s2) {
+                if (min3f(fminf(m[0], m[1]), m[2], m[3]) < s2) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) keepTwo(__uint_as_float(r[j]), col0 + c + j, s1, i1, s2, i2);
+                    for (int g = 0; g < 4; ++g) {
+                        if (!(m[g] < s2)) continue;
+#pragma unroll
+                        for (int j = 8 * g; j < 8 * g + 8; ++j)
+                            keepTwo(__uint_as_float(r[j]), col0 + c + j, s1, i1, s2, i2);
+                    }
                 }
             }
             tcFenceBefore();
@@ -629,8 +669,8 @@ void kmeansRun(const float* dX, uint64_t n, uint64_t D, uint64_t k, const Kmeans
                                                                               packedC.as<uint8_t>());
             TBLAEQ_LAUNCHED();
             assignTcKernel<<<static_cast<unsigned>(nTilesP), kAssignThreads, kAssignSmem, s>>>(
-                packedP.as<uint8_t>(), packedC.as<uint8_t>(), n, static_cast<uint32_t>(nTilesC), cand.as<uint2>(),
-                status.as<uint32_t>());
+                packedP.as<uint8_t>(), packedC.as<uint8_t>(), n, static_cast<uint32_t>(nTilesC), dX,
+                centroids.as<float>(), Di, it > 0, cand.as<uint2>(), status.as<uint32_t>());
             TBLAEQ_LAUNCHED();
             refineKernel<<<gridFor(n, 256), 256, 0, s>>>(dX, cand.as<uint2>(), Cd.as<double>(), n, Di,
                                                          labels.as<uint32_t>());
