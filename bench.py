@@ -496,8 +496,19 @@ def main():
     achieved = alg_bytes / final_mean_s / 1e9
     per_level = [{"level": m, "ms": level_ms[m], "algorithmic_bytes": level_bytes(m),
                   "GB/s": level_bytes(m) / (level_ms[m] / 1e3) / 1e9} for m in range(H)]
+    # Fewer kernels than levels: the batch ran as one sweep, which reads the boxes and, once each, the
+    # nodes above the clusters and the clusters' grid boxes (4·D), then the boxes and records of the
+    # groups it tests and the points of those it keeps, and writes the results and their offsets.
+    sweep = 0 < graph["kernels"] < H
+    if sweep:
+        alg_bytes = (args.nq * 16 * D + sum(mesh_nodes[:H - 2]) * (8 * D + 16) + mesh_nodes[H - 2] * 4 * D
+                     + groups["groups"] * (8 * D + 16) + groups["points"] * 4 * D + results * 8 + (args.nq + 1) * 8)
+        achieved = alg_bytes / final_mean_s / 1e9
+        per_level = [{"level": "sweep over all levels", "ms": level_ms[dom], "algorithmic_bytes": alg_bytes,
+                      "GB/s": achieved}]
     dom_kind = (["direct", "staged", "node-major"][variants[dom]] if dom < len(variants) else "direct")
-    dom_name = ("finest level: point groups + float points" if dom == H - 1 and groups["groups"]
+    dom_name = ("range sweep (upper, sweep, gather)" if sweep
+                else "finest level: point groups + float points" if dom == H - 1 and groups["groups"]
                 else "finest level" if dom == H - 1 else f"level {dom} (mesh {dom - 1} -> mesh {dom}), {dom_kind}")
 
     # Plain: one query at a time through the same engine (no batching, no graph).
@@ -643,7 +654,7 @@ def main():
         "roofline": {"bound": "host link" if finest_streamed else "hbm", "achieved": achieved,
                      "peak": None if finest_streamed else peak, "unit": "GB/s",
                      "frac": None if finest_streamed else achieved / peak,
-                     "traffic": None if finest_streamed else profiled_traffic(cfg_name, args.nq, dom, H),
+                     "traffic": None if finest_streamed or sweep else profiled_traffic(cfg_name, args.nq, dom, H),
                      "kernel": dom_name,
                      "peak_kind": f"{peak_kind} hbm_gbs", "algorithmic_bytes_per_launch": alg_bytes,
                      "launch_ms": final_mean_s * 1e3, "per_level": per_level, "point_groups": groups},

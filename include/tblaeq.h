@@ -193,7 +193,8 @@ void* tblaeq_stream(tblaeq_handle* h);
 int tblaeq_set_timing(tblaeq_handle* h, int on);
 
 /* Elapsed milliseconds per stage of the last batch: [0] workspace reset + root frontier,
- * [1..height] one per mesh expand (the last one is the finest level), [height+1] result offsets.
+ * [1..height] one per mesh expand (the last one is the finest level), [height+1] result offsets. A
+ * sweep (exact batches with default options) reports its whole time at the finest level.
  * Returns the number of stages written (at most cap), or -1 when timing is off. */
 int tblaeq_stage_times(tblaeq_handle* h, float* ms, int cap);
 

@@ -619,9 +619,13 @@ void BatchEngine::enqueueRangeSweep(const double* dBoxes, uint32_t nq, unsigned 
     a.ids = resIds_.as<uint64_t>();
     a.vals = (flags & kWantVals) ? resVals_.as<double>() : nullptr;
     a.resultCap = static_cast<uint32_t>(caps_.results);
-    launchRangeSweep(a, stream_);
     if (timing_)
-        for (int m = 0; m <= H; ++m) record(2 + m);
+        for (int m = 0; m + 1 < H; ++m) record(2 + m);
+    launchRangeSweep(a, stream_);
+    if (timing_) {  // all of it in the last mesh's stage
+        record(1 + H);
+        record(2 + H);
+    }
 }
 
 void BatchEngine::enqueueLaunches(const double* dBoxes, uint32_t nq, int mode, unsigned flags) {

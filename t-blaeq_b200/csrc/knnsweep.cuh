@@ -4,19 +4,20 @@
 // the query is within a few percent of the true K-th distance (measured over the synthetic indexes,
 // D = 3..16, K = 10..100: 1.00-1.06 of it with 17 clusters), so one bound per query, taken from them,
 // leaves almost nothing for a second one to prune. (2) Testing every (query, cluster) pair against
-// that bound is cheap when it is dense: a centre stays in a thread's registers, the queries come
-// from shared memory, and the pair costs 2 D float operations and no list, sort or atomic.
+// that bound is cheap when it is dense: a pair is one product on the matrix units, with no list, sort
+// or atomic.
 //
 //   probe   one CTA per query walks down from the root with a beam, takes the points of its
 //           best-ranked clusters and selects their K-th distance (tau);
-//   bound   one thread per cluster tests all queries of a block: bit (cluster, query) = the
-//           cluster's sphere reaches within tau of the query;
+//   bound   a warp holds 32 clusters and walks 256 queries: bit (cluster, query) = the cluster's
+//           sphere reaches within tau of the query;
 //   sweep   one warp per cluster gathers the queries whose bit is set, 32 at a time, tests them
 //           against the cluster's point groups (boxes), and the groups' points against the queries
-//           whose box test passed, one point per lane;
+//           whose box test passed, one point per lane, or above eight dimensions against all 32 as
+//           a product;
 //   finish  per query, the K smallest candidates by (FP64 squared distance, id).
 //
-// The tests run in single precision with a margin that covers every rounding (queryMargin in
+// The tests run in single precision with a margin that covers every rounding (sweepPrepareKernel in
 // knnsweep.cu), so they only ever let too much through; a point that passes is measured in FP64 from
 // the decoded coordinates (fma in dimension order) before it becomes a candidate. The candidates
 // are therefore exactly the points whose FP64 squared distance lies within tau^2 (1 + 1e-9).
