@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(1024) sweepPrepareKernel(KnnSweepArgs a, uint3
 // ---- probe ----------------------------------------------------------------------------------------
 constexpr int kProbeThreads = 256;
 constexpr int kProbeWarps = kProbeThreads / 32;
+constexpr uint32_t kProbeBins = 2048;  // of an 11-bit digit
 
 __device__ __forceinline__ uint64_t shflXor64(uint64_t v, int o) { return __shfl_xor_sync(FULL, v, o); }
 
@@ -166,15 +167,18 @@ __device__ __forceinline__ double pointDist2(const double* p, const double* y, i
 }
 
 // One CTA per query. Every warp keeps the 32 best of the nodes it ranked in registers; the eight lists
-// merge through shared memory once per level. The chain of levels is what bounds it (a few thousand
-// nodes and points per query, latency between the levels), so each CTA is small and several share
-// an SM: 252 us for 4,096 queries (N = 10M, D = 8), 39 us for one.
+// merge through shared memory, pairwise, once per level. The chain of levels is what bounds it (a few
+// thousand nodes and points per query, latency between the levels; an instruction in 55% of the issue
+// slots at five CTAs an SM, and six with fewer registers measured 234 us), so each CTA is small. 4,096
+// queries (N = 10M, D = 8): 226 us, 28 us for one; 250 and 31 us while every point searched its range, a
+// warp merged all lists in turn and the selection counted four eight-bit digits.
 template <int DP>
-__global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(KnnSweepArgs a, int phase) {
+__global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(const __grid_constant__ KnnSweepArgs a, int phase) {
     __shared__ uint64_t sMerge[kProbeWarps][32];
     __shared__ uint32_t sBeg[32], sPre[33];
     __shared__ float sKeys[kProbePoints];
-    __shared__ uint32_t sHist[256];
+    __shared__ __align__(16) uint32_t sHist[kProbeBins];
+    __shared__ uint32_t sWarp[kProbeWarps];
     __shared__ uint32_t sSel[2], sTauUb;
     __shared__ uint64_t sScored[32];
     const uint32_t q = blockIdx.x;
@@ -224,11 +228,14 @@ __global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(KnnSweepArgs a, 
         }
         sMerge[warp][lane] = best.best;
         __syncthreads();
-        if (warp == 0) {
-            for (int w = 1; w < kProbeWarps; ++w) best.merge(sMerge[w][lane], lane);
-            sMerge[0][lane] = best.best;
+#pragma unroll
+        for (int half = kProbeWarps / 2; half > 0; half >>= 1) {
+            if (warp < half) {
+                best.merge(sMerge[warp + half][lane], lane);
+                sMerge[warp][lane] = best.best;
+            }
+            __syncthreads();
         }
-        __syncthreads();
     };
     // Node j of mesh m: its centre's distance, less the subtree radius (the sphere's lower bound) when
     // bySphere. A node with K points below it bounds the K-th distance by its far side.
@@ -366,49 +373,62 @@ __global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(KnnSweepArgs a, 
         atomicAdd(a.hdr + 2 * H, n);
         atomicAdd(a.work, static_cast<unsigned long long>(n));
     }
-    for (uint32_t i = tid; i < n; i += kProbeThreads)
-        sKeys[i] = rowDist2<DP>(p, a.pointsF + static_cast<size_t>(itemOf(i)) * DP);
-    if (tid == 0) {
-        sSel[0] = 0;  // prefix chosen so far
-        sSel[1] = K;  // rank within it
+    // A warp per range of rows (a cluster or a group), four rows of a lane in flight.
+    for (uint32_t r = warp; r < nList; r += kProbeWarps) {
+        const uint32_t at = sPre[r];
+        if (at >= n) break;
+        const uint32_t cnt = min(sPre[r + 1], n) - at;
+        const float* rowsF = a.pointsF + static_cast<size_t>(sBeg[r]) * DP;
+#pragma unroll 4
+        for (uint32_t i = lane; i < cnt; i += 32) sKeys[at + i] = rowDist2<DP>(p, rowsF + static_cast<size_t>(i) * DP);
     }
-    __syncthreads();
+    if (tid == 0) {
+        sSel[0] = 0;  // digits chosen so far
+        sSel[1] = K;  // rank among the keys that have them
+    }
+    // A bound just above the K-th smallest: the upper 22 bits of its key (2^-14 of the squared distance),
+    // by two counts of 11-bit digits (non-negative floats order like integers). Eight-bit digits put
+    // nearly all keys of the first count into one or two bins, whose atomics then queue up.
     if (n >= K) {
-        // Radix selection over the keys' bits (non-negative floats order like integers).
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            sHist[tid] = 0;
+        for (int shift = 20; shift >= 9; shift -= 11) {
+            for (uint32_t i = tid; i < kProbeBins / 4; i += kProbeThreads)
+                reinterpret_cast<uint4*>(sHist)[i] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
-            const uint32_t prefix = sSel[0], mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
+            const uint32_t chosen = sSel[0], need = sSel[1];
             for (uint32_t i = tid; i < n; i += kProbeThreads) {
                 const uint32_t key = __float_as_uint(sKeys[i]);
-                if ((key & mask) == prefix) atomicAdd(&sHist[(key >> shift) & 255u], 1u);
+                if (shift == 20 || (key >> 20) == chosen) atomicAdd(&sHist[(key >> shift) & (kProbeBins - 1)], 1u);
             }
             __syncthreads();
-            if (warp == 0) {
-                uint32_t c[8], sum = 0;
+            constexpr int kOwn = kProbeBins / kProbeThreads;
+            uint32_t c[kOwn], sum = 0;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    c[i] = sHist[lane * 8 + i];
-                    sum += c[i];
-                }
-                uint32_t inc = sum;
+            for (int i = 0; i < kOwn; i += 4) {
+                const uint4 h = *reinterpret_cast<const uint4*>(&sHist[tid * kOwn + i]);
+                c[i] = h.x;
+                c[i + 1] = h.y;
+                c[i + 2] = h.z;
+                c[i + 3] = h.w;
+                sum += h.x + h.y + h.z + h.w;
+            }
+            uint32_t inc = sum;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t t = __shfl_up_sync(FULL, inc, o);
-                    if (lane >= o) inc += t;
-                }
-                const uint32_t need = sSel[1];
-                __syncwarp();
-                uint32_t before = inc - sum;
-                if (before < need && need <= inc) {
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += t;
+            }
+            if (lane == 31) sWarp[warp] = inc;
+            __syncthreads();
+            for (int w = 0; w < warp; ++w) inc += sWarp[w];
+            uint32_t before = inc - sum;
+            if (before < need && need <= inc) {  // one thread
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        if (before < need && need <= before + c[i]) {
-                            sSel[0] = prefix | (static_cast<uint32_t>(lane * 8 + i) << shift);
-                            sSel[1] = need - before;
-                        }
-                        before += c[i];
+                for (int i = 0; i < kOwn; ++i) {
+                    if (before < need && need <= before + c[i]) {
+                        sSel[0] = (chosen << 11) | static_cast<uint32_t>(tid * kOwn + i);
+                        sSel[1] = need - before;
                     }
+                    before += c[i];
                 }
             }
             __syncthreads();
@@ -417,7 +437,7 @@ __global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(KnnSweepArgs a, 
     if (tid == 0) {
         double tau = static_cast<double>(__uint_as_float(sTauUb));
         if (n >= K)
-            tau = fmin(tau, sqrt(static_cast<double>(__uint_as_float(sSel[0]))) * static_cast<double>(kRel) +
+            tau = fmin(tau, sqrt(static_cast<double>(__uint_as_float((sSel[0] << 9) | 0x1ffu))) * static_cast<double>(kRel) +
                                 static_cast<double>(margin));
         const double t = (tau + static_cast<double>(margin)) * (1.0 + 1e-7);
         a.tau[q] = tau;

@@ -24,7 +24,7 @@
 //
 // Measured on B200 against the level-synchronous walk (beam, wave 1, node-major completion in two
 // refinement stages; about 90 launches), device time of one batch: 4,096 queries, K = 20 / 100, N = 10M,
-// D = 8: 11.4 -> 0.89 ms; 300 queries there: 3.0 -> 0.21 ms; one query: 0.38 -> 0.08 ms; 1,000 queries,
+// D = 8: 11.4 -> 0.86 ms; 300 queries there: 3.0 -> 0.20 ms; one query: 0.38 -> 0.08 ms; 1,000 queries,
 // N = 5M, D = 16, scored: 40 -> 2.15 ms.
 #pragma once
 
