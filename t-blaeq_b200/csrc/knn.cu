@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(1024) stepKernel(const uint64_t* keys, const u
 }
 
 constexpr int kTopKStage = 4096;  // candidates a CTA sorts in shared memory
-constexpr uint64_t kTopKCount = 512;  // candidates a CTA places by counting (one per thread)
+constexpr uint64_t kTopKCount = 512;  // candidates a CTA places by counting
 
 // The double of an orderKey.
 __device__ __forceinline__ double keyValue(uint64_t b) {
@@ -195,60 +195,101 @@ __device__ __forceinline__ double keyValue(uint64_t b) {
     return __longlong_as_double(static_cast<long long>(b));
 }
 
-__global__ void __launch_bounds__(512) topKKernel(const uint64_t* offA, const uint64_t* idsA, const double* d2A,
-                                                  uint64_t capA, const uint64_t* offB, const uint64_t* idsB,
-                                                  const double* d2B, uint64_t capB, const uint32_t* Kq,
-                                                  const uint64_t* outOff, uint64_t* outIds, double* outD2,
-                                                  uint32_t* outCount, uint32_t* status, const uint32_t* cntA) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t* sk = reinterpret_cast<uint64_t*>(smem);
-    uint64_t* sv = sk + kTopKStage;
-    const uint32_t q = blockIdx.x;
-    const uint64_t a0 = offA[q], slots = offA[q + 1] - a0;
-    const uint64_t na = cntA ? std::min<uint64_t>(cntA[q], slots) : slots;
-    const uint64_t b0 = offB ? offB[q] : 0, nb = offB ? offB[q + 1] - b0 : 0;
-    const uint64_t n = na + nb;
-    const uint32_t K = Kq[q];
-    // Candidates beyond the arrays mean the producer overflowed: never read them.
-    if (a0 + na > capA || (offB && b0 + nb > capB)) {
-        if (threadIdx.x == 0) {
-            if (outCount) outCount[q] = 0;
-            atomicOr(status, kStatusOverflowEntries);
-        }
-        return;
+constexpr int kTopKThreads = 512;
+constexpr int kTopKSmallThreads = 128;
+constexpr uint64_t kTopKSmall = 256;  // candidates a CTA of kTopKSmallThreads places
+constexpr uint32_t kTopKResident = 148 * 3;  // CTAs of kTopKThreads resident at once (the stage)
+
+struct TopKArgs {
+    const uint64_t* offA;
+    const uint64_t* idsA;
+    const double* d2A;
+    uint64_t capA;
+    const uint64_t* offB;
+    const uint64_t* idsB;
+    const double* d2B;
+    uint64_t capB;
+    const uint32_t* Kq;
+    const uint64_t* outOff;
+    uint64_t* outIds;
+    double* outD2;
+    uint32_t* outCount;
+    uint32_t* status;
+    const uint32_t* cntA;
+};
+
+// Candidates of one query: list A (cntA of its slots, when given), then list B.
+struct TopKList {
+    uint64_t a0, na, b0, n, keep;
+    bool usable;  // candidates beyond the arrays mean the producer overflowed: never read them
+    __device__ __forceinline__ TopKList(const TopKArgs& a, uint32_t q) {
+        a0 = a.offA[q];
+        const uint64_t slots = a.offA[q + 1] - a0;
+        na = a.cntA ? std::min<uint64_t>(a.cntA[q], slots) : slots;
+        b0 = a.offB ? a.offB[q] : 0;
+        const uint64_t nb = a.offB ? a.offB[q + 1] - b0 : 0;
+        n = na + nb;
+        keep = std::min<uint64_t>(a.Kq[q], n);
+        usable = !(a0 + na > a.capA || (a.offB && b0 + nb > a.capB));
     }
-    const uint64_t keep = std::min<uint64_t>(K, n);
-    auto keyAt = [&](uint64_t i) -> uint64_t { return i < na ? orderKey(d2A[a0 + i]) : orderKey(d2B[b0 + i - na]); };
-    auto idAt = [&](uint64_t i) -> uint64_t {
-        if (i < na) return idsA ? idsA[a0 + i] : a0 + i;  // no id array: the candidate's position
-        return idsB ? idsB[b0 + i - na] : b0 + i - na;
-    };
-    if (threadIdx.x == 0 && outCount) outCount[q] = static_cast<uint32_t>(keep);
-    if (keep == 0) return;
-    const uint64_t o = outOff[q];
-    if (n <= kTopKCount) {
-        // One candidate per thread: its place is the number of smaller ones, counted over the staged
-        // keys (broadcast reads), instead of the sort's log^2 rounds with a barrier each. 4,096 queries
-        // of about 70 candidates take 68 us this way (about 60: 79 us sorted).
-        const uint32_t t = threadIdx.x;
-        uint64_t k = ~0ull, v = ~0ull;
-        if (t < n) {
-            k = keyAt(t);
-            v = idAt(t);
-            sk[2 * t] = k;
-            sk[2 * t + 1] = v;
+    // Writes the count, or the overflow; false when nothing is left to do.
+    __device__ __forceinline__ bool begin(const TopKArgs& a, uint32_t q) const {
+        if (threadIdx.x == 0) {
+            if (a.outCount) a.outCount[q] = usable ? static_cast<uint32_t>(keep) : 0u;
+            if (!usable) atomicOr(a.status, kStatusOverflowEntries);
         }
-        __syncthreads();
-        if (t >= n) return;
+        return usable && keep > 0;
+    }
+    __device__ __forceinline__ uint64_t key(const TopKArgs& a, uint64_t i) const {
+        return i < na ? orderKey(a.d2A[a0 + i]) : orderKey(a.d2B[b0 + i - na]);
+    }
+    __device__ __forceinline__ uint64_t id(const TopKArgs& a, uint64_t i) const {
+        if (i < na) return a.idsA ? a.idsA[a0 + i] : a0 + i;  // no id array: the candidate's position
+        return a.idsB ? a.idsB[b0 + i - na] : b0 + i - na;
+    }
+};
+
+// At most MOST candidates: a candidate's place is the number of smaller ones, counted over the
+// staged keys (broadcast reads), instead of the sort's log^2 rounds with a barrier each.
+template <int THREADS, uint64_t MOST>
+__device__ __forceinline__ void topKCount(const TopKArgs& a, const TopKList& l, uint64_t o, ulonglong2* stage) {
+    constexpr int kOwn = (static_cast<int>(MOST) + THREADS - 1) / THREADS;
+    const uint32_t n = static_cast<uint32_t>(l.n), keep = static_cast<uint32_t>(l.keep);
+    for (uint32_t i = threadIdx.x; i < n; i += THREADS) stage[i] = make_ulonglong2(l.key(a, i), l.id(a, i));
+    __syncthreads();
+#pragma unroll 1
+    for (int j = 0; j < kOwn; ++j) {
+        const uint32_t t = threadIdx.x + j * THREADS;
+        if (t >= n) break;
+        const ulonglong2 own = stage[t];
         uint32_t place = 0;
-        for (uint32_t i = 0; i < static_cast<uint32_t>(n); ++i) {
-            const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(sk + 2 * i);
-            place += (c.x < k || (c.x == k && (c.y < v || (c.y == v && i < t)))) ? 1u : 0u;
+#pragma unroll 4
+        for (uint32_t i = 0; i < n; ++i) {
+            const ulonglong2 c = stage[i];
+            const bool tie = (c.x == own.x) & ((c.y < own.y) | ((c.y == own.y) & (i < t)));
+            place += ((c.x < own.x) | tie) ? 1u : 0u;
         }
         if (place < keep) {
-            outIds[o + place] = v;
-            outD2[o + place] = keyValue(k);
+            a.outIds[o + place] = own.y;
+            a.outD2[o + place] = keyValue(own.x);
         }
+    }
+}
+
+// One query by a whole CTA of kTopKThreads.
+__device__ void topKBlock(const TopKArgs& a, uint32_t q, unsigned char* smem) {
+    uint64_t* sk = reinterpret_cast<uint64_t*>(smem);
+    uint64_t* sv = sk + kTopKStage;
+    const TopKList l(a, q);
+    if (!l.begin(a, q)) return;
+    const uint64_t n = l.n, keep = l.keep;
+    auto keyAt = [&](uint64_t i) -> uint64_t { return l.key(a, i); };
+    auto idAt = [&](uint64_t i) -> uint64_t { return l.id(a, i); };
+    uint64_t* outIds = a.outIds;
+    double* outD2 = a.outD2;
+    const uint64_t o = a.outOff[q];
+    if (n <= kTopKCount) {
+        topKCount<kTopKThreads, kTopKCount>(a, l, o, reinterpret_cast<ulonglong2*>(smem));
         return;
     }
     // Sorts sk/sv[0, count) by (key, id) with a bitonic network and writes the first `keep`.
@@ -395,6 +436,42 @@ __global__ void __launch_bounds__(512) topKKernel(const uint64_t* offA, const ui
             outD2[o + r] = d;
         }
         __syncthreads();
+    }
+}
+
+// Few queries: a CTA each.
+__global__ void __launch_bounds__(kTopKThreads) topKKernel(const __grid_constant__ TopKArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    topKBlock(a, blockIdx.x, smem);
+}
+
+// Many queries: a query has a hundred or so candidates, so most of kTopKThreads idle and the sort's stage
+// lets three such CTAs on an SM. Here a small CTA takes a query of at most kTopKSmall candidates, sixteen
+// an SM, and topKRestKernel's CTAs take the others: 4,096 queries of 20 or 100 results 68 -> 53 us for both.
+// From four rounds of CTAs on, and not above kTopKSmall: 1,000 queries at D = 16, most with more than 256
+// candidates, took 148 us with small CTAs for up to 512, a CTA each 57 to 66 us.
+__global__ void __launch_bounds__(kTopKSmallThreads) topKSmallKernel(const __grid_constant__ TopKArgs a) {
+    __shared__ ulonglong2 sStage[kTopKSmall];
+    const uint32_t q = blockIdx.x;
+    const TopKList l(a, q);
+    if ((l.usable && l.n > kTopKSmall) || !l.begin(a, q)) return;
+    topKCount<kTopKSmallThreads, kTopKSmall>(a, l, a.outOff[q], sStage);
+}
+
+__global__ void __launch_bounds__(kTopKThreads) topKRestKernel(const __grid_constant__ TopKArgs a, uint32_t nq) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t base = blockIdx.x; base < nq; base += 32ull * gridDim.x) {
+        const uint64_t mine = base + static_cast<uint64_t>(lane) * gridDim.x;
+        bool large = false;
+        if (mine < nq) {
+            const TopKList l(a, static_cast<uint32_t>(mine));
+            large = l.usable && l.n > kTopKSmall;
+        }
+        for (uint32_t left = __ballot_sync(0xffffffffu, large); left; left &= left - 1) {  // the same in every warp
+            topKBlock(a, static_cast<uint32_t>(base + (__ffs(left) - 1ull) * gridDim.x), smem);
+            __syncthreads();
+        }
     }
 }
 
@@ -593,12 +670,19 @@ void launchTopK(const uint64_t* offA, const uint64_t* idsA, const double* d2A, u
     const size_t smem = static_cast<size_t>(kTopKStage) * 16;
     static bool attr = false;
     if (!attr) {
-        TBLAEQ_CUDA(cudaFuncSetAttribute(topKKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
+        for (const void* f : {reinterpret_cast<const void*>(topKKernel), reinterpret_cast<const void*>(topKRestKernel)})
+            TBLAEQ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         attr = true;
     }
-    topKKernel<<<nq, 512, smem, s>>>(offA, idsA, d2A, capA, offB, idsB, d2B, capB, K, outOff, outIds, outD2, outCount,
-                                     status, cntA);
+    const TopKArgs a{offA, idsA, d2A, capA, offB, idsB, d2B, capB, K, outOff, outIds, outD2, outCount, status, cntA};
+    if (nq <= 4 * kTopKResident) {
+        topKKernel<<<nq, kTopKThreads, smem, s>>>(a);
+        TBLAEQ_LAUNCHED();
+        return;
+    }
+    topKSmallKernel<<<nq, kTopKSmallThreads, 0, s>>>(a);
+    TBLAEQ_LAUNCHED();
+    topKRestKernel<<<kTopKResident, kTopKThreads, smem, s>>>(a, nq);
     TBLAEQ_LAUNCHED();
 }
 

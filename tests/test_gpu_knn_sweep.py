@@ -95,3 +95,13 @@ def test_bound_products_far_from_the_origin(tb, oracle_mod, cuda, D, nq, offset,
     pts, ids = h.decode_points(np.arange(6000))
     P = np.ascontiguousarray(pts[rng.integers(0, 6000, nq)] + rng.normal(0, 0.3 * scale, (nq, D)))
     _check(tb, oracle_mod, h, pts, ids, P, 9)
+
+
+@pytest.mark.parametrize("nq", [900, 1776, 1777, 2500])
+def test_finish_of_few_and_many_candidates(tb, oracle_mod, cuda, nq):
+    """Either side of the finish's forms: K from none past the candidates a CTA counts, ties included."""
+    h, pts, ids = _index(tb, 4, N=8000, ratios=(40, 10))
+    rng = np.random.default_rng(nq)
+    P = np.ascontiguousarray(pts[rng.integers(0, len(pts), nq)] + rng.normal(0, 0.5, (nq, 4)))
+    P[::7] = P[0]
+    _check(tb, oracle_mod, h, pts, ids, P, rng.choice(np.array([0, 1, 31, 127, 240, 256, 512, 700], np.uint32), nq))
