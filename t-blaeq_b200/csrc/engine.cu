@@ -1604,8 +1604,10 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
         launchKnnSweepPoints(a, stream_);
     }
     if (timing_) record(1 + H);
+    // The results' places are fixed by K alone: a query with fewer candidates would leave some unwritten, so
+    // the batch runs the walk then.
     launchTopK(a.candOff, a.candId, a.candD2, a.candCap, nullptr, nullptr, nullptr, 0, dK, nq, a.outOff,
-               knnIds_.as<uint64_t>(), knnD2_.as<double>(), nullptr, a.status, stream_, a.candCnt);
+               knnIds_.as<uint64_t>(), knnD2_.as<double>(), nullptr, a.status, stream_, a.candCnt, kStatusKnnFallback);
     if (timing_) record(2 + H);
 }
 

@@ -216,6 +216,7 @@ struct TopKArgs {
     uint32_t* outCount;
     uint32_t* status;
     const uint32_t* cntA;
+    uint32_t shortStatus;
 };
 
 // Candidates of one query: list A (cntA of its slots, when given), then list B.
@@ -237,6 +238,8 @@ struct TopKList {
         if (threadIdx.x == 0) {
             if (a.outCount) a.outCount[q] = usable ? static_cast<uint32_t>(keep) : 0u;
             if (!usable) atomicOr(a.status, kStatusOverflowEntries);
+            // (After an overflow the producer may have left lists empty; the host reruns the batch.)
+            if (a.shortStatus && n < a.outOff[q + 1] - a.outOff[q] && *a.status == 0) atomicOr(a.status, a.shortStatus);
         }
         return usable && keep > 0;
     }
@@ -665,7 +668,7 @@ void launchStep(const uint64_t* keys, const uint32_t* labels, const uint32_t* cn
 void launchTopK(const uint64_t* offA, const uint64_t* idsA, const double* d2A, uint64_t capA, const uint64_t* offB,
                 const uint64_t* idsB, const double* d2B, uint64_t capB, const uint32_t* K, uint32_t nq,
                 const uint64_t* outOff, uint64_t* outIds, double* outD2, uint32_t* outCount, uint32_t* status,
-                cudaStream_t s, const uint32_t* cntA) {
+                cudaStream_t s, const uint32_t* cntA, uint32_t shortStatus) {
     if (nq == 0) return;
     const size_t smem = static_cast<size_t>(kTopKStage) * 16;
     static bool attr = false;
@@ -674,7 +677,7 @@ void launchTopK(const uint64_t* offA, const uint64_t* idsA, const double* d2A, u
             TBLAEQ_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         attr = true;
     }
-    const TopKArgs a{offA, idsA, d2A, capA, offB, idsB, d2B, capB, K, outOff, outIds, outD2, outCount, status, cntA};
+    const TopKArgs a{offA, idsA, d2A, capA, offB, idsB, d2B, capB, K, outOff, outIds, outD2, outCount, status, cntA, shortStatus};
     if (nq <= 4 * kTopKResident) {
         topKKernel<<<nq, kTopKThreads, smem, s>>>(a);
         TBLAEQ_LAUNCHED();

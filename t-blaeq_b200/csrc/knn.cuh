@@ -42,13 +42,14 @@ void launchStep(const uint64_t* keys, const uint32_t* labels, const uint32_t* cn
 // outOff[q]; outCount[q] receives how many. Status bit kStatusOverflowEntries when a query has
 // more candidates than the selection can stage.
 // cntA (optional): offA gives slots, of which only the first cntA[q] hold candidates. outCount may be
-// null. Up to 512 candidates are placed by counting, up to 4,096 sorted, more selected by radix.
+// null. shortStatus (optional): status bits raised when a query has fewer candidates than its place in
+// outOff, which then has nq + 1 entries, holds results. Up to 512 candidates are placed by counting, up to 4,096 sorted, more selected by radix.
 // capA / capB are the capacities of the candidate arrays: a query whose candidates lie beyond them
 // (the producer overflowed and the host will rerun the batch) is skipped and flagged.
 void launchTopK(const uint64_t* offA, const uint64_t* idsA, const double* d2A, uint64_t capA, const uint64_t* offB,
                 const uint64_t* idsB, const double* d2B, uint64_t capB, const uint32_t* K, uint32_t nq,
                 const uint64_t* outOff, uint64_t* outIds, double* outD2, uint32_t* outCount, uint32_t* status,
-                cudaStream_t s, const uint32_t* cntA = nullptr);
+                cudaStream_t s, const uint32_t* cntA = nullptr, uint32_t shortStatus = 0);
 
 // Lower bound and ranking score of every entry of the last KNN frontier: lb = max(centre distance -
 // subtree radius, distance to the entry's box) (conservative), score = lb.

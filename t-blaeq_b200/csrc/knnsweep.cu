@@ -10,6 +10,9 @@ namespace {
 
 constexpr uint32_t FULL = 0xffffffffu;
 constexpr float kRel = 1.00001f;  // the float sums' relative error: (D + 3) 2^-24 < 2.1e-6 for D <= 32
+// What underflow can take from a float square, and from its root: D + 3 roundings of at most the smallest
+// normal float each, under 1e-36.
+constexpr double kTiny2 = 1e-36, kTiny = 1e-18;
 
 __device__ __forceinline__ uint32_t floatKey(float f) {  // order-preserving bits
     const uint32_t u = __float_as_uint(f);
@@ -439,11 +442,14 @@ __global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(const __grid_con
         if (n >= K)
             tau = fmin(tau, sqrt(static_cast<double>(__uint_as_float((sSel[0] << 9) | 0x1ffu))) * static_cast<double>(kRel) +
                                 static_cast<double>(margin));
+        // Both come from float squares, which lose up to kTiny2 where they are denormal (coordinates of
+        // 1e-19 and less), and the finish compares FP64 distances with tau.
+        tau += kTiny;
         const double t = (tau + static_cast<double>(margin)) * (1.0 + 1e-7);
         a.tau[q] = tau;
         a.tauF[q] = __double2float_ru(t);
         const double s = t * static_cast<double>(kRel);
-        a.thrF[q] = __double2float_ru(s * s + 1e-36);  // the least a float square can miss by underflow
+        a.thrF[q] = __double2float_ru(s * s + kTiny2);
     }
 }
 

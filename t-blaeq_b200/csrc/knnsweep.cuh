@@ -105,7 +105,8 @@ struct KnnSweepArgs {
 };
 
 // Bits of KnnSweepArgs::status beyond DeviceStatus: this batch needs the level-synchronous path (a
-// coordinate beyond kSweepMaxAbs or not finite, or a K beyond the probe's stage).
+// coordinate beyond kSweepMaxAbs or not finite, a K beyond the probe's stage, or fewer candidates than
+// neighbours).
 constexpr uint32_t kStatusKnnFallback = 1u << 5;
 
 void launchKnnSweepPrepare(const KnnSweepArgs& a, cudaStream_t s);
