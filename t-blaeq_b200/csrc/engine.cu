@@ -421,8 +421,14 @@ void BatchEngine::enqueueRange(const double* dBoxes, uint32_t nq, int mode, unsi
         graphKey_ = key;
         graphKernels_ = nKernels;
         graphNodes_ = nNodes;
+        graphSweep_ = lastSweep_;
+        graphGroups_ = groupsThisBatch_;
     }
     TBLAEQ_CUDA(cudaGraphLaunch(graphExec_, stream_));
+    // A replay leaves the state its capture left: other batches may have run in between.
+    lastKnn_ = lastCompletion_ = false;
+    lastSweep_ = graphSweep_;
+    groupsThisBatch_ = graphGroups_;
 }
 
 bool BatchEngine::useNodeMajor(int mode) const {

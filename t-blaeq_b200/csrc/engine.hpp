@@ -318,6 +318,7 @@ private:
     std::vector<cudaEvent_t> events_;
     cudaGraphExec_t graphExec_ = nullptr;
     uint64_t graphKernels_ = 0, graphNodes_ = 0;
+    bool graphSweep_ = false, graphGroups_ = false;  // lastSweep_ and groupsThisBatch_ of the captured batch
     struct GraphKey {
         const double* boxes = nullptr;
         uint32_t nq = 0;
