@@ -86,7 +86,7 @@ constexpr int upperWarps() {
 // launch spent its time on chains of loads: 78 us for 4,096 queries x 2,100 nodes.
 template <int DP>
 __global__ void __launch_bounds__(upperWarps<DP>() * 32) rangeUpperKernel(RangeSweepArgs a, uint32_t wordsPerBlock,
-                                                                            int byUnit) {
+                                                                            uint32_t wordBlocks, int byUnit) {
     constexpr int WARPS = upperWarps<DP>();
     constexpr int THREADS = WARPS * 32;
     constexpr int ROW = 3 * DP + 4;  // a staged node: lo, hi, centre, radius
@@ -99,7 +99,9 @@ __global__ void __launch_bounds__(upperWarps<DP>() * 32) rangeUpperKernel(RangeS
     __shared__ uint32_t sWord[WARPS][kUpperNodes];
     const int D = a.D, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int last = a.height - 3;  // the mesh whose bits are kept
-    const uint32_t unit0 = blockIdx.y * kUpperChunk;
+    // One grid axis for both: the y axis ends at 65,535 blocks, and an index of small fan-outs has more chunks.
+    const uint32_t chunk = blockIdx.x / wordBlocks, wordBlock = blockIdx.x - chunk * wordBlocks;
+    const uint32_t unit0 = chunk * kUpperChunk;
     const uint32_t nUnits = last >= 0 ? min(kUpperChunk, a.nUpper - unit0) : 0u;
     if (tid < 2 * static_cast<int>(kRangeMaxHeight)) sCount[tid] = 0;
     auto stage = [&](float* to, int m, uint32_t g, int piece) {
@@ -123,16 +125,16 @@ __global__ void __launch_bounds__(upperWarps<DP>() * 32) rangeUpperKernel(RangeS
     if (last > 0)
         for (uint32_t i = tid; i < nUnits * PIECES; i += THREADS)
             stage(sParent[i / PIECES], last - 1, a.upper[unit0 + i / PIECES].node, i % PIECES);
-    if (blockIdx.y == 0 && blockIdx.x == 0 && tid == 0) {
+    if (blockIdx.x == 0 && tid == 0) {
         a.hdr[0] = a.nq;
         a.hdr[1] = a.nq * a.level[0].count;
     }
     __syncthreads();
-    const uint32_t w1 = min(a.words, (blockIdx.x + 1) * wordsPerBlock);
-    for (uint32_t w = blockIdx.x * wordsPerBlock + (byUnit ? 0 : warp); w < w1; w += byUnit ? 1 : WARPS) {
+    const uint32_t w1 = min(a.words, (wordBlock + 1) * wordsPerBlock);
+    for (uint32_t w = wordBlock * wordsPerBlock + (byUnit ? 0 : warp); w < w1; w += byUnit ? 1 : WARPS) {
         const uint32_t q = w * 32 + lane, n = min(32u, a.nq - w * 32);
         const bool qv = q < a.nq;
-        const bool writes = blockIdx.y == 0 && (!byUnit || warp == 0);
+        const bool writes = chunk == 0 && (!byUnit || warp == 0);
         // The word's boxes as floats: outward for the box tests, inward for the points'. Padding
         // dimensions hold [-1, 1] around the data's 0.
         __syncwarp();
@@ -787,7 +789,8 @@ void launchPadded(const RangeSweepArgs& a, cudaStream_t s) {
     const bool byUnit = chunks * wordSteps < 592;
     const uint32_t steps = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(16, chunks * wordSteps / 1184)));
     const uint32_t perBlock = byUnit ? 1 : steps * uw;
-    rangeUpperKernel<DP><<<dim3((a.words + perBlock - 1) / perBlock, chunks), uw * 32, 0, s>>>(a, perBlock, byUnit ? 1 : 0);
+    const uint32_t wordBlocks = (a.words + perBlock - 1) / perBlock;  // (useRangeSweep bounds nodes x words)
+    rangeUpperKernel<DP><<<chunks * wordBlocks, uw * 32, 0, s>>>(a, perBlock, wordBlocks, byUnit ? 1 : 0);
     TBLAEQ_LAUNCHED();
     constexpr int WARPS = SweepShape<DP, ROWS>::kWarps;
     static const int full = residentBlocks(reinterpret_cast<const void*>(rangeSweepKernel<DP, ROWS>), WARPS * 32);
