@@ -1483,10 +1483,11 @@ bool BatchEngine::useKnnSweep(unsigned flags) const {
            di_.maxAbs <= kSweepMaxAbs;
 }
 
-// Queries per block of the sweep: the bits of a block take at most 512 MiB.
+// Queries per block of the sweep: the bits of a block take at most 512 MiB, and the bound's grid has a row
+// of blocks per 256 queries.
 uint32_t BatchEngine::knnSweepBlock(uint32_t nq) const {
     const uint64_t rows = std::max<uint64_t>(1, di_.meshCount[di_.height - 2]);
-    const uint64_t words = std::max<uint64_t>(8, (512ull << 20) / (rows * 4) / 8 * 8);
+    const uint64_t words = std::min<uint64_t>(8 * 65535, std::max<uint64_t>(8, (512ull << 20) / (rows * 4) / 8 * 8));
     return static_cast<uint32_t>(std::min<uint64_t>(nq, words * 32));
 }
 

@@ -27,3 +27,25 @@ def test_range_over_many_upper_nodes(tb, cuda):
         h.set_launch_shapes([0] * 4, [100] * 4)
         assert np.array_equal(got[0], r.offsets.numpy()) and np.array_equal(got[1], r.ids.numpy())
         assert got[2] == h.level_counts() and got[0][-1] >= 70
+
+
+def test_knn_over_many_queries(tb, cuda):
+    """More queries than the bound's grid has rows for (65,535 of 256)."""
+    N, nq = 2000, 65535 * 256 + 77
+    X = np.random.default_rng(1).permutation(np.linspace(1.0, 100.0, N)).astype(np.float32)[:, None]
+    h, _ = tb.QueryHandler.build(X, height=3, ratios=(20, 10), iters=3, seed=1)
+    h.prepare_for_query(tb.LevelPolicy.L0)
+    pts, ids = h.decode_points(np.arange(N))
+    order = np.argsort(pts[:, 0], kind="stable")
+    x, ids = pts[order, 0], ids[order]
+    assert np.all(np.diff(x) > 0)
+    P = np.random.default_rng(3).uniform(0.0, 101.0, nq)
+    right = np.clip(np.searchsorted(x, P), 1, N - 1)
+    d = np.stack([P - x[right - 1], P - x[right]], 1)
+    d2 = d * d  # one dimension: the squared distance is this one rounded product
+    tie = (d2[:, 0] == d2[:, 1]) & (ids[right - 1] > ids[right])
+    near = np.where((d2[:, 1] < d2[:, 0]) | tie, right, right - 1)
+    r = h.query_batch(tb.QueryType.POINT, P[:, None], tb.Mode.EXACT, K=1)
+    assert r.total == nq and np.array_equal(r.offsets.numpy(), np.arange(nq + 1, dtype=np.uint64))
+    assert np.array_equal(r.dist2.numpy(), d2.min(1))
+    assert np.array_equal(r.ids.numpy(), ids[near])
