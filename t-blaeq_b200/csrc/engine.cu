@@ -536,7 +536,8 @@ bool BatchEngine::useRangeSweep(uint32_t nq, int mode, unsigned flags) const {
     for (size_t m = 0; m < variants_.size(); ++m)
         if (variants_[m] != kVariantDirect || grids_[m] != 100) return false;
     const uint64_t upper = di_.height > 2 ? di_.meshCount[di_.height - 3] : 1;
-    return rangeSweepBitBytes(upper, nq) <= (1ull << 30) && nq <= (1u << 21);
+    return rangeSweepBitBytes(upper, nq) <= (1ull << 30) && nq <= (1u << 21) &&
+           rangeSweepTasks(di_.unitCount, nq).count <= kRangeTasksMax;
 }
 
 // Segments a query may have: 262,144 over the batch at first, at most what the gather can order.

@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(upperWarps<DP>() * 32) rangeUpperKernel(RangeS
 }
 
 // ---- sweep ----------------------------------------------------------------------------------------
-constexpr uint32_t kBlockWords = 32;  // most query words of a task
+constexpr uint32_t kBlockWords = kRangeTaskQueries / 32;  // most query words of a task
 
 // ROWS: a cluster's hits leave in the order of its rows, as the level-synchronous path returns them at
 // dimensions where it tests no point groups; elsewhere in point-group order.
@@ -794,17 +794,10 @@ void launchPadded(const RangeSweepArgs& a, cudaStream_t s) {
     TBLAEQ_LAUNCHED();
     constexpr int WARPS = SweepShape<DP, ROWS>::kWarps;
     static const int full = residentBlocks(reinterpret_cast<const void*>(rangeSweepKernel<DP, ROWS>), WARPS * 32);
-    // A task is a part of a unit's clusters and a block of queries. Large batches take whole units and
-    // as many queries as leave several tasks for every resident warp; small ones split both, so that a
-    // query that holds a whole unit is not one warp's serial work (1.0M results of 301 boxes, D = 3:
-    // the sweep takes 179 us with whole units, 92 us in parts).
-    const uint64_t pairs = static_cast<uint64_t>(a.nUnits) * a.nq;
-    const uint32_t parts = pairs >= (4u << 20) ? 1u : pairs >= (1u << 20) ? 2u : 4u;
-    uint32_t qPer = kBlockWords * 32;
-    while (qPer > 4 && static_cast<uint64_t>(a.nUnits) * parts * ((a.nq + qPer - 1) / qPer) < 12288) qPer >>= 1;
-    const uint32_t nTasks = a.nUnits * parts * ((a.nq + qPer - 1) / qPer);
-    const int blocks = std::min<int>(full, static_cast<int>((nTasks + WARPS - 1) / WARPS));
-    rangeSweepKernel<DP, ROWS><<<std::max(1, blocks), WARPS * 32, 0, s>>>(a, nTasks, qPer, parts);
+    const RangeSweepTasks t = rangeSweepTasks(a.nUnits, a.nq);
+    const uint32_t nTasks = static_cast<uint32_t>(t.count);
+    const uint32_t blocks = std::min<uint32_t>(static_cast<uint32_t>(full), (nTasks + WARPS - 1) / WARPS);
+    rangeSweepKernel<DP, ROWS><<<std::max(1u, blocks), WARPS * 32, 0, s>>>(a, nTasks, t.qPer, t.parts);
     TBLAEQ_LAUNCHED();
     // A few queries may hold many results each: several blocks share a query then.
     const uint32_t shares = std::max<uint32_t>(1u, 4736u / a.nq);
