@@ -432,7 +432,10 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
                                 RangeSegment{(static_cast<uint64_t>(up) << 32) | run, pos, nHit};
                         else
                             atomicOr(a.status, kStatusOverflowItems);
-                        if (pos + nHit > a.rawCap || pos + nHit < pos) atomicOr(a.status, kStatusOverflowEntries);
+                        if (pos + nHit < pos)  // past 2^32 hits the count no longer tells how many
+                            atomicOr(a.status, kStatusOverflowSum);
+                        else if (pos + nHit > a.rawCap)
+                            atomicOr(a.status, kStatusOverflowEntries);
                     }
                     pos = __shfl_sync(FULL, pos, 0);
                     for (uint32_t i = lane; i < nHit; i += 32)

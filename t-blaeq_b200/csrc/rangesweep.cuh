@@ -142,8 +142,8 @@ struct RangeSweepArgs {
     uint32_t resultCap;
 };
 
-// kStatusOverflowItems here: a query has more segments than segSlots (rawCnt and the headers tell the
-// other capacities).
+// kStatusOverflowItems here: a query has more segments than segSlots; kStatusOverflowSum: more than 2^32
+// hits (rawCnt and the headers tell the other capacities).
 void launchRangeSweep(const RangeSweepArgs& a, cudaStream_t s);
 // (query, unit block) tasks etc. are sized inside; bytes of `bits` for nq queries:
 uint64_t rangeSweepBitBytes(uint64_t lastUpper, uint64_t nq);

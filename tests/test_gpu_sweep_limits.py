@@ -1,4 +1,6 @@
 """Sizes at which a sweep's launch meets a limit of the grid."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -49,3 +51,18 @@ def test_knn_over_many_queries(tb, cuda):
     assert r.total == nq and np.array_equal(r.offsets.numpy(), np.arange(nq + 1, dtype=np.uint64))
     assert np.array_equal(r.dist2.numpy(), d2.min(1))
     assert np.array_equal(r.ids.numpy(), ids[near])
+
+
+def test_range_results_beyond_32_bits(tb, cuda):
+    """More than 2^32 results: told at once, as the level-synchronous launches do, and the handle goes on."""
+    N = 500_000
+    h = tb.QueryHandler.generate(N, 3, 1.0, 100.0, False, 4, (100, 50, 20), 5, 2.5)
+    h.prepare_for_query(tb.LevelPolicy.L0)
+    wide = np.repeat(np.array([[-1e3] * 3 + [1e3] * 3]), 2 ** 32 // N + 2, axis=0)
+    with pytest.raises(tb.TblaeqError, match="2\\^32") as e:
+        h.query_batch(tb.QueryType.RANGE, wide, tb.Mode.EXACT)
+    runs = ctypes.c_uint64()
+    assert tb.lib().tblaeq_last_batch_runs(h._h, ctypes.byref(runs)) == 0
+    assert e.value.code == 4 and runs.value == 1
+    r = h.query_batch(tb.QueryType.RANGE, wide[:2], tb.Mode.EXACT)
+    assert r.total == 2 * N
