@@ -43,7 +43,7 @@ void BatchEngine::resetWorkspace() noexcept {
                          &swLive_, &swCand_, &swEnt_, &rsBits_, &rsBoxF_, &rsRaw_, &rsSegs_})
         m->release();
     rsRawCap_ = 0;
-    rsSegFactor_ = 1;
+    rsSegWant_ = 0;
     swQcap_ = 0;
     swLast_ = false;
     swCandCap_ = swEntCap_ = 0;
@@ -540,25 +540,55 @@ bool BatchEngine::useRangeSweep(uint32_t nq, int mode, unsigned flags) const {
            rangeSweepTasks(di_.unitCount, nq).count <= kRangeTasksMax;
 }
 
-// Segments a query may have: 262,144 over the batch at first, at most what the gather can order.
-uint32_t BatchEngine::rangeSweepSlots(uint32_t nq) const {
-    const uint64_t each = std::max<uint64_t>(64, 262144 / nq) * rsSegFactor_;
-    return static_cast<uint32_t>(std::min<uint64_t>(kRangeSegments, each));
+// Segments of the sweep a query may have: 262,144 over the batch or 64 at first, then what an overflow asked
+// for, as long as the batch's segments take at most 1 GiB and the gather can order them.
+uint32_t BatchEngine::rangeSweepSlotsMost(uint32_t nq) const {
+    const uint64_t most = std::max<uint64_t>({64, 262144 / nq, (1ull << 30) / sizeof(RangeSegment) / nq});
+    return static_cast<uint32_t>(std::min<uint64_t>(kRangeSegments, most));
 }
 
-void BatchEngine::reserveRangeSweep(uint32_t nq) {
+uint32_t BatchEngine::rangeSweepSlots(uint32_t nq) const {
+    const uint32_t each = std::max<uint32_t>({64u, 262144u / nq, rsSegWant_});
+    return std::min(rangeSweepSlotsMost(nq), each);
+}
+
+bool BatchEngine::roomFor(uint64_t need, uint64_t held) {
+    size_t freeB = 0, totalB = 0;
+    TBLAEQ_CUDA(cudaMemGetInfo(&freeB, &totalB));
+    return need <= freeB + held;
+}
+
+bool BatchEngine::reserveRangeSweep(uint32_t nq) {
     const uint64_t DP = paddedDims(di_.D), upper = di_.height > 2 ? di_.meshCount[di_.height - 3] : 1;
-    const uint64_t bits = rangeSweepBitBytes(upper, nq), segs = static_cast<uint64_t>(nq) * rangeSweepSlots(nq) * sizeof(RangeSegment);
-    if (rsBits_.bytes() < bits || rsBoxF_.bytes() < nq * (5 * DP + 1) * 4 || rsSegs_.bytes() < segs || rsRawCap_ < caps_.results) {
-        dropGraph();
-        if (rsBits_.bytes() < bits) rsBits_.alloc(bits);
-        if (rsBoxF_.bytes() < nq * (5 * DP + 1) * 4) rsBoxF_.alloc(nq * (5 * DP + 1) * 4);
-        if (rsSegs_.bytes() < segs) rsSegs_.alloc(segs);
-        if (rsRawCap_ < caps_.results) {
-            rsRaw_.alloc(caps_.results * 4);
-            rsRawCap_ = caps_.results;
+    struct Grow {
+        DeviceMem* m;
+        uint64_t bytes;
+    } grow[] = {{&rsBits_, rangeSweepBitBytes(upper, nq)},
+                {&rsBoxF_, nq * (5 * DP + 1) * 4},
+                {&rsSegs_, static_cast<uint64_t>(nq) * rangeSweepSlots(nq) * sizeof(RangeSegment)},
+                {&rsRaw_, caps_.results * 4}};
+    uint64_t need = 0, held = 0;
+    for (const Grow& g : grow)
+        if (g.m->bytes() < g.bytes) {
+            need += g.bytes;
+            held += g.m->bytes();
         }
+    if (need == 0) return true;
+    dropGraph();
+    bool fits = roomFor(need, held);
+    try {
+        for (const Grow& g : grow)
+            if (fits && g.m->bytes() < g.bytes) g.m->alloc(g.bytes);
+    } catch (const CudaError& e) {
+        if (e.code != cudaErrorMemoryAllocation) throw;
+        fits = false;
     }
+    rsRawCap_ = rsRaw_.bytes() / 4;
+    if (fits) return true;
+    for (DeviceMem* m : {&rsBits_, &rsBoxF_, &rsSegs_, &rsRaw_}) m->release();
+    rsRawCap_ = 0;
+    rsSkip_ = kRangeSkip;
+    return false;
 }
 
 bool BatchEngine::rangeSweepReady(uint32_t nq, unsigned flags) const {
@@ -866,22 +896,26 @@ BatchOutput BatchEngine::output(uint32_t nq, unsigned flags) const {
     return o;
 }
 
-// After an overflow of the sweep: room for all hits it counted, or more segments per query. A batch
-// whose queries have more segments than the gather orders (each of at least one result) runs level by
-// level, and so do the next ones for a while.
+// After an overflow of the sweep: room for all hits it counted, and for the most segments a query has. A
+// batch whose queries have more segments than the gather orders (each of at least one result), or than
+// rangeSweepSlots lets the batch have, runs level by level, and so do the next ones for a while.
 void BatchEngine::growRangeSweep(uint32_t nq, uint32_t st, unsigned flags) {
     const uint32_t hits = controlWord(offTickets_ + 4);
     dropGraph();
+    if (st & kStatusOverflowItems) {
+        std::vector<uint32_t> segs(nq);
+        TBLAEQ_CUDA(cudaMemcpyAsync(segs.data(), zeroBlock_.as<char>() + offQsegs_, nq * 4ull, cudaMemcpyDeviceToHost, stream_));
+        TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+        const uint32_t most = *std::max_element(segs.begin(), segs.end());
+        if (most > rangeSweepSlotsMost(nq))
+            rsSkip_ = kRangeSkip;
+        else
+            rsSegWant_ = std::max(rsSegWant_, most);
+    }
     if (hits > caps_.results) {
         EngineCaps want = caps_;
         want.results = static_cast<uint64_t>(hits) + hits / 4 + 4096;
         reserve(want, qcap_, haveVals_ || (flags & kWantVals) ? kWantVals : 0);
-    }
-    if (st & kStatusOverflowItems) {
-        if (rangeSweepSlots(nq) >= kRangeSegments)
-            rsSkip_ = 16;
-        else
-            rsSegFactor_ *= 4;
     }
 }
 
@@ -890,11 +924,8 @@ BatchOutput BatchEngine::runRange(const double* dBoxes, uint32_t nq, int mode, u
     reserve(caps_, nq, flags);
     for (int attempt = 0; attempt < 16; ++attempt) {
         lastRuns_ = static_cast<uint32_t>(attempt + 1);
-        const bool sweep = useRangeSweep(nq, mode, flags);
-        if (sweep)
-            reserveRangeSweep(nq);
-        else if (useNodeMajor(mode))
-            reserveNodeMajor(flags);
+        const bool sweep = useRangeSweep(nq, mode, flags) && reserveRangeSweep(nq);
+        if (!sweep && useNodeMajor(mode)) reserveNodeMajor(flags);
         enqueueRange(dBoxes, nq, mode, flags);
         // The status word and the result total (the results' header) come back in one copy, and the
         // caller's copies with them: one host synchronisation.

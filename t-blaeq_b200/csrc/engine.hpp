@@ -275,13 +275,17 @@ private:
     uint32_t controlHeader(int level, int which) const { return controlWord(offHdr_ + (2 * level + which) * 4); }
     // Exact range batches as one sweep (rangesweep.cuh): workspace, and whether the last range batch ran it.
     DeviceMem rsBits_, rsBoxF_, rsRaw_, rsSegs_;
-    uint32_t rsSegFactor_ = 1, rsSkip_ = 0;
+    static constexpr uint32_t kRangeSkip = 16;  // batches that run level by level after one the sweep could not serve
+    uint32_t rsSegWant_ = 0, rsSkip_ = 0;
     uint64_t rsRawCap_ = 0;
     size_t offQsegs_ = 0;
     bool rsOff_ = false, lastSweep_ = false;
     bool useRangeSweep(uint32_t nq, int mode, unsigned flags) const;
     uint32_t rangeSweepSlots(uint32_t nq) const;
-    void reserveRangeSweep(uint32_t nq);
+    uint32_t rangeSweepSlotsMost(uint32_t nq) const;
+    bool reserveRangeSweep(uint32_t nq);  // false: no memory for it, the batch runs level by level
+    // Whether `need` bytes fit in free device memory and `held`, which the caller releases first.
+    static bool roomFor(uint64_t need, uint64_t held);
     bool rangeSweepReady(uint32_t nq, unsigned flags) const;
     void enqueueRangeSweep(const double* dBoxes, uint32_t nq, unsigned flags);
     void growRangeSweep(uint32_t nq, uint32_t st, unsigned flags);
