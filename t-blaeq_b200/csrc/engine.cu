@@ -47,7 +47,7 @@ void BatchEngine::resetWorkspace() noexcept {
     swQcap_ = 0;
     swLast_ = false;
     swCandCap_ = swEntCap_ = 0;
-    swFactor_ = 1;
+    swCandGrown_ = false;
     caps_ = EngineCaps{};
     qcap_ = 0;
     haveVals_ = false;
@@ -1523,39 +1523,66 @@ uint32_t BatchEngine::knnSweepBlock(uint32_t nq) const {
     return static_cast<uint32_t>(std::min<uint64_t>(nq, words * 32));
 }
 
-void BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK) {
+bool BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand) {
     const uint64_t D = di_.D, DP = paddedDims(D), nC = di_.meshCount[di_.height - 2];
-    if (swQcap_ < nq) {
-        swQcap_ = nq;
-        // tau, result offsets, candidate offsets (8 bytes); float rows; margin, tauF, thrF, counts,
-        // entry offsets and counts (4 bytes)
-        swQuery_.alloc((static_cast<uint64_t>(nq) + 1) * (3 * 8 + DP * 4 + 6 * 4) + 1024);
-    }
     const uint32_t block = knnSweepBlock(nq);
     const uint64_t words = block <= 32 ? 1 : (((static_cast<uint64_t>(block) + 31) / 32 + 3) / 4 * 4);
-    if (swBits_.bytes() < nC * words * 4) swBits_.alloc(nC * words * 4);
-    if (swLive_.bytes() < nC * 4 + 256) swLive_.alloc(nC * 4 + 256);
-    const uint64_t cand = swFactor_ * (4 * sumK + 64ull * nq);
-    if (swCandCap_ < cand) {
-        swCand_.alloc(cand * 16);
-        swCandCap_ = cand;
-    }
+    const uint64_t results = std::max<uint64_t>(sumK, 1);
+    uint64_t entries = 0;
     if (scorer_) {
         // The clusters under the beam: probeBeam_ nodes' children per query, grown on overflow.
         const uint64_t up = di_.height > 2 ? std::max<uint64_t>(1, di_.meshCount[di_.height - 3]) : 0;
         const uint64_t each = std::min<uint64_t>(nC, up ? probeBeam_ * ((nC + up - 1) / up) : nC);
-        const uint64_t want = std::max<uint64_t>(swEntCap_, nq * each * 5 / 4 + 1024);
-        if (swEnt_.bytes() < want * (4 + 4 + 8)) swEnt_.alloc(want * (4 + 4 + 8));
-        swEntCap_ = want;
+        entries = std::max<uint64_t>(swEntCap_, nq * each * 5 / 4 + 1024);
+        if (entries > 0xffffffffull) return false;  // their counter has 32 bits
     }
-    if (knnCap_ < std::max<uint64_t>(sumK, 1)) {
-        knnCap_ = std::max<uint64_t>(sumK, 1);
-        knnIds_.alloc(knnCap_ * 8);
-        knnD2_.alloc(knnCap_ * 8);
+    // Candidates that only an earlier batch's ties asked for are given back.
+    const bool shrink = swCandGrown_ && 2 * cand < swCandCap_;
+    struct Grow {
+        DeviceMem* m;
+        uint64_t bytes;
+        bool grow;
+    } grow[] = {// tau, result offsets, candidate offsets (8 bytes); float rows; margin, tauF, thrF, candidate
+                // counts and wants, entry offsets and counts (4 bytes)
+                {&swQuery_, (static_cast<uint64_t>(nq) + 1) * (3 * 8 + DP * 4 + 7 * 4) + 1024, swQcap_ < nq},
+                {&swBits_, nC * words * 4, swBits_.bytes() < nC * words * 4},
+                {&swLive_, nC * 4 + 256, swLive_.bytes() < nC * 4 + 256},
+                {&swCand_, cand * 16, shrink || swCandCap_ < cand},
+                {&swEnt_, entries * (4 + 4 + 8), swEnt_.bytes() < entries * (4 + 4 + 8)},
+                {&knnIds_, results * 8, knnCap_ < results},
+                {&knnD2_, results * 8, knnCap_ < results}};
+    uint64_t need = 0, held = 0;
+    for (const Grow& g : grow)
+        if (g.grow) {
+            need += g.bytes;
+            held += g.m->bytes();
+        }
+    if (need) {
+        bool fits = roomFor(need, held);
+        try {
+            for (const Grow& g : grow)
+                if (fits && g.grow) g.m->alloc(g.bytes);
+        } catch (const CudaError& e) {
+            if (e.code != cudaErrorMemoryAllocation) throw;
+            fits = false;
+        }
+        if (!fits) {
+            for (const Grow& g : grow) g.m->release();
+            swQcap_ = 0;
+            swCandCap_ = swEntCap_ = knnCap_ = 0;
+            swCandGrown_ = false;
+            return false;
+        }
     }
+    swQcap_ = std::max(swQcap_, nq);
+    if (shrink || swCandCap_ < cand) swCandCap_ = cand;
+    if (shrink) swCandGrown_ = false;
+    if (scorer_) swEntCap_ = entries;
+    knnCap_ = std::max(knnCap_, results);
+    return true;
 }
 
-void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK) {
+void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, bool grown) {
     lastKnn_ = true;
     lastCompletion_ = true;
     const int H = static_cast<int>(di_.height);
@@ -1597,8 +1624,11 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
     a.candCnt = reinterpret_cast<uint32_t*>(a.thrF + q1);
     a.entOff = a.candCnt + q1;
     a.entCnt = a.entOff + q1;
+    swWant_ = a.entCnt + q1;
+    a.candWant = grown ? swWant_ : nullptr;
     swOff_ = a.outOff;
-    a.candFactor = static_cast<uint32_t>(swFactor_);
+    swCandOff_ = a.candOff;
+    swCnt_ = a.candCnt;
     a.candCap = swCandCap_;
     a.candId = swCand_.as<uint64_t>();
     a.candD2 = reinterpret_cast<double*>(a.candId + swCandCap_);
@@ -1651,13 +1681,20 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
 }
 
 bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o) {
-    // Candidate slots start at 4 K + 64 a query (the bound is within a few percent of the K-th
-    // distance, so about 1.5 K pass); ties and bounds that stayed loose grow them, at most 256-fold.
+    // Candidate slots are 4 K + 64 a query (the bound is within a few percent of the K-th distance, so
+    // about 1.5 K pass). Where ties or a loose bound pass more, every query's count is known after the
+    // run, and a second one gives each its own.
     const uint64_t cap = std::min<uint64_t>(sumK, nq * di_.meshCount[di_.height - 1]);
+    uint64_t cand = 4 * cap + 64ull * nq;
+    bool grown = false;
     for (int attempt = 0; attempt < 8; ++attempt) {
         lastRuns_ = static_cast<uint32_t>(attempt + 1);
-        reserveKnnSweep(nq, cap);
-        enqueueKnnSweep(dPoints, nq, dK);
+        if (!reserveKnnSweep(nq, cap, cand)) {
+            if (grown || nq == 1) return false;
+            throw SplitBatch("the KNN sweep's buffers exceed free device memory or 32-bit counts; split the batch");
+        }
+        swCandGrown_ = swCandGrown_ || grown;
+        enqueueKnnSweep(dPoints, nq, dK, grown);
         swLast_ = true;  // output() names the sweep's offsets
         if (after_) after_(afterCtx_, output(nq, 0));
         fetchControl();
@@ -1675,11 +1712,19 @@ bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t
         }
         if (scorer_ && entries > swEntCap_) {
             swEntCap_ = entries + entries / 4;
-        } else if (swFactor_ >= 256) {
-            swFactor_ = 1;
-            return false;
+        } else if (st & kStatusOverflowItems) {
+            std::vector<uint64_t> off(nq + 1ull);
+            std::vector<uint32_t> cnt(nq);
+            TBLAEQ_CUDA(cudaMemcpyAsync(off.data(), swCandOff_, off.size() * 8, cudaMemcpyDeviceToHost, stream_));
+            TBLAEQ_CUDA(cudaMemcpyAsync(cnt.data(), swCnt_, cnt.size() * 4, cudaMemcpyDeviceToHost, stream_));
+            TBLAEQ_CUDA(cudaMemcpyAsync(swWant_, swCnt_, cnt.size() * 4, cudaMemcpyDeviceToDevice, stream_));
+            TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
+            cand = 0;
+            for (uint32_t i = 0; i < nq; ++i) cand += std::max<uint64_t>(off[i + 1] - off[i], cnt[i]);
+            grown = true;
+            swCandGrown_ = false;  // nothing is given back while this batch needs it
         } else {
-            swFactor_ *= 4;
+            return false;
         }
     }
     return false;

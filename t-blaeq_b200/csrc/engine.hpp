@@ -293,13 +293,15 @@ private:
     // runKnnSweep returns false when the batch needs the level-synchronous path instead.
     DeviceMem swQuery_, swBits_, swLive_, swCand_, swEnt_;
     uint32_t swQcap_ = 0;
-    uint64_t swCandCap_ = 0, swEntCap_ = 0, swFactor_ = 1;
-    uint64_t* swOff_ = nullptr;
+    uint64_t swCandCap_ = 0, swEntCap_ = 0;
+    uint64_t *swOff_ = nullptr, *swCandOff_ = nullptr;
+    uint32_t *swCnt_ = nullptr, *swWant_ = nullptr;
+    bool swCandGrown_ = false;  // swCand_ holds more than batches without many ties ask for
     bool swLast_ = false, knnTrace_ = false;
     bool useKnnSweep(unsigned flags) const;
     uint32_t knnSweepBlock(uint32_t nq) const;
-    void reserveKnnSweep(uint32_t nq, uint64_t sumK);
-    void enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK);
+    bool reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand);  // false: no memory for it
+    void enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, bool grown);
     bool runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o);
 
     void growFromHeaders();

@@ -55,7 +55,8 @@ __global__ void __launch_bounds__(1024) sweepPrepareKernel(KnnSweepArgs a, uint3
         const uint32_t q = base + tid;
         const uint32_t K = q < a.nq ? a.K[q] : 0u;
         const unsigned long long r = min(static_cast<unsigned long long>(K), static_cast<unsigned long long>(a.nPoints));
-        const unsigned long long c = q < a.nq ? static_cast<unsigned long long>(a.candFactor) * (4ull * r + 64ull) : 0ull;
+        unsigned long long c = q < a.nq ? 4ull * r + 64ull : 0ull;
+        if (a.candWant && q < a.nq) c = max(c, static_cast<unsigned long long>(a.candWant[q]));
         unsigned long long ir = r, ic = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -498,7 +499,7 @@ __global__ void __launch_bounds__(kBoundThreads) knnBoundBitsKernel(const __grid
     constexpr int W = STEPS <= 2 ? kBoundWords : kBoundWords / 2;  // words staged at once (48 KB of shared memory)
     __shared__ __align__(16) float4 sB[W][4][STEPS][32];  // hi, hi, lo, lo of a lane's two dimensions
     __shared__ __align__(8) float2 sE[W][4][32];
-    if (*a.status) return;
+    if (*a.status & ~kStatusOverflowItems) return;
     const KnnSweepLevel& L = a.level[a.height - 2];
     const uint32_t w0 = blockIdx.y * kBoundWords;
     const uint32_t left = a.qEnd - a.qBegin > w0 * 32 ? a.qEnd - a.qBegin - w0 * 32 : 0u;  // queries from w0 on
@@ -663,7 +664,7 @@ __device__ __forceinline__ bool measureInline(const KnnSweepArgs& a, uint32_t ro
         a.candD2[pos] = d2;
         return true;
     }
-    atomicOr(a.status, kStatusOverflowEntries);
+    atomicOr(a.status, kStatusOverflowItems);
     return false;
 }
 
@@ -774,7 +775,7 @@ __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(const __grid_con
     __shared__ float sThr[kSweepWarps][32];
     __shared__ uint32_t sId[kSweepWarps][32];
     __shared__ __align__(16) float sBox[kSweepWarps][kSweepGroups][2 * DP];
-    if (*a.status) return;
+    if (*a.status & ~kStatusOverflowItems) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned long long tested = 0;
     uint32_t kept = 0;              // this lane's candidates
@@ -870,7 +871,7 @@ __global__ void __launch_bounds__(kSweepThreads, DP <= 16 ? 4 : 2) knnSweepMmaKe
     constexpr int STEPS = (DP + 7) / 8;
     __shared__ uint32_t sList[kSweepWarps][kSweepList];
     __shared__ __align__(16) float sBox[kSweepWarps][kSweepGroups][2 * DP];
-    if (*a.status) return;
+    if (*a.status & ~kStatusOverflowItems) return;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int quad = lane >> 2, kc = 2 * (lane & 3);  // fragment row, first of the lane's two dimensions in a step
     const KnnSweepLevel& L = a.level[a.height - 2];

@@ -79,7 +79,7 @@ struct KnnSweepArgs {
     uint64_t* candOff;      // nq + 1: candidate slots
     uint32_t* candCnt;      // nq
     uint64_t candCap;       // slots in all
-    uint32_t candFactor;    // slots per query: candFactor * (4 K + 64)
+    const uint32_t* candWant;  // nq (or null): slots per query are 4 K + 64, or this where it is more
     uint64_t* candId;
     double* candD2;
     uint32_t beam;
@@ -104,7 +104,8 @@ struct KnnSweepArgs {
     uint32_t* status;
 };
 
-// Bits of KnnSweepArgs::status beyond DeviceStatus: this batch needs the level-synchronous path (a
+// kStatusOverflowItems here: a query has more candidates than slots; counting goes on to the end of the
+// batch. Bits of KnnSweepArgs::status beyond DeviceStatus: this batch needs the level-synchronous path (a
 // coordinate beyond kSweepMaxAbs or not finite, a K beyond the probe's stage, or fewer candidates than
 // neighbours).
 constexpr uint32_t kStatusKnnFallback = 1u << 5;

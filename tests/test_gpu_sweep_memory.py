@@ -62,3 +62,60 @@ def test_range_without_memory_for_the_sweep(tb, cuda, nth):
         tb.lib().tblaeq_debug_fail_alloc_after(0)
     for _ in range(20):
         _same(_range(tb, h, Q), want)
+
+
+def _knn(tb, h, P, K):
+    r = h.query_batch(tb.QueryType.POINT, P, tb.Mode.EXACT, K=K)
+    return r.offsets.numpy().copy(), r.ids.numpy().copy(), r.dist2.numpy().copy()
+
+
+def _brute(oracle_mod, pts, ids, P, K):
+    b = oracle_mod.brute_query(pts, ids, oracle_mod.KNN, np.ascontiguousarray(P), K=K)
+    return b.offsets, b.ids, b.dist2
+
+
+def _equal(got, want):
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+def test_ties_of_one_batch_are_not_reserved_for_the_next(tb, oracle_mod, cuda):
+    """3,000 points at one distance: a second run holds them; 100,000 other queries take no more for it."""
+    X = np.full((6000, 4), 7.0, np.float32)
+    X[3000:] += np.random.default_rng(0).uniform(5, 20, (3000, 4)).astype(np.float32)
+    h, _ = tb.QueryHandler.build(X, height=3, ratios=(50, 10), iters=3, seed=1)
+    h.prepare_for_query(tb.LevelPolicy.L0)
+    pts, ids = h.decode_points(np.arange(6000))
+    ties = np.full((33, 4), 7.0)
+    other = np.ascontiguousarray(X[np.random.default_rng(1).integers(3000, 6000, 100_000)] + 0.25)
+    want = _brute(oracle_mod, pts, ids, ties, 12)
+    small = _brute(oracle_mod, pts, ids, other[:50], 100)
+    start = tb.lib().tblaeq_live_device_bytes()
+    for _ in range(2):
+        _equal(_knn(tb, h, ties, 12), want)
+        assert h.knn_batch_info()["runs"] == 2
+    got = _knn(tb, h, other, 100)
+    assert tb.lib().tblaeq_live_device_bytes() - start < 4 << 30
+    _equal((got[0][:51], got[1][:5000], got[2][:5000]), small)
+
+
+@pytest.mark.parametrize("learned", [False, True])
+@pytest.mark.parametrize("nth", [2, 4, 6])
+def test_knn_without_memory_for_the_sweep(tb, oracle_mod, cuda, nth, learned):
+    """A refused allocation asks for a smaller batch (which callers split), a single query takes the walk."""
+    h, pts = _index(tb, 8, 30_000, (40, 20, 10))
+    ids = h.decode_points(np.arange(len(pts)))[1]
+    if learned:
+        h.scorer_train(np.ascontiguousarray(pts[:256] + 0.3), K=10, max_samples=2000, epochs=1, seed=1)
+    P = np.ascontiguousarray(pts[:200] + 0.5)
+    want = _brute(oracle_mod, pts, ids, P, 10)
+    _range(tb, h, np.ascontiguousarray(np.concatenate([P, P], 1)))  # the workspace shared with range batches
+    one = _brute(oracle_mod, pts, ids, P[:1], 10)
+    tb.lib().tblaeq_debug_fail_alloc_after(nth)  # the first is the staged K
+    try:
+        _equal(_knn(tb, h, P, 10), want)
+    finally:
+        tb.lib().tblaeq_debug_fail_alloc_after(0)
+    info = h.knn_batch_info()
+    assert info["traversals"] == 2 and "KNN sweep" in info["split_reason"]
+    _equal(_knn(tb, h, P[:1], 10), one)
+    _equal(_knn(tb, h, P, 10), want)
