@@ -48,6 +48,7 @@ void BatchEngine::resetWorkspace() noexcept {
     swLast_ = false;
     swCandCap_ = swEntCap_ = 0;
     swCandGrown_ = false;
+    swFactor_ = 1;
     caps_ = EngineCaps{};
     qcap_ = 0;
     haveVals_ = false;
@@ -1582,7 +1583,7 @@ bool BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand) {
     return true;
 }
 
-void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, bool grown) {
+void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint32_t factor, bool grown) {
     lastKnn_ = true;
     lastCompletion_ = true;
     const int H = static_cast<int>(di_.height);
@@ -1626,6 +1627,7 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
     a.entCnt = a.entOff + q1;
     swWant_ = a.entCnt + q1;
     a.candWant = grown ? swWant_ : nullptr;
+    a.candFactor = factor;
     swOff_ = a.outOff;
     swCandOff_ = a.candOff;
     swCnt_ = a.candCnt;
@@ -1682,19 +1684,29 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
 
 bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o) {
     // Candidate slots are 4 K + 64 a query (the bound is within a few percent of the K-th distance, so
-    // about 1.5 K pass). Where ties or a loose bound pass more, every query's count is known after the
-    // run, and a second one gives each its own.
+    // about 1.5 K pass); 4 or 16 times that once a batch needed it (D = 16: 1,000 queries, N = 5M, K = 20,
+    // some above 576), where that takes at most 8 GiB. Where ties or a loose bound pass more, every
+    // query's count is known after the run, and a second one gives each its own; the batches after it don't
+    // keep those.
     const uint64_t cap = std::min<uint64_t>(sumK, nq * di_.meshCount[di_.height - 1]);
-    uint64_t cand = 4 * cap + 64ull * nq;
+    const uint64_t least = 4 * cap + 64ull * nq;
+    uint32_t factor = swFactor_;
+    while (factor > 1 && factor * least * 16 > (8ull << 30)) factor /= 4;
+    uint64_t cand = factor * least;
     bool grown = false;
     for (int attempt = 0; attempt < 8; ++attempt) {
         lastRuns_ = static_cast<uint32_t>(attempt + 1);
         if (!reserveKnnSweep(nq, cap, cand)) {
+            if (!grown && factor > 1) {
+                factor = 1;
+                cand = least;
+                continue;
+            }
             if (grown || nq == 1) return false;
             throw SplitBatch("the KNN sweep's buffers exceed free device memory or 32-bit counts; split the batch");
         }
         swCandGrown_ = swCandGrown_ || grown;
-        enqueueKnnSweep(dPoints, nq, dK, grown);
+        enqueueKnnSweep(dPoints, nq, dK, factor, grown);
         swLast_ = true;  // output() names the sweep's offsets
         if (after_) after_(afterCtx_, output(nq, 0));
         fetchControl();
@@ -1719,10 +1731,21 @@ bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t
             TBLAEQ_CUDA(cudaMemcpyAsync(cnt.data(), swCnt_, cnt.size() * 4, cudaMemcpyDeviceToHost, stream_));
             TBLAEQ_CUDA(cudaMemcpyAsync(swWant_, swCnt_, cnt.size() * 4, cudaMemcpyDeviceToDevice, stream_));
             TBLAEQ_CUDA(cudaStreamSynchronize(stream_));
-            cand = 0;
-            for (uint32_t i = 0; i < nq; ++i) cand += std::max<uint64_t>(off[i + 1] - off[i], cnt[i]);
-            grown = true;
-            swCandGrown_ = false;  // nothing is given back while this batch needs it
+            uint64_t all = 0;
+            uint32_t wanted = factor;
+            for (uint32_t i = 0; i < nq; ++i) {
+                const uint64_t slots = off[i + 1] - off[i];
+                all += std::max<uint64_t>(slots, cnt[i]);
+                while (wanted <= 16 && !grown && cnt[i] > slots / factor * wanted) wanted *= 4;
+            }
+            if (!grown && wanted <= 16 && wanted * least * 16 <= (8ull << 30)) {
+                swFactor_ = factor = wanted;
+                cand = factor * least;
+            } else {
+                cand = all;
+                grown = true;
+                swCandGrown_ = false;  // nothing is given back while this batch needs it
+            }
         } else {
             return false;
         }

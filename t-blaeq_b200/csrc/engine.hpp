@@ -296,12 +296,13 @@ private:
     uint64_t swCandCap_ = 0, swEntCap_ = 0;
     uint64_t *swOff_ = nullptr, *swCandOff_ = nullptr;
     uint32_t *swCnt_ = nullptr, *swWant_ = nullptr;
+    uint32_t swFactor_ = 1;     // 1, 4 or 16: see runKnnSweep
     bool swCandGrown_ = false;  // swCand_ holds more than batches without many ties ask for
     bool swLast_ = false, knnTrace_ = false;
     bool useKnnSweep(unsigned flags) const;
     uint32_t knnSweepBlock(uint32_t nq) const;
     bool reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand);  // false: no memory for it
-    void enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, bool grown);
+    void enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint32_t factor, bool grown);
     bool runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o);
 
     void growFromHeaders();

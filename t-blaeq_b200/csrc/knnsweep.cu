@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(1024) sweepPrepareKernel(KnnSweepArgs a, uint3
         const uint32_t q = base + tid;
         const uint32_t K = q < a.nq ? a.K[q] : 0u;
         const unsigned long long r = min(static_cast<unsigned long long>(K), static_cast<unsigned long long>(a.nPoints));
-        unsigned long long c = q < a.nq ? 4ull * r + 64ull : 0ull;
+        unsigned long long c = q < a.nq ? a.candFactor * (4ull * r + 64ull) : 0ull;
         if (a.candWant && q < a.nq) c = max(c, static_cast<unsigned long long>(a.candWant[q]));
         unsigned long long ir = r, ic = c;
 #pragma unroll

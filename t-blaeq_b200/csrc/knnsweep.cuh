@@ -79,7 +79,8 @@ struct KnnSweepArgs {
     uint64_t* candOff;      // nq + 1: candidate slots
     uint32_t* candCnt;      // nq
     uint64_t candCap;       // slots in all
-    const uint32_t* candWant;  // nq (or null): slots per query are 4 K + 64, or this where it is more
+    uint32_t candFactor;       // slots per query: candFactor * (4 K + 64),
+    const uint32_t* candWant;  // or this where it is more (nq, or null)
     uint64_t* candId;
     double* candD2;
     uint32_t beam;
