@@ -230,6 +230,12 @@ uint64_t BatchEngine::lastTotal(uint32_t nq) {
 }
 
 size_t BatchEngine::workspaceBytes() const {
+    size_t t = levelBytes();
+    for (const DeviceMem* m : {&swQuery_, &swBits_, &swLive_, &swCand_, &swEnt_, &rsBits_, &rsBoxF_, &rsRaw_, &rsSegs_}) t += m->bytes();
+    return t;
+}
+
+size_t BatchEngine::levelBytes() const {
     size_t t = zeroBlock_.bytes() + offsets_.bytes() + resIds_.bytes() + resVals_.bytes() + resQ_.bytes() +
                resDist_.bytes() + nmList_.bytes() + nmNodeOff_.bytes() + nmUnitOff_.bytes() + rawIds_.bytes() +
                rawQ_.bytes() + rawVals_.bytes();
@@ -279,7 +285,7 @@ void BatchEngine::reserve(const EngineCaps& want, uint32_t nq, unsigned flags) {
         const uint64_t needR = growR ? c.results * (20 + ((wantVals || haveVals_) ? 8 * D : 0)) : 0;
         size_t freeB = 0, totalB = 0;
         TBLAEQ_CUDA(cudaMemGetInfo(&freeB, &totalB));
-        const uint64_t held = workspaceBytes(), margin = 512ull << 20;
+        const uint64_t held = levelBytes(), margin = 512ull << 20;
         if (needF + needR > freeB + held && needF + needR > margin)
             throw SplitBatch("batch workspace (" + std::to_string((needF + needR) >> 20) +
                              " MiB) exceeds free device memory; split the batch");

@@ -199,7 +199,9 @@ public:
     // a timeout) calls it on the way out: no later launch can see a capacity whose buffer is gone.
     void resetWorkspace() noexcept;
     const EngineCaps& caps() const { return caps_; }
+    // What the batches so far hold: the level-synchronous launches' buffers (levelBytes) and the sweeps'.
     size_t workspaceBytes() const;
+    size_t levelBytes() const;
     int launchesPerBatch() const { return static_cast<int>(di_.height) + 2; }
     cudaStream_t stream() const { return stream_; }
 

@@ -119,3 +119,19 @@ def test_knn_without_memory_for_the_sweep(tb, oracle_mod, cuda, nth, learned):
     assert info["traversals"] == 2 and "KNN sweep" in info["split_reason"]
     _equal(_knn(tb, h, P[:1], 10), one)
     _equal(_knn(tb, h, P, 10), want)
+
+
+def test_serving_admission_counts_the_sweep(tb, cuda):
+    """A lane's slots follow its memory budget: 2,000 KNN requests of K = 2,000 hold 258 MB of candidates
+    alone, so 64 MiB admit fewer than 700 at once."""
+    h, pts = _index(tb, 6, 60_000, (60, 20, 5))
+    n = 2000
+    rows = np.ascontiguousarray(np.concatenate([pts[:n] + 0.1, np.zeros((n, 6))], 1))
+    with tb.Server(h, max_batch=n, memory_budget=64 << 20, learned=False, lanes=2) as srv:
+        for wave in range(3):
+            srv.stats(reset=True)
+            srv.replay(np.zeros(n, np.int32), rows, np.full(n, 2000, np.uint32), np.zeros(n))
+            assert srv.wait_idle()
+            s = srv.stats()
+            assert s["completed"] == n and s["failed"] == 0
+            assert wave == 0 or s["max_batch"] < 700
