@@ -258,10 +258,11 @@ static BatchOutput runKnnChunked(tblaeq_handle* h, const double* dQueries, uint6
         const uint64_t c = std::min(chunk, nq - i);
         uint64_t sk = 0;
         for (uint64_t q = i; q < i + c; ++q) sk += k[q];
+        const uint32_t maxK = *std::max_element(k.begin() + i, k.begin() + i + c);
         BatchOutput co;
         try {
             co = rt.engine->runKnn(dQueries + i * D, static_cast<uint32_t>(c), h->kStage.as<uint32_t>() + i, sk,
-                                   flags & ~static_cast<unsigned>(TBLAEQ_WANT_LEVELS));
+                                   flags & ~static_cast<unsigned>(TBLAEQ_WANT_LEVELS), maxK);
         } catch (const CudaError& e) {
             // Too large for the 32-bit traversal space or for the free device memory (the engine
             // released its workspace on the way out): halve the chunk.
@@ -312,11 +313,13 @@ static int runBatch(tblaeq_handle* h, const tblaeq_batch* b, const double* dQuer
             return fail(TBLAEQ_ERR_INVALID, "batched KNN is exact; use tblaeq_level for the reference's STEP sets");
         std::vector<uint32_t> k(b->nq);
         uint64_t sumK = 0;
+        uint32_t maxK = 0;
         for (uint64_t i = 0; i < b->nq; ++i) {
             const uint64_t v = b->kPerQuery ? b->kPerQuery[i] : b->K;
             if (v > 0xffffffffull) return fail(TBLAEQ_ERR_INVALID, "K too large");
             k[i] = static_cast<uint32_t>(v);
             sumK += v;
+            maxK = std::max(maxK, k[i]);
         }
         if (h->kStage.bytes() < std::max<size_t>(b->nq, 1) * 4) h->kStage.alloc(std::max<size_t>(b->nq, 1) * 4);
         if (b->nq) copyIn(h, h->kStage.get(), k.data(), b->nq * 4, 1);
@@ -329,7 +332,8 @@ static int runBatch(tblaeq_handle* h, const tblaeq_batch* b, const double* dQuer
             o = runKnnChunked(h, dQueries, b->nq, k, b->flags, limit);
         } else {
             try {
-                o = rt.engine->runKnn(dQueries, static_cast<uint32_t>(b->nq), h->kStage.as<uint32_t>(), sumK, b->flags);
+                o = rt.engine->runKnn(dQueries, static_cast<uint32_t>(b->nq), h->kStage.as<uint32_t>(), sumK, b->flags,
+                                       maxK);
                 h->lastKnnChunk = b->nq;
                 h->lastKnnRuns = 1;
             } catch (const CudaError& e) {

@@ -1514,12 +1514,12 @@ bool BatchEngine::growKnnMajor() {
     return grew;
 }
 
-bool BatchEngine::useKnnSweep(unsigned flags) const {
+bool BatchEngine::useKnnSweep(unsigned flags, uint32_t maxK) const {
     // Per-level counts and the scorer's training traces describe the level-synchronous walk, and so do
     // the options that change it; a streamed last interval has no decoded points on the device.
     return twoWave_ && knnNodeMajor_ && probeBeam_ > 0 && knnGroups_ && !knnTrace_ && !(flags & kWantLevels) &&
            di_.height >= 2 && di_.height <= kSweepMaxHeight && di_.pointsD.bytes() && di_.pointsF.bytes() &&
-           di_.maxAbs <= kSweepMaxAbs;
+           di_.maxAbs <= kSweepMaxAbs && maxK <= kProbePoints / 2;
 }
 
 // Queries per block of the sweep: the bits of a block take at most 512 MiB, and the bound's grid has a row
@@ -1690,7 +1690,7 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
 
 bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o) {
     // Candidate slots are 4 K + 64 a query (the bound is within a few percent of the K-th distance, so
-    // about 1.5 K pass); 4 or 16 times that once a batch needed it (D = 16: 1,000 queries, N = 5M, K = 20,
+    // about 1.5 K pass); 4 to 64 times that once a batch needed it (D = 16: 1,000 queries, N = 5M, K = 20,
     // some above 576), where that takes at most 8 GiB. Where ties or a loose bound pass more, every
     // query's count is known after the run, and a second one gives each its own; the batches after it don't
     // keep those.
@@ -1742,9 +1742,9 @@ bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t
             for (uint32_t i = 0; i < nq; ++i) {
                 const uint64_t slots = off[i + 1] - off[i];
                 all += std::max<uint64_t>(slots, cnt[i]);
-                while (wanted <= 16 && !grown && cnt[i] > slots / factor * wanted) wanted *= 4;
+                while (wanted <= kSweepFactorMax && !grown && cnt[i] > slots / factor * wanted) wanted *= 4;
             }
-            if (!grown && wanted <= 16 && wanted * least * 16 <= (8ull << 30)) {
+            if (!grown && wanted <= kSweepFactorMax && wanted * least * 16 <= (8ull << 30)) {
                 swFactor_ = factor = wanted;
                 cand = factor * least;
             } else {
@@ -1760,11 +1760,11 @@ bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t
 }
 
 BatchOutput BatchEngine::runKnn(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK,
-                                unsigned flags) {
+                                unsigned flags, uint32_t maxK) {
     WorkspaceGuard guard(*this);
     reserve(caps_, nq, flags);
     swLast_ = false;
-    if (nq > 0 && useKnnSweep(flags)) {
+    if (nq > 0 && useKnnSweep(flags, maxK)) {
         BatchOutput o;
         if (runKnnSweep(dPoints, nq, dK, sumK, o)) return o;
     }

@@ -55,9 +55,10 @@ public:
     BatchOutput runRange(const double* dBoxes, uint32_t nq, int mode, unsigned flags);
 
     // Exact KNN batch: dPoints = nq rows of D coordinates, dK = neighbours per query (device),
-    // sumK = sum of K over the batch (host). Results: per-query offsets, ids and squared distances,
+    // sumK = sum of K over the batch (host), maxK = the largest (0: not known). Results: per-query offsets, ids and squared distances,
     // ascending by (distance, id). Blocks until done.
-    BatchOutput runKnn(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, unsigned flags);
+    BatchOutput runKnn(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, unsigned flags,
+                       uint32_t maxK = 0);
     void enqueueKnn(const double* dPoints, uint32_t nq, const uint32_t* dK, unsigned flags);
     // Two-wave final level (default on): rank the last frontier's clusters, expand the best few per
     // query to bound the K-th distance by real points, then expand only the clusters that bound
@@ -298,10 +299,10 @@ private:
     uint64_t swCandCap_ = 0, swEntCap_ = 0;
     uint64_t *swOff_ = nullptr, *swCandOff_ = nullptr;
     uint32_t *swCnt_ = nullptr, *swWant_ = nullptr;
-    uint32_t swFactor_ = 1;     // 1, 4 or 16: see runKnnSweep
+    uint32_t swFactor_ = 1;     // 1, 4, 16 or 64: see runKnnSweep
     bool swCandGrown_ = false;  // swCand_ holds more than batches without many ties ask for
     bool swLast_ = false, knnTrace_ = false;
-    bool useKnnSweep(unsigned flags) const;
+    bool useKnnSweep(unsigned flags, uint32_t maxK) const;
     uint32_t knnSweepBlock(uint32_t nq) const;
     bool reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand);  // false: no memory for it
     void enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint32_t factor, bool grown);

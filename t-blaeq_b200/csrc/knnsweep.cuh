@@ -43,6 +43,8 @@ constexpr double kSweepMaxAbs = 1e18;
 // Points a probe reads at most (its selection stage), and so the largest K it can bound.
 constexpr uint32_t kProbePoints = 4096;
 constexpr uint32_t kSweepMaxHeight = 16;
+// Most times 4 K + 64 candidate slots a query that batches keep for the ones after them (a power of four).
+constexpr uint32_t kSweepFactorMax = 64;
 
 struct KnnSweepLevel {
     const float* x;        // centres, paddedDims floats per node

@@ -241,7 +241,7 @@ void Server::runGroup(Lane& lane, std::vector<Request>& batch, size_t begin, siz
             TBLAEQ_CUDA(cudaMemcpyAsync(lane.dk.get(), hk.data(), n * 4, cudaMemcpyHostToDevice, lane.stream));
             try {
                 o = lane.engine->runKnn(lane.dq.as<double>(), static_cast<uint32_t>(n), lane.dk.as<uint32_t>(), sumK,
-                                        flags);
+                                        flags, *std::max_element(hk.begin(), hk.end()));
             } catch (const SplitBatch&) {
                 if (n == 1) throw;
                 const size_t mid = begin + n / 2;
