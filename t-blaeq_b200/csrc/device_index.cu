@@ -57,9 +57,10 @@ void DeviceMem::release() {
     n_ = 0;
 }
 
-DerivedArrays computeDerived(const HostIndex& idx) {
+DerivedArrays computeDerived(const HostIndex& idx, bool resident) {
     const uint64_t D = idx.D, H = idx.height;
     DerivedArrays out;
+    out.sweeps = resident && D <= 32 && H <= kRangeMaxHeight;
     out.cbeg.resize(H - 1);
     out.ccnt.resize(H - 1);
     out.leaf.resize(H - 1);
@@ -112,10 +113,10 @@ DerivedArrays computeDerived(const HostIndex& idx) {
 
     out.nodeX.resize(H - 1);
     for (uint64_t m = 0; m + 1 < H; ++m) out.nodeX[m] = dec[m];
-    out.parent.assign(parent.begin(), parent.begin() + static_cast<ptrdiff_t>(H - 1));
     // Units of the range sweep: every last upper node's clusters, nodes in depth-first order, split
     // evenly into at most kRangeUnit.
-    {
+    if (out.sweeps) {
+        out.parent.assign(parent.begin(), parent.begin() + static_cast<ptrdiff_t>(H - 1));
         auto split = [&](uint32_t node, uint32_t first, uint32_t n) {
             const uint32_t parts = (n + kRangeUnit - 1) / kRangeUnit;
             for (uint32_t i = 0; i < parts; ++i) {
@@ -164,7 +165,7 @@ DerivedArrays computeDerived(const HostIndex& idx) {
     const uint64_t DP = paddedDims(D);
     for (const auto& mesh : dec)
         for (double v : mesh) out.maxAbs = std::max(out.maxAbs, std::fabs(v));
-    if (H >= 2 && D <= 32) {
+    if (H >= 2 && (out.sweeps || floatPointsSupported(D))) {
         // Point groups: every finest cluster's rows, reordered within the cluster's own row range by
         // median splits along the widest dimension until at most kPointGroup rows remain, and the
         // float copy of the points in that order.
@@ -424,6 +425,116 @@ HostMapping& HostMapping::operator=(HostMapping&& o) noexcept {
     return *this;
 }
 
+namespace {
+
+// Float points and point groups.
+size_t floatCopyBytes(const DerivedArrays& der) {
+    return der.pointsF.size() * 4 + der.pointPerm.size() * 4 + der.groupBox.size() * 4 + der.groupFirst.size() * 16 +
+           der.clusterGroup.size() * 16;
+}
+
+void uploadFloatCopy(const HostIndex& idx, const DerivedArrays& der, DeviceIndex& di, cudaStream_t s) {
+    di.pointsF = upload(der.pointsF, s);
+    di.pointPerm = upload(der.pointPerm, s);
+    const size_t G = der.groupFirst.size(), nCl = der.clusterGroup.size() - 1;
+    std::vector<NodeRec> grec(G), crec(nCl);
+    for (size_t g = 0; g < G; ++g) grec[g] = NodeRec{0.0, der.groupFirst[g], der.groupCount[g]};
+    for (size_t c = 0; c < nCl; ++c)
+        crec[c] = NodeRec{der.radSub[idx.height - 2][c], der.clusterGroup[c], der.clusterGroup[c + 1] - der.clusterGroup[c]};
+    di.groupRec = upload(grec, s);
+    di.groupBox = upload(der.groupBox, s);
+    di.clusterGroups = upload(crec, s);
+    TBLAEQ_CUDA(cudaStreamSynchronize(s));
+}
+
+// What only the sweeps read. An index that leaves no room for it (half of the free memory at most: the
+// workspaces need the rest) is served by the level-synchronous launches.
+void uploadSweepArrays(const HostIndex& idx, const DerivedArrays& der, DeviceIndex& di, cudaStream_t s) {
+    const uint64_t D = idx.D, DP = paddedDims(D), H = idx.height;
+    uint64_t nodes = 0;
+    for (uint64_t m = 0; m + 1 < H; ++m) nodes += der.cbeg[m].size();
+    const bool floatCopy = !floatPointsSupported(D);
+    uint64_t need = (der.units.size() + der.upperUnits.size()) * sizeof(RangeUnit) + idx.meshCount(H - 2) * DP * 4 +
+                    nodes * (DP * 4 + 4 + 4 + (DP != D ? 2 * DP * 4 : 0));
+    if (floatCopy) need += floatCopyBytes(der);
+    size_t freeB = 0, totalB = 0;
+    TBLAEQ_CUDA(cudaMemGetInfo(&freeB, &totalB));
+    if (need > freeB / 2) return;
+    try {
+        if (floatCopy) uploadFloatCopy(idx, der, di, s);
+        di.nodeXF.resize(H - 1);
+        di.radF.resize(H - 1);
+        di.aabbP.resize(H - 1);
+        di.parent.resize(H - 1);
+        di.maxAbs = der.maxAbs;
+        for (uint64_t m = 1; m + 1 < H; ++m) di.parent[m] = upload(der.parent[m], s);
+        di.units = upload(der.units, s);
+        di.unitCount = static_cast<uint32_t>(der.units.size());
+        di.upperUnits = upload(der.upperUnits, s);
+        di.upperUnitCount = static_cast<uint32_t>(der.upperUnits.size());
+        const uint64_t n = idx.meshCount(H - 2), n0 = idx.meshCount(0);
+        for (uint64_t d = 0; d < D; ++d) {
+            double lo = std::numeric_limits<double>::infinity(), hi = -lo;
+            for (uint64_t i = 0; i < n0; ++i) {
+                if (der.ccnt[0][i] == 0) continue;
+                lo = std::min(lo, static_cast<double>(der.aabb[0][i * 2 * D + d]));
+                hi = std::max(hi, static_cast<double>(der.aabb[0][i * 2 * D + D + d]));
+            }
+            const double ext = hi - lo;
+            di.gridMin[d] = ext > 0.0 && std::isfinite(ext) ? lo : 0.0;
+            di.gridScale[d] = ext > 0.0 && std::isfinite(ext) ? kRangeGrid / ext : 0.0;
+        }
+        std::vector<uint32_t> grid(n * DP, 0u);
+        for (uint64_t i = 0; i < n; ++i) {
+            for (uint64_t d = 0; d < DP; ++d) {
+                uint32_t l = 0, h = 0;
+                if (d < D) {
+                    const float* b = &der.aabb[H - 2][i * 2 * D];
+                    l = rangeGridLower(b[d], di.gridMin[d], di.gridScale[d]);
+                    h = rangeGridUpper(b[D + d], di.gridMin[d], di.gridScale[d]);
+                }
+                grid[i * DP + d / 2] |= l << (16 * (d & 1));
+                grid[i * DP + DP / 2 + d / 2] |= (h | 0x8000u) << (16 * (d & 1));
+            }
+        }
+        di.clusterGrid = upload(grid, s);
+        TBLAEQ_CUDA(cudaStreamSynchronize(s));
+        for (uint64_t m = 0; m + 1 < H; ++m) {
+            const size_t n = der.cbeg[m].size();
+            // Padded float centres and rounded-up subtree radii, for the KNN probe and sweep.
+            std::vector<float> xf(n * DP, 0.f), rf(n);
+            for (size_t i = 0; i < n; ++i) {
+                for (uint64_t d = 0; d < D; ++d) xf[i * DP + d] = static_cast<float>(der.nodeX[m][i * D + d]);
+                float r = static_cast<float>(der.radSub[m][i]);
+                if (static_cast<double>(r) < der.radSub[m][i]) r = std::nextafter(r, std::numeric_limits<float>::infinity());
+                rf[i] = r;
+            }
+            di.nodeXF[m] = upload(xf, s);
+            di.radF[m] = upload(rf, s);
+            std::vector<float> bp;
+            if (DP != D) {
+                bp.assign(n * 2 * DP, 0.f);
+                for (size_t i = 0; i < n; ++i)
+                    for (uint64_t d = 0; d < D; ++d) {
+                        bp[i * 2 * DP + d] = der.aabb[m][i * 2 * D + d];
+                        bp[i * 2 * DP + DP + d] = der.aabb[m][i * 2 * D + D + d];
+                    }
+                di.aabbP[m] = upload(bp, s);
+            }
+            TBLAEQ_CUDA(cudaStreamSynchronize(s));
+        }
+        di.sweeps = true;
+    } catch (const CudaError& e) {
+        if (e.code != cudaErrorMemoryAllocation) throw;
+        for (auto* v : {&di.nodeXF, &di.radF, &di.aabbP, &di.parent}) v->clear();
+        for (DeviceMem* m : {&di.units, &di.upperUnits, &di.clusterGrid}) m->release();
+        if (floatCopy)
+            for (DeviceMem* m : {&di.pointsF, &di.pointPerm, &di.groupRec, &di.groupBox, &di.clusterGroups}) m->release();
+    }
+}
+
+}  // namespace
+
 std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const DerivedArrays& der, cudaStream_t s,
                                               const std::vector<int>& residency) {
     if (!residency.empty() && residency.size() != idx.intervals)
@@ -480,45 +591,6 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
     di->leaf.resize(idx.height - 1);
     di->aabb.resize(idx.height - 1);
     di->nodeX.resize(idx.height - 1);
-    di->nodeXF.resize(idx.height - 1);
-    di->radF.resize(idx.height - 1);
-    di->aabbP.resize(idx.height - 1);
-    di->maxAbs = der.maxAbs;
-    di->parent.resize(idx.height - 1);
-    for (uint64_t m = 1; m + 1 < idx.height; ++m) di->parent[m] = upload(der.parent[m], s);
-    di->units = upload(der.units, s);
-    di->unitCount = static_cast<uint32_t>(der.units.size());
-    di->upperUnits = upload(der.upperUnits, s);
-    if (idx.D <= 32) {
-        const uint64_t D = idx.D, DP = paddedDims(D), n = idx.meshCount(idx.height - 2), n0 = idx.meshCount(0);
-        for (uint64_t d = 0; d < D; ++d) {
-            double lo = std::numeric_limits<double>::infinity(), hi = -lo;
-            for (uint64_t i = 0; i < n0; ++i) {
-                if (der.ccnt[0][i] == 0) continue;
-                lo = std::min(lo, static_cast<double>(der.aabb[0][i * 2 * D + d]));
-                hi = std::max(hi, static_cast<double>(der.aabb[0][i * 2 * D + D + d]));
-            }
-            const double ext = hi - lo;
-            di->gridMin[d] = ext > 0.0 && std::isfinite(ext) ? lo : 0.0;
-            di->gridScale[d] = ext > 0.0 && std::isfinite(ext) ? kRangeGrid / ext : 0.0;
-        }
-        std::vector<uint32_t> grid(n * DP, 0u);
-        for (uint64_t i = 0; i < n; ++i) {
-            for (uint64_t d = 0; d < DP; ++d) {
-                uint32_t l = 0, h = 0;
-                if (d < D) {
-                    const float* b = &der.aabb[idx.height - 2][i * 2 * D];
-                    l = rangeGridLower(b[d], di->gridMin[d], di->gridScale[d]);
-                    h = rangeGridUpper(b[D + d], di->gridMin[d], di->gridScale[d]);
-                }
-                grid[i * DP + d / 2] |= l << (16 * (d & 1));
-                grid[i * DP + DP / 2 + d / 2] |= (h | 0x8000u) << (16 * (d & 1));
-            }
-        }
-        di->clusterGrid = upload(grid, s);
-        TBLAEQ_CUDA(cudaStreamSynchronize(s));
-    }
-    di->upperUnitCount = static_cast<uint32_t>(der.upperUnits.size());
     for (uint32_t n : der.ccnt[idx.height - 2]) di->maxCluster = std::max(di->maxCluster, n);
     for (uint64_t m = 0; m + 1 < idx.height; ++m) {
         const size_t n = der.cbeg[m].size();
@@ -532,27 +604,6 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
         di->leaf[m] = upload(der.leaf[m], s);
         di->aabb[m] = upload(der.aabb[m], s);
         di->nodeX[m] = upload(der.nodeX[m], s);
-        // Padded float centres and rounded-up subtree radii, for the KNN probe and sweep.
-        const uint64_t DP = paddedDims(idx.D);
-        std::vector<float> xf(n * DP, 0.f), rf(n);
-        for (size_t i = 0; i < n; ++i) {
-            for (uint64_t d = 0; d < idx.D; ++d) xf[i * DP + d] = static_cast<float>(der.nodeX[m][i * idx.D + d]);
-            float r = static_cast<float>(der.radSub[m][i]);
-            if (static_cast<double>(r) < der.radSub[m][i]) r = std::nextafter(r, std::numeric_limits<float>::infinity());
-            rf[i] = r;
-        }
-        di->nodeXF[m] = upload(xf, s);
-        di->radF[m] = upload(rf, s);
-        std::vector<float> bp;
-        if (DP != idx.D) {
-            bp.assign(n * 2 * DP, 0.f);
-            for (size_t i = 0; i < n; ++i)
-                for (uint64_t d = 0; d < idx.D; ++d) {
-                    bp[i * 2 * DP + d] = der.aabb[m][i * 2 * idx.D + d];
-                    bp[i * 2 * DP + DP + d] = der.aabb[m][i * 2 * idx.D + idx.D + d];
-                }
-            di->aabbP[m] = upload(bp, s);
-        }
         TBLAEQ_CUDA(cudaStreamSynchronize(s));
     }
     if (!der.pointsD.empty() && idx.intervals > 0 && res(idx.intervals - 1) == kResident) {
@@ -563,28 +614,13 @@ std::unique_ptr<DeviceIndex> buildDeviceIndex(const HostIndex& idx, const Derive
     // the device even when those rows are streamed, as long as they take at most a quarter of the
     // free memory: the exact range batch then decides nearly every point on the device and reads
     // a row across the host link only near a face of a box.
-    bool floatCopy = !der.pointsF.empty() && idx.intervals > 0;
-    if (floatCopy && res(idx.intervals - 1) != kResident) {
-        const size_t need = der.pointsF.size() * 4 + der.pointPerm.size() * 4 + der.groupBox.size() * 4 +
-                            der.groupFirst.size() * 16 + der.clusterGroup.size() * 16;
+    const bool resident = idx.intervals > 0 && res(idx.intervals - 1) == kResident;
+    if (floatPointsSupported(idx.D) && !der.pointsF.empty() && idx.intervals > 0) {
         size_t freeB = 0, totalB = 0;
         TBLAEQ_CUDA(cudaMemGetInfo(&freeB, &totalB));
-        floatCopy = need * 4 <= freeB;
+        if (resident || floatCopyBytes(der) * 4 <= freeB) uploadFloatCopy(idx, der, *di, s);
     }
-    if (floatCopy) {
-        di->pointsF = upload(der.pointsF, s);
-        di->pointPerm = upload(der.pointPerm, s);
-        const size_t G = der.groupFirst.size(), nCl = der.clusterGroup.size() - 1;
-        std::vector<NodeRec> grec(G), crec(nCl);
-        for (size_t g = 0; g < G; ++g) grec[g] = NodeRec{0.0, der.groupFirst[g], der.groupCount[g]};
-        for (size_t c = 0; c < nCl; ++c)
-            crec[c] = NodeRec{der.radSub[idx.height - 2][c], der.clusterGroup[c],
-                              der.clusterGroup[c + 1] - der.clusterGroup[c]};
-        di->groupRec = upload(grec, s);
-        di->groupBox = upload(der.groupBox, s);
-        di->clusterGroups = upload(crec, s);
-        TBLAEQ_CUDA(cudaStreamSynchronize(s));
-    }
+    if (der.sweeps && resident) uploadSweepArrays(idx, der, *di, s);
     TBLAEQ_CUDA(cudaStreamSynchronize(s));
     return di;
 }

@@ -124,6 +124,7 @@ struct DerivedArrays {
     // point-group order where floatPointsSupported(D) (pointPerm maps back to rows), else in row order.
     std::vector<double> pointsD;
     double maxAbs = 0.0;                 // largest |coordinate| of any mesh
+    bool sweeps = false;                 // the arrays of the sweeps (parent, units; groups at any D) are there
     // Parent position of every node (mesh m: position in mesh m-1; mesh 0 empty), meshes 0 .. height-2.
     std::vector<std::vector<uint32_t>> parent;
     std::vector<RangeUnit> units;        // the finest clusters in traversal order, see rangesweep.cuh
@@ -135,7 +136,8 @@ constexpr uint32_t kPointGroup = 32;
 
 // Host computation of the position-space node arrays, including subtree radii from the decoded
 // hierarchy (decoded exactly like the traversal: y = P[j] * x_parent, one rounded multiply).
-DerivedArrays computeDerived(const HostIndex& idx);
+// `resident`: the last interval's rows are to be on the device, which the sweeps need.
+DerivedArrays computeDerived(const HostIndex& idx, bool resident);
 
 // A page-locked host range mapped into the device address space (zero-copy reads by kernels);
 // unregistered when destroyed. The host memory must outlive it and must not move.
@@ -183,6 +185,7 @@ struct DeviceIndex {
     std::vector<DeviceMem> aabb;             // mesh m < height-1: outward-rounded float box of the points below
     std::vector<DeviceMem> nodeX;            // mesh m < height-1: decoded coordinates (D doubles per node)
     std::vector<DeviceMem> nodeXF, radF;     // mesh m < height-1: the same as padded floats; subtree radius, rounded up
+    bool sweeps = false;                     // nodeXF, radF, aabbP, parent, units and grid are there
     double maxAbs = 0.0;                     // largest |coordinate| of any mesh
     std::vector<DeviceMem> parent;           // mesh 1 <= m < height-1: position of each node's parent (uint32)
     DeviceMem units;                         // RangeUnit: the finest clusters in traversal order

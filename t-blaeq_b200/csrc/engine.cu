@@ -535,7 +535,7 @@ void BatchEngine::enqueueNodeMajorLevel(int m, int buf, const double* dBoxes, ui
 bool BatchEngine::useRangeSweep(uint32_t nq, int mode, unsigned flags) const {
     // Per-level counts per query, chosen launch shapes and the tests switched off all ask for the
     // level-synchronous launches, and so does a streamed last interval (no decoded points on the device).
-    if (mode != kModeExact || (flags & kWantLevels) || nq == 0 || rsOff_ || rsSkip_ || !floatPoints_ || !pointGroups_ ||
+    if (!di_.sweeps || mode != kModeExact || (flags & kWantLevels) || nq == 0 || rsOff_ || rsSkip_ || !floatPoints_ || !pointGroups_ ||
         lookbackTestHookSet() || di_.height < 2 || di_.height > kRangeMaxHeight || !di_.pointsF.bytes() ||
         !di_.pointsD.bytes() || di_.unitCount == 0 ||
         (!floatPointsSupported(di_.D) && di_.maxCluster > kRangeRowsCluster))
@@ -1517,7 +1517,7 @@ bool BatchEngine::growKnnMajor() {
 bool BatchEngine::useKnnSweep(unsigned flags, uint32_t maxK) const {
     // Per-level counts and the scorer's training traces describe the level-synchronous walk, and so do
     // the options that change it; a streamed last interval has no decoded points on the device.
-    return twoWave_ && knnNodeMajor_ && probeBeam_ > 0 && knnGroups_ && !knnTrace_ && !(flags & kWantLevels) &&
+    return di_.sweeps && twoWave_ && knnNodeMajor_ && probeBeam_ > 0 && knnGroups_ && !knnTrace_ && !(flags & kWantLevels) &&
            di_.height >= 2 && di_.height <= kSweepMaxHeight && di_.pointsD.bytes() && di_.pointsF.bytes() &&
            di_.maxAbs <= kSweepMaxAbs && maxK <= kProbePoints / 2;
 }

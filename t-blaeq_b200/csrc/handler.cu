@@ -142,12 +142,12 @@ void QueryHandler::prepareForQuery(const IndexPolicy& policy) {
     auto rt = std::make_unique<Runtime>();
     rt->host = host_.get();
     TBLAEQ_CUDA(cudaStreamCreateWithFlags(&rt->stream, cudaStreamNonBlocking));
-    const DerivedArrays der = computeDerived(*host_);
     std::vector<int> residency(host_->intervals, kResident);
     for (size_t l = 0; l < residency.size(); ++l) {
         if (policy.levels[l] == LevelPolicy::L2) residency[l] = kRowsOnHost;
         if (policy.levels[l] == LevelPolicy::L3) residency[l] = kRowsAndMapOnHost;
     }
+    const DerivedArrays der = computeDerived(*host_, !residency.empty() && residency.back() == kResident);
     rt->dev = buildDeviceIndex(*host_, der, rt->stream, residency);
     rt->engine = std::make_unique<BatchEngine>(*rt->dev, rt->stream);
     rt->pluginEngine = std::make_unique<BatchEngine>(*rt->dev, rt->stream);

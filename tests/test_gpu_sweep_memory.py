@@ -135,3 +135,45 @@ def test_serving_admission_counts_the_sweep(tb, cuda):
             s = srv.stats()
             assert s["completed"] == n and s["failed"] == 0
             assert wave == 0 or s["max_batch"] < 700
+
+
+@pytest.mark.parametrize("D", [5, 8])
+def test_index_without_memory_for_the_sweep_arrays(tb, oracle_mod, cuda, D):
+    """What only the sweeps read is optional: an index whose last uploads are refused prepares and answers
+    by the level-synchronous launches."""
+    lib, N = tb.lib(), 20_000
+
+    def make():
+        return tb.QueryHandler.generate(N, D, 1.0, 100.0, False, 4, (40, 20, 5), 3, 2.5)
+
+    h = make()
+    at = lib.tblaeq_live_device_bytes()
+    h.prepare_for_query(tb.LevelPolicy.L0)
+    whole = lib.tblaeq_live_device_bytes() - at
+    pts, ids = h.decode_points(np.arange(N))
+    P = np.ascontiguousarray(pts[:60] + 0.5)
+    Q = np.ascontiguousarray(np.concatenate([P - 12.0, P + 12.0], 1))
+    want, near = _levels(tb, h, Q), _brute(oracle_mod, pts, ids, P, 9)
+    h.close()
+    failed = served = 0
+    for nth in range(1, 200):
+        g = make()
+        at = lib.tblaeq_live_device_bytes()
+        lib.tblaeq_debug_fail_alloc_after(nth)
+        try:
+            g.prepare_for_query(tb.LevelPolicy.L0)
+        except tb.TblaeqError as e:
+            assert e.code == 4 and lib.tblaeq_live_device_bytes() == at
+            failed += 1
+            continue
+        finally:
+            lib.tblaeq_debug_fail_alloc_after(0)
+        held = lib.tblaeq_live_device_bytes() - at
+        if held == whole:  # every allocation was granted
+            break
+        assert held < whole
+        _same(_range(tb, g, Q), want)
+        _equal(_knn(tb, g, P, 9), near)
+        served += 1
+        g.close()
+    assert failed >= 10 and served >= 10
