@@ -649,32 +649,32 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
 }
 
 // ---- gather ---------------------------------------------------------------------------------------
-constexpr int kGatherThreads = 128;
 
 // One block per (query, share of its results). Orders the query's segments by key (counting for a few,
 // a bitonic network for many), then every thread finds its results' segments by bisection.
-__global__ void __launch_bounds__(kGatherThreads) rangeGatherKernel(RangeSweepArgs a, uint32_t shares, uint32_t slotCap,
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) rangeGatherKernel(RangeSweepArgs a, uint32_t shares, uint32_t slotCap,
                                                                    int scanned) {
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* sKey = reinterpret_cast<uint64_t*>(smem);
     uint32_t* sSlot = reinterpret_cast<uint32_t*>(sKey + slotCap);
     uint32_t* sEnd = sSlot + slotCap;  // inclusive lengths, in order (a segment's first hit then replaces its slot)
     __shared__ unsigned long long sBase;
-    __shared__ unsigned long long sWarp[kGatherThreads / 32];
-    __shared__ uint32_t sCarry, sW32[kGatherThreads / 32];
+    __shared__ unsigned long long sWarp[THREADS / 32];
+    __shared__ uint32_t sCarry, sW32[THREADS / 32];
     const uint32_t q = blockIdx.x / shares, share = blockIdx.x - q * shares;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (*a.status) return;
     // Results of the queries before this one.
     unsigned long long sum = 0;
-    for (uint32_t i = tid; !scanned && i < q; i += kGatherThreads) sum += a.qcount[i];
+    for (uint32_t i = tid; !scanned && i < q; i += THREADS) sum += a.qcount[i];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
     if (lane == 0) sWarp[warp] = sum;
     __syncthreads();
     if (tid == 0) {
         unsigned long long t = 0;
-        for (int i = 0; i < kGatherThreads / 32; ++i) t += sWarp[i];
+        for (int i = 0; i < THREADS / 32; ++i) t += sWarp[i];
         if (scanned) t = a.offsets[q];
         sBase = t;
         if (share == 0) {
@@ -692,8 +692,8 @@ __global__ void __launch_bounds__(kGatherThreads) rangeGatherKernel(RangeSweepAr
     const uint32_t n = min(a.qsegs[q], min(a.segSlots, slotCap));
     const unsigned long long base = sBase;
     if (total == 0 || base + total > a.resultCap) return;
-    const uint32_t per = (total + shares - 1) / shares;
-    const uint32_t r0 = min(total, share * per), r1 = min(total, r0 + per);
+    const uint32_t per = max(8u * THREADS, (total + shares - 1) / shares);
+    const uint32_t r0 = share * per < total ? share * per : total, r1 = min(total, r0 + per);
     if (r0 >= r1) return;
     const RangeSegment* segs = a.segs + static_cast<size_t>(q) * a.segSlots;
     if (n == 1) {
@@ -705,12 +705,12 @@ __global__ void __launch_bounds__(kGatherThreads) rangeGatherKernel(RangeSweepAr
     } else {
         uint32_t size = 1;
         while (size < n) size <<= 1;
-        for (uint32_t i = tid; i < size; i += kGatherThreads) {
+        for (uint32_t i = tid; i < size; i += THREADS) {
             sKey[i] = i < n ? segs[i].key : ~0ull;
             sSlot[i] = i;
         }
         __syncthreads();
-        if (n <= kGatherThreads) {
+        if (n <= THREADS) {
             uint32_t place = 0;
             if (static_cast<uint32_t>(tid) < n) {
                 const uint64_t k = sKey[tid];
@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(kGatherThreads) rangeGatherKernel(RangeSweepAr
         } else {
             for (uint32_t s = 2; s <= size; s <<= 1)
                 for (uint32_t stride = s >> 1; stride > 0; stride >>= 1) {
-                    for (uint32_t t = tid; t < size / 2; t += kGatherThreads) {
+                    for (uint32_t t = tid; t < size / 2; t += THREADS) {
                         const uint32_t lo = 2 * t - (t & (stride - 1)), hi = lo + stride;
                         const bool asc = (lo & s) == 0;
                         if (asc == (sKey[lo] > sKey[hi])) {
@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(kGatherThreads) rangeGatherKernel(RangeSweepAr
                 }
         }
         __syncthreads();
-        for (uint32_t i0 = 0; i0 < n; i0 += kGatherThreads) {
+        for (uint32_t i0 = 0; i0 < n; i0 += THREADS) {
             const uint32_t i = i0 + tid;
             uint32_t inc = i < n ? segs[sSlot[i]].len : 0u;
 #pragma unroll
@@ -754,11 +754,11 @@ __global__ void __launch_bounds__(kGatherThreads) rangeGatherKernel(RangeSweepAr
                 sSlot[i] = segs[sSlot[i]].pos;
             }
             __syncthreads();
-            if (tid == kGatherThreads - 1) sCarry = before + inc;
+            if (tid == THREADS - 1) sCarry = before + inc;
             __syncthreads();
         }
     }
-    for (uint32_t r = r0 + tid; r < r1; r += kGatherThreads) {
+    for (uint32_t r = r0 + tid; r < r1; r += THREADS) {
         uint32_t lo = 0, hi = n - 1;  // the first segment that ends past r
         while (lo < hi) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -802,15 +802,22 @@ void launchPadded(const RangeSweepArgs& a, cudaStream_t s) {
     const uint32_t blocks = std::min<uint32_t>(static_cast<uint32_t>(full), (nTasks + WARPS - 1) / WARPS);
     rangeSweepKernel<DP, ROWS><<<std::max(1u, blocks), WARPS * 32, 0, s>>>(a, nTasks, t.qPer, t.parts);
     TBLAEQ_LAUNCHED();
-    // A few queries may hold many results each: several blocks share a query then.
-    const uint32_t shares = std::max<uint32_t>(1u, 4736u / a.nq);
+    // A few queries may hold many results each, and every block of a query orders all of its segments: large
+    // blocks share a query then, about as many as are resident at once, at least 4,096 results each. 20 boxes
+    // with 6.4M results (N = 1M, D = 2): the gather takes 132 us; 590 us with 236 shares of 128 threads,
+    // 180 us with 88 of 512. 300 boxes with 14.9M: 520 us for the batch with four shares, 630 with one.
+    const bool few = a.nq <= 592;
+    const uint32_t shares = few ? std::max(4u, 592u / a.nq) : std::max<uint32_t>(1u, 4736u / a.nq);
     // Each block sums the counts before its query, unless that many reads would cost more than a scan.
     const bool scanned = a.nq > 8192;
     if (scanned) launchExclusiveScan(a.qcount, a.offsets, a.nq, s);
     const uint32_t slotCap = std::min(a.segSlots, kRangeSegments);
     uint32_t pow2 = 1;
     while (pow2 < slotCap) pow2 <<= 1;
-    rangeGatherKernel<<<a.nq * shares, kGatherThreads, pow2 * 16, s>>>(a, shares, pow2, scanned ? 1 : 0);
+    if (few)
+        rangeGatherKernel<512><<<a.nq * shares, 512, pow2 * 16, s>>>(a, shares, pow2, scanned ? 1 : 0);
+    else
+        rangeGatherKernel<128><<<a.nq * shares, 128, pow2 * 16, s>>>(a, shares, pow2, scanned ? 1 : 0);
     TBLAEQ_LAUNCHED();
 }
 
