@@ -544,7 +544,8 @@ bool BatchEngine::useRangeSweep(uint32_t nq, int mode, unsigned flags) const {
         if (variants_[m] != kVariantDirect || grids_[m] != 100) return false;
     const uint64_t upper = di_.height > 2 ? di_.meshCount[di_.height - 3] : 1;
     return rangeSweepBitBytes(upper, nq) <= (1ull << 30) && nq <= (1u << 21) &&
-           rangeSweepTasks(di_.unitCount, nq).count <= kRangeTasksMax;
+           rangeSweepTasks(di_.unitCount, nq).count <= kRangeTasksMax &&
+           !rangeSweepNarrow(di_.height, di_.meshCount[0], upper, di_.meshCount[di_.height - 2], di_.unitCount, nq);
 }
 
 // Segments of the sweep a query may have: 262,144 over the batch or 64 at first, then what an overflow asked
@@ -1514,7 +1515,15 @@ bool BatchEngine::growKnnMajor() {
     return grew;
 }
 
-bool BatchEngine::useKnnSweep(unsigned flags, uint32_t maxK) const {
+bool BatchEngine::useKnnSweep(uint32_t nq, unsigned flags, uint32_t maxK) const {
+    // A probe reads 32 clusters: where those hold fewer than K points, the bound is loose or missing and the
+    // walk is the faster, unless the index is so small that the candidate slots hold it all (41 queries of K =
+    // 600, fan-outs 4 and 3: N = 60,000 1.8 ms against the walk's 5, N = 600,000 18 against 11; 300 queries of K
+    // = 170, fan-outs 5, N = 1M: 133 against 29; at K = 155 the sweep is the faster). So it is for a few queries
+    // over a wide mesh 0, which one CTA a query ranks (one query, 111,000 nodes: 411 us against 336; ten: as fast).
+    const uint64_t nodes = di_.meshCount[0], clusters = di_.meshCount[di_.height - 2], points = di_.meshCount[di_.height - 1];
+    if (static_cast<uint64_t>(maxK) * clusters > 32 * points && points > kSweepFactorMax * (4ull * maxK + 64)) return false;
+    if (di_.height > 2 && nodes > 65536 && nq < 8) return false;
     // Per-level counts and the scorer's training traces describe the level-synchronous walk, and so do
     // the options that change it; a streamed last interval has no decoded points on the device.
     return di_.sweeps && twoWave_ && knnNodeMajor_ && probeBeam_ > 0 && knnGroups_ && !knnTrace_ && !(flags & kWantLevels) &&
@@ -1764,7 +1773,7 @@ BatchOutput BatchEngine::runKnn(const double* dPoints, uint32_t nq, const uint32
     WorkspaceGuard guard(*this);
     reserve(caps_, nq, flags);
     swLast_ = false;
-    if (nq > 0 && useKnnSweep(flags, maxK)) {
+    if (nq > 0 && useKnnSweep(nq, flags, maxK)) {
         BatchOutput o;
         if (runKnnSweep(dPoints, nq, dK, sumK, o)) return o;
     }

@@ -302,7 +302,7 @@ private:
     uint32_t swFactor_ = 1;     // 1, 4, 16 or 64: see runKnnSweep
     bool swCandGrown_ = false;  // swCand_ holds more than batches without many ties ask for
     bool swLast_ = false, knnTrace_ = false;
-    bool useKnnSweep(unsigned flags, uint32_t maxK) const;
+    bool useKnnSweep(uint32_t nq, unsigned flags, uint32_t maxK) const;
     uint32_t knnSweepBlock(uint32_t nq) const;
     bool reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand);  // false: no memory for it
     void enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint32_t factor, bool grown);

@@ -82,6 +82,22 @@ inline RangeSweepTasks rangeSweepTasks(uint64_t nUnits, uint64_t nq) {
     return t;
 }
 
+// Whether the level-synchronous launches serve a batch sooner than the sweep: on indexes of small fan-outs,
+// whose units are mostly empty lanes and whose last upper mesh is most of the hierarchy. `top`, `upper` and
+// `clusters` are the nodes of mesh 0, the last upper mesh and the finest clusters. Three cases, each on
+// an index of many units and fewer than twelve clusters a node, measured as sweep / levels in us:
+// - few queries: 0.8 ns a task against about 40 us of saved launches and, a query, 0.01 ns a node of mesh 0
+//   and 0.3 us. One box: fan-outs 2, N = 1M, D = 8: 801 / 96; fan-outs 4, D = 5, N = 2M: 411 / 79; fan-outs
+//   6, N = 1M: 125 / 100. 100 boxes there: 108 / 167 with fan-outs 6, 170 / 186 with 4.
+// - fan-outs below four: 8,000 boxes, fan-outs 2, N = 1M: 12,028 / 9,612; fan-outs 3, N = 3M: 8,444 / 5,489;
+//   fan-outs 4, N = 1M: 2,122 / 2,388.
+// - five meshes and more, below eight: fan-outs 5, N = 1M: 100 boxes 136 / 174, 1,000 398 / 293, 8,000 2,400 / 1,080.
+inline bool rangeSweepNarrow(uint64_t height, uint64_t top, uint64_t upper, uint64_t clusters, uint64_t nUnits, uint64_t nq) {
+    if (height <= 2 || nUnits <= 16384 || clusters >= 12 * upper) return false;
+    return rangeSweepTasks(nUnits, nq).count > 50000 + nq * (375 + 12 * top / 1000) ||
+           (clusters < 4 * upper && (nUnits > 65536 || nq >= 2048)) || (height >= 5 && clusters < 8 * upper && nq >= 512);
+}
+
 struct RangeSegment {
     uint64_t key;  // unit, then the run's number within it
     uint32_t pos;  // first hit

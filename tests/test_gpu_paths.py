@@ -126,3 +126,32 @@ def test_walk_wave_one(tb, walk):
     finally:
         h.set_knn_wave1(16.0)
     assert len(set(rows.values())) == 3, rows
+
+
+@pytest.mark.parametrize("D,N,ratios,nq,sweeps", [(3, 1_000_000, (2, 2, 2), 1, False), (3, 1_000_000, (2, 2, 2), 3000, False),
+                                                  (3, 500_000, (4, 4), 1, False), (3, 500_000, (4, 4), 600, True),
+                                                  (3, 2_000_000, (5, 5, 3, 3), 700, False), (3, 1_000_000, (100, 2, 2), 1, True)])
+def test_narrow_indexes(tb, cuda, D, N, ratios, nq, sweeps):
+    """Small fan-outs over many nodes: the level-synchronous launches, with the sweep's results."""
+    h, pts = _index(tb, D, N, ratios)
+    Q = _boxes(pts, nq, 5, 0.001, 0.01)
+    assert (_launches(tb, h, tb.QueryType.RANGE, Q) == 3) == sweeps
+    r = h.query_batch(tb.QueryType.RANGE, Q, tb.Mode.EXACT)
+    offs, ids = r.offsets.numpy().astype(np.int64), r.ids.numpy()
+    names = h.decode_points(np.arange(N))[1]
+    for q in (0, nq // 2, nq - 1):
+        inside = names[((pts >= Q[q, :D]) & (pts <= Q[q, D:])).all(1)]
+        assert np.array_equal(np.sort(ids[offs[q]:offs[q + 1]]), np.sort(inside))
+
+
+@pytest.mark.parametrize("N,ratios,nq,K,sweeps", [(500_000, (5, 5), 40, 165, False), (500_000, (5, 5), 40, 155, True),
+                                                  (2_000_000, (3, 3, 3), 1, 2, False), (2_000_000, (3, 3, 3), 8, 2, True)])
+def test_knn_paths_of_small_fan_outs(tb, oracle_mod, cuda, N, ratios, nq, K, sweeps):
+    h, pts = _index(tb, 4, N, ratios)
+    ids = h.decode_points(np.arange(N))[1]
+    P = np.ascontiguousarray(pts[::N // nq][:nq] + 0.2)
+    launches = _launches(tb, h, tb.QueryType.POINT, P, K)
+    assert (launches <= 10) == sweeps  # five, and five more where slots grow
+    r = h.query_batch(tb.QueryType.POINT, P, tb.Mode.EXACT, K=K)
+    b = oracle_mod.brute_query(pts, ids, oracle_mod.KNN, P, K=K)
+    assert np.array_equal(r.ids.numpy(), b.ids) and np.array_equal(r.dist2.numpy(), b.dist2)

@@ -8,14 +8,14 @@ pytestmark = pytest.mark.gpu
 
 
 def test_range_over_many_upper_nodes(tb, cuda):
-    """Fan-outs of two: 280,000 parents, four a block, are more blocks than a y axis has (65,535). Wide
-    boxes have more segments than the gather orders and end in the level launches, narrow ones sweep."""
-    N = 2_240_000
-    h = tb.QueryHandler.generate(N, 1, 1.0, 100.0, False, 4, (2, 2, 2), 5, 2.5)
+    """270,000 parents, four a block, are more blocks than a y axis has (65,535). Wide boxes have more segments
+    than the gather orders and end in the level launches, narrow ones sweep."""
+    N = 4_320_000
+    h = tb.QueryHandler.generate(N, 1, 1.0, 100.0, False, 4, (2, 4, 2), 5, 2.5)
     h.prepare_for_query(tb.LevelPolicy.L0)
-    assert 280_000 in h.info()["meshSizes"]
+    assert 270_000 in h.info()["meshSizes"]
     rng = np.random.default_rng(2)
-    c = h.decode_points(rng.integers(0, N, 70))[0]
+    c = h.decode_points(rng.integers(0, N, 300))[0]
     for widest in (1e-5, 1e-2):
         hw = np.exp(rng.uniform(np.log(1e-6), np.log(widest), c.shape)) * 100
         Q = np.ascontiguousarray(np.concatenate([c - hw, c + hw], 1))
@@ -28,7 +28,7 @@ def test_range_over_many_upper_nodes(tb, cuda):
         r = h.query_batch(tb.QueryType.RANGE, Q, tb.Mode.EXACT)
         h.set_launch_shapes([0] * 4, [100] * 4)
         assert np.array_equal(got[0], r.offsets.numpy()) and np.array_equal(got[1], r.ids.numpy())
-        assert got[2] == h.level_counts() and got[0][-1] >= 70
+        assert got[2] == h.level_counts() and got[0][-1] >= 300
 
 
 def test_knn_over_many_queries(tb, cuda):
