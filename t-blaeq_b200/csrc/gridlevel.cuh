@@ -18,8 +18,17 @@
 namespace tblaeq {
 
 // Largest grid of this path: the sums take p^2 / 2 comparisons (16,384 entries: 134M) and one CTA scans
-// the kept counts. Larger grids sort.
+// the kept counts. Larger grids sort, and from half of that on those whose K reaches far into the grid, as the
+// sums end at K: above an eighth of its children (estimated from the meshes' sizes). Counted / sorted, a call:
+// 8,000 entries, K = all 1M children: 150 / 192 us; 16,129 entries, K = 3% 196 / 197, all 322 / 225; 15,625
+// entries, K = 2% 485 / 507, half 614 / 544. (At D = 32, where the sorted path's expands carry long rows, 507 / 714
+// for all of 16,129 entries.)
 constexpr uint64_t kGridLevelMax = 16384;
+inline bool gridLevelCounts(uint64_t p, uint64_t D, bool knn, uint64_t K, uint64_t nodes, uint64_t children) {
+    if (p == 0 || p > kGridLevelMax) return false;
+    return !knn || p <= kGridLevelMax / 2 || D >= 16 || static_cast<double>(K) * static_cast<double>(nodes) * 8.0 <=
+                                                 static_cast<double>(p) * static_cast<double>(children);
+}
 
 struct GridLevelArgs {
     const uint64_t* ids;

@@ -180,7 +180,8 @@ LevelResult B200Strategy::runLevel(size_t l, SparseGrid* curGrid, QueryType qTyp
         out.cap = cap;
     }
     uint64_t n = 0;
-    if (cur.nnz > 0 && cur.nnz <= kGridLevelMax && D <= 32 && !lookbackTestHookSet()) {
+    const bool counted = gridLevelCounts(cur.nnz, D, qType != QueryType::RANGE, K, h.meshCount(l), h.meshCount(l + 1));
+    if (counted && D <= 32 && !lookbackTestHookSet()) {
         GridLevelArgs a{};
         a.ids = cur.ids;
         a.vals = cur.vals;
