@@ -1544,6 +1544,7 @@ bool BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand) {
     const uint32_t block = knnSweepBlock(nq);
     const uint64_t words = block <= 32 ? 1 : (((static_cast<uint64_t>(block) + 31) / 32 + 3) / 4 * 4);
     const uint64_t results = std::max<uint64_t>(sumK, 1);
+    const uint64_t live = align256(nC * 4 + 256) + (DP <= 8 && block > kSweepSliced ? nC * ((words + 31) / 32) * sizeof(uint4) : 0);
     uint64_t entries = 0;
     if (scorer_) {
         // The clusters under the beam: probeBeam_ nodes' children per query, grown on overflow.
@@ -1562,7 +1563,7 @@ bool BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand) {
                 // counts and wants, entry offsets and counts (4 bytes)
                 {&swQuery_, (static_cast<uint64_t>(nq) + 1) * (3 * 8 + DP * 4 + 7 * 4) + 1024, swQcap_ < nq},
                 {&swBits_, nC * words * 4, swBits_.bytes() < nC * words * 4},
-                {&swLive_, nC * 4 + 256, swLive_.bytes() < nC * 4 + 256},
+                {&swLive_, live, swLive_.bytes() < live},
                 {&swCand_, cand * 16, shrink || swCandCap_ < cand},
                 {&swEnt_, entries * (4 + 4 + 8), swEnt_.bytes() < entries * (4 + 4 + 8)},
                 {&knnIds_, results * 8, knnCap_ < results},
@@ -1605,9 +1606,8 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
     const uint64_t D = di_.D, DP = paddedDims(D);
     char* z = zeroBlock_.as<char>();
     if (timing_) record(0);
-    // Tickets, status, headers and the work counters (neighbours in the block).
+    // Tickets, status and headers (neighbours in the block).
     TBLAEQ_CUDA(cudaMemsetAsync(z + offTickets_, 0, offQcount_ - offTickets_, stream_));
-    TBLAEQ_CUDA(cudaMemsetAsync(z + offWork_, 0, 16, stream_));
     KnnSweepArgs a{};
     a.D = static_cast<int>(D);
     a.height = H;
@@ -1653,7 +1653,11 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
     a.waveFactor = waveScale_ * static_cast<double>(di_.meshCount[H - 2]) / static_cast<double>(di_.meshCount[H - 1]);
     a.liveCnt = swLive_.as<uint32_t>();
     a.ticket = a.liveCnt + 1;
+    a.heavyCnt = a.liveCnt + 2;
+    a.heavyTicket = a.liveCnt + 3;
+    a.reached = reinterpret_cast<unsigned long long*>(a.liveCnt + 4);
     a.live = a.liveCnt + 64;
+    a.heavy = reinterpret_cast<uint4*>(swLive_.as<char>() + align256(di_.meshCount[H - 2] * 4 + 256));
     a.bits = swBits_.as<uint32_t>();
     a.hdr = hdrPtr(0);
     a.work = reinterpret_cast<unsigned long long*>(z + offWork_);
@@ -1685,7 +1689,8 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
         a.qEnd = std::min(nq, q0 + block);
         const uint32_t n = a.qEnd - q0;
         a.words = n <= 32 ? 1 : ((n + 31) / 32 + 3) / 4 * 4;
-        if (q0) TBLAEQ_CUDA(cudaMemsetAsync(a.liveCnt, 0, 8, stream_));  // live clusters and the ticket
+        a.sliced = DP <= 8 && n > kSweepSliced;
+        if (q0) TBLAEQ_CUDA(cudaMemsetAsync(a.liveCnt, 0, 24, stream_));  // live clusters, slices, the tickets, bits set
         launchKnnSweepBound(a, stream_);
         launchKnnSweepPoints(a, stream_);
     }

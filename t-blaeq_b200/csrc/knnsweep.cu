@@ -49,6 +49,10 @@ __global__ void __launch_bounds__(1024) sweepPrepareKernel(KnnSweepArgs a, uint3
         sCarryR = sCarryC = 0;
         *a.liveCnt = 0;
         *a.ticket = 0;
+        *a.heavyCnt = 0;
+        *a.heavyTicket = 0;
+        *a.reached = 0;
+        a.work[0] = a.work[1] = 0;
     }
     __syncthreads();
     for (uint32_t base = 0; base < a.nq; base += blockDim.x) {
@@ -505,7 +509,10 @@ __global__ void __launch_bounds__(kBoundThreads) knnBoundBitsKernel(const __grid
     constexpr int W = STEPS <= 2 ? kBoundWords : kBoundWords / 2;  // words staged at once (48 KB of shared memory)
     __shared__ __align__(16) float4 sB[W][4][STEPS][32];  // hi, hi, lo, lo of a lane's two dimensions
     __shared__ __align__(8) float2 sE[W][4][32];
+    __shared__ unsigned long long sReached;
     if (*a.status & ~kStatusOverflowItems) return;
+    uint32_t reached = 0;  // pairs whose bit is set
+    if (threadIdx.x == 0) sReached = 0;
     const KnnSweepLevel& L = a.level[a.height - 2];
     const uint32_t w0 = blockIdx.y * kBoundWords;
     const uint32_t left = a.qEnd - a.qBegin > w0 * 32 ? a.qEnd - a.qBegin - w0 * 32 : 0u;  // queries from w0 on
@@ -620,6 +627,7 @@ __global__ void __launch_bounds__(kBoundThreads) knnBoundBitsKernel(const __grid
                 const uint32_t near = quadTranspose(~bytes, j);
                 word[w] = valid ? near : 0u;
                 any |= word[w];
+                reached += __popc(word[w]);
             }
             if (c < c1) {
                 uint32_t* out = a.bits + static_cast<size_t>(c) * a.words + w0 + wb;
@@ -649,6 +657,11 @@ __global__ void __launch_bounds__(kBoundThreads) knnBoundBitsKernel(const __grid
             }
         }
     }
+    if (!a.sliced) return;
+    reached = __reduce_add_sync(FULL, reached);
+    if (lane == 0) atomicAdd(&sReached, static_cast<unsigned long long>(reached));
+    __syncthreads();
+    if (tid == 0 && sReached) atomicAdd(a.reached, sReached);
 }
 
 // ---- sweep ----------------------------------------------------------------------------------------
@@ -679,7 +692,15 @@ __device__ __noinline__ bool measure(const KnnSweepArgs& a, uint32_t row, uint32
 
 // Deals the clusters to the warps and hands each cluster's queries (the set bits of its row) to
 // batch(cluster, first list entry, n <= 32).
-template <class Batch>
+//
+// SLICED: in batches above kSweepSliced queries, 32 words of a cluster with more than that many, in a cluster
+// of more than twice what a warp would have if all were dealt out evenly, are left to a second launch
+// (sweepSlices). A batch whose queries lie together, or far outside the data, reaches a hundred clusters with
+// nearly all of its queries; one warp for each of those took 11.9 ms (4,096 queries, K = 100, N = 1M, D = 3;
+// the level-synchronous walk 4.9) where spread queries take 0.36. In slices it takes 0.76; the second launch
+// costs 2 to 5 us where there are none. (Taken by the same launch's warps as they run out of clusters it took
+// 18 ms: most have left when the first slice appears.)
+template <bool SLICED, class Batch>
 __device__ __forceinline__ void sweepClusters(const KnnSweepArgs& a, uint32_t* list, Batch&& batch) {
     const int lane = threadIdx.x & 31;
     const bool listed = a.qEnd - a.qBegin <= kBoundWords * 32;
@@ -709,6 +730,11 @@ __device__ __forceinline__ void sweepClusters(const KnnSweepArgs& a, uint32_t* l
             }
             const uint32_t add = __shfl_sync(FULL, inc, 31);
             if (add == 0) continue;
+            if (SLICED && add > kSweepSliced && a.sliced &&
+                static_cast<uint64_t>(add) * ((a.words + 31u) / 32u) * kSweepWarps * gridDim.x > 2ull * *a.reached) {
+                if (lane == 0) a.heavy[atomicAdd(a.heavyCnt, 1u)] = make_uint4(c, w0, add, 0u);
+                continue;
+            }
             uint32_t at = n + inc - own;
             const uint32_t q0 = a.qBegin + (w0 + lane) * 32;
             while (word) {
@@ -731,6 +757,37 @@ __device__ __forceinline__ void sweepClusters(const KnnSweepArgs& a, uint32_t* l
         }
         const uint32_t full = n / 32 * 32;
         if (n > full) batch(c, full, n - full);
+        __syncwarp();
+    }
+}
+
+// What sweepClusters left, in slices of one to sixteen words with about kSweepSlice queries, a warp each.
+constexpr uint32_t kSweepSlice = 64;
+template <class Batch>
+__device__ __forceinline__ void sweepSlices(const KnnSweepArgs& a, uint32_t* list, Batch&& batch) {
+    const uint32_t lane = threadIdx.x & 31, total = *a.heavyCnt * 32u;
+    while (true) {
+        uint32_t t = 0;
+        if (lane == 0) t = atomicAdd(a.heavyTicket, 1u);
+        t = __shfl_sync(FULL, t, 0);
+        if (t >= total) break;
+        const uint4 e = a.heavy[t / 32u];  // cluster, first word, queries
+        const uint32_t per = (32u * kSweepSlice + e.z - 1u) / e.z, w0 = e.y + t % 32u * per;
+        const uint32_t w1 = min(min(e.y + 32u, a.words), w0 + per);
+        if (t % 32u * per >= 32u || w0 >= w1) continue;  // the entry has fewer slices
+        uint32_t word = w0 + lane < w1 ? a.bits[static_cast<size_t>(e.x) * a.words + w0 + lane] : 0u;
+        uint32_t inc = __popc(word);
+        const uint32_t own = inc;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, inc, o);
+            if (lane >= static_cast<uint32_t>(o)) inc += v;
+        }
+        const uint32_t n = __shfl_sync(FULL, inc, 31);
+        const uint32_t q0 = a.qBegin + (w0 + lane) * 32;
+        for (uint32_t at = inc - own; word; word &= word - 1) list[at++] = q0 + __ffs(word) - 1;
+        __syncwarp();
+        for (uint32_t from = 0; from < n; from += 32) batch(e.x, from, min(32u, n - from));
         __syncwarp();
     }
 }
@@ -774,7 +831,7 @@ __device__ __forceinline__ float boxGap2(const float* b, const float (&p)[DP]) {
 // memory, so no lane idles for another query's sake. Bound by the float pipe and the latency of a
 // cluster's first loads. 84M (query, point) tests of 4,096 queries, N = 10M, D = 8: 383 us (422 us before
 // the box test took three-input maxima and packed pairs; the walk's point passes: 2.9 ms for 187M).
-template <int DP>
+template <int DP, bool SLICES>
 __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(const __grid_constant__ KnnSweepArgs a) {
     __shared__ uint32_t sList[kSweepWarps][kSweepList];
     __shared__ __align__(16) float sP[kSweepWarps][32][DP];
@@ -851,7 +908,10 @@ __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(const __grid_con
         }
     };
 
-    sweepClusters(a, sList[w], batch);
+    if constexpr (SLICES)
+        sweepSlices(a, sList[w], batch);
+    else
+        sweepClusters<true>(a, sList[w], batch);
     if (lane == 0 && tested) atomicAdd(a.work + 1, tested);
     kept = __reduce_add_sync(FULL, kept);
     if (lane == 0 && kept) atomicAdd(a.hdr + 2 * (a.height + 1), kept);
@@ -1033,7 +1093,9 @@ __global__ void __launch_bounds__(kSweepThreads, DP <= 16 ? 4 : 2) knnSweepMmaKe
         }
     };
 
-    sweepClusters(a, sList[w], batch);
+    // (Not in slices: a product takes less time a query. 4,096 queries at one place, K = 100, N = 500k, D = 12: 14 ms,
+    // the level-synchronous walk 17.)
+    sweepClusters<false>(a, sList[w], batch);
     if (lane == 0 && tested) atomicAdd(a.work + 1, tested);
     kept = __reduce_add_sync(FULL, kept);
     if (lane == 0 && kept) atomicAdd(a.hdr + 2 * (a.height + 1), kept);
@@ -1099,10 +1161,15 @@ void launchKnnSweepPoints(const KnnSweepArgs& a, cudaStream_t s) {
         if constexpr (DP > 8)
             kern = knnSweepMmaKernel<DP>;
         else
-            kern = knnSweepKernel<DP>;
+            kern = knnSweepKernel<DP, false>;
         static const int grid = residentBlocks(reinterpret_cast<const void*>(kern), kSweepThreads);
         kern<<<grid, kSweepThreads, 0, s>>>(a);
         TBLAEQ_LAUNCHED();
+        if constexpr (DP <= 8) {
+            if (!a.sliced) return;
+            knnSweepKernel<DP, true><<<std::min(grid, 296), kSweepThreads, 0, s>>>(a);
+            TBLAEQ_LAUNCHED();
+        }
     });
 }
 

@@ -14,7 +14,8 @@
 //   sweep   one warp per cluster gathers the queries whose bit is set, 32 at a time, tests them
 //           against the cluster's point groups (boxes), and the groups' points against the queries
 //           whose box test passed, one point per lane, or above eight dimensions against all 32 as
-//           a product;
+//           a product. Clusters that many queries reach go to a second launch in slices of their
+//           queries (batches above 512, up to eight dimensions);
 //   finish  per query, the K smallest candidates by (FP64 squared distance, id).
 //
 // The tests run in single precision with a margin that covers every rounding (sweepPrepareKernel in
@@ -40,6 +41,9 @@ constexpr uint32_t paddedDims(uint64_t D) { return static_cast<uint32_t>((D + 3)
 
 // Largest |coordinate| (data or query) the float tests take: squared distances stay finite.
 constexpr double kSweepMaxAbs = 1e18;
+// Batches and clusters of more queries are sliced (sweepClusters). Up to it a cluster is one warp's work, 1.4 ms
+// at worst (512 queries at one place, K = 100, N = 1M, D = 3), as long as the level-synchronous walk takes.
+constexpr uint32_t kSweepSliced = 512;
 // Points a probe reads at most (its selection stage), and so the largest K it can bound.
 constexpr uint32_t kProbePoints = 4096;
 constexpr uint32_t kSweepMaxHeight = 16;
@@ -101,6 +105,13 @@ struct KnnSweepArgs {
     uint32_t* live;         // clusters with a bit set (blocks of at most 256 queries)
     uint32_t* liveCnt;
     uint32_t* ticket;
+    // Clusters that many queries reach (cluster, first of 32 words, queries there), at most one entry per 32
+    // words of every cluster: see sweepClusters.
+    int sliced;             // blocks above kSweepSliced queries, up to eight (padded) dimensions
+    uint4* heavy;
+    uint32_t* heavyCnt;
+    uint32_t* heavyTicket;
+    unsigned long long* reached;  // bits set
     uint32_t* hdr;          // the engine's level headers: (entries, items) of levels 0 .. height + 1
     unsigned long long* total; // results of the batch
     unsigned long long* work;  // [0] points the probe measured, [1] points the sweep tested

@@ -1,8 +1,8 @@
 """Which path a batch takes, and the level-synchronous walk's options on the walk itself.
 
 The sweeps' tests compare the default dispatch with the level-synchronous launches: this file asserts, by
-launch counts, that the default batches of those sizes do sweep (three launches for range, five for KNN,
-seven with a scorer) and which fall back. Options that only the walk knows (refinement, point groups in
+launch counts, that the default batches of those sizes do sweep (three launches for range, five for KNN, six
+above 512 queries, two more with a scorer) and which fall back. Options that only the walk knows (refinement, point groups in
 its point pass, wave 1) are tested with per-level counts asked for, which the sweeps don't serve: they
 change the walk's work and none of its results.
 """
@@ -64,10 +64,10 @@ def test_range_heights_and_clusters_sweep(tb, oracle_mod, cuda, D, ratios, sweep
 def test_knn_sweeps(tb, cuda, D, nq):
     h, pts = _index(tb, D)
     P = np.ascontiguousarray(pts[:nq] + 0.3)
-    assert _launches(tb, h, tb.QueryType.POINT, P, 7) == 5
+    assert _launches(tb, h, tb.QueryType.POINT, P, 7) == 5 + (nq > 512)
     assert _launches(tb, h, tb.QueryType.POINT, P, 7, tb.WANT_LEVELS) > 7
     h.scorer_train(np.ascontiguousarray(pts[:256] + 0.3), K=10, max_samples=2000, epochs=1, seed=1)
-    assert _launches(tb, h, tb.QueryType.POINT, P, 7) == 7
+    assert _launches(tb, h, tb.QueryType.POINT, P, 7) == 7 + (nq > 512)
 
 
 def _check_walk(tb, h, P, Kq, brute):
