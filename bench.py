@@ -496,10 +496,11 @@ def main():
     achieved = alg_bytes / final_mean_s / 1e9
     per_level = [{"level": m, "ms": level_ms[m], "algorithmic_bytes": level_bytes(m),
                   "GB/s": level_bytes(m) / (level_ms[m] / 1e3) / 1e9} for m in range(H)]
-    # Fewer kernels than levels: the batch ran as one sweep, which reads the boxes and, once each, the
-    # nodes above the clusters and the clusters' grid boxes (4·D), then the boxes and records of the
-    # groups it tests and the points of those it keeps, and writes the results and their offsets.
-    sweep = 0 < graph["kernels"] < H
+    # At most five kernels (the level-synchronous launches are H + 4): the batch ran as one sweep, which
+    # reads the boxes and, once each, the nodes above the clusters and the clusters' grid boxes (4·D),
+    # then the boxes and records of the groups it tests and the points of those it keeps, and writes the
+    # results and their offsets.
+    sweep = 0 < graph["kernels"] <= 5
     if sweep:
         alg_bytes = (args.nq * 16 * D + sum(mesh_nodes[:H - 2]) * (8 * D + 16) + mesh_nodes[H - 2] * 4 * D
                      + groups["groups"] * (8 * D + 16) + groups["points"] * 4 * D + results * 8 + (args.nq + 1) * 8)

@@ -53,4 +53,28 @@ struct SplitBatch : CudaError {
         TBLAEQ_CUDA(cudaGetLastError());                                      \
     } while (0)
 
+// A launch whose blocks may be placed before the launch ahead of it in the stream has ended (programmatic
+// dependent launch), so that its start costs no time of its own: the kernel ahead calls letNextLaunchStart,
+// and this one reads nothing before waitForEarlierLaunch, which returns when all of the other's writes are
+// visible.
+#ifdef __CUDACC__
+__device__ __forceinline__ void letNextLaunchStart() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void waitForEarlierLaunch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+void launchEarly(void (*kernel)(Params...), unsigned blocks, unsigned threads, cudaStream_t s, const Args&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    TBLAEQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+    TBLAEQ_LAUNCHED();
+}
+#endif
+
 }  // namespace tblaeq

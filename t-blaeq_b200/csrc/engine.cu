@@ -40,7 +40,7 @@ void BatchEngine::resetWorkspace() noexcept {
                          &cmpKids_, &cmpEntryOff_, &cmpKidOff_, &offsets_, &boxF_, &tau_, &candOff_, &knnCount_,
                          &knnOff_, &knnIds_, &knnD2_, &lbE_, &scoreE_, &sel_, &offF_, &waveM_, &selCount_, &selOff_,
                          &selIds_, &selD2_, &candOffB_, &candOffS_, &resIdsB_, &resQB_, &resDistB_, &swQuery_, &swBits_,
-                         &swLive_, &swCand_, &swEnt_, &rsBits_, &rsBoxF_, &rsRaw_, &rsSegs_})
+                         &swLive_, &swCand_, &swEnt_, &rsBits_, &rsBoxF_, &rsRaw_, &rsSegs_, &rsSlices_})
         m->release();
     rsRawCap_ = 0;
     rsSegWant_ = 0;
@@ -231,7 +231,8 @@ uint64_t BatchEngine::lastTotal(uint32_t nq) {
 
 size_t BatchEngine::workspaceBytes() const {
     size_t t = levelBytes();
-    for (const DeviceMem* m : {&swQuery_, &swBits_, &swLive_, &swCand_, &swEnt_, &rsBits_, &rsBoxF_, &rsRaw_, &rsSegs_}) t += m->bytes();
+    for (const DeviceMem* m : {&swQuery_, &swBits_, &swLive_, &swCand_, &swEnt_, &rsBits_, &rsBoxF_, &rsRaw_, &rsSegs_, &rsSlices_})
+        t += m->bytes();
     return t;
 }
 
@@ -319,7 +320,7 @@ void BatchEngine::reserve(const EngineCaps& want, uint32_t nq, unsigned flags) {
         offDesc_ = off;
         off = align256(off + (H + 1) * tileCap_ * 8);
         offTickets_ = off;
-        off = align256(off + (H + 2) * 4);
+        off = align256(off + (H + 4) * 4);
         offStatus_ = off;
         off = align256(off + 4);
         offHdr_ = off;
@@ -574,7 +575,8 @@ bool BatchEngine::reserveRangeSweep(uint32_t nq) {
     } grow[] = {{&rsBits_, rangeSweepBitBytes(upper, nq)},
                 {&rsBoxF_, nq * (5 * DP + 1) * 4},
                 {&rsSegs_, static_cast<uint64_t>(nq) * rangeSweepSlots(nq) * sizeof(RangeSegment)},
-                {&rsRaw_, caps_.results * 4}};
+                {&rsRaw_, caps_.results * 4},
+                {&rsSlices_, kRangeSlices * sizeof(uint2)}};
     uint64_t need = 0, held = 0;
     for (const Grow& g : grow)
         if (g.m->bytes() < g.bytes) {
@@ -593,7 +595,7 @@ bool BatchEngine::reserveRangeSweep(uint32_t nq) {
     }
     rsRawCap_ = rsRaw_.bytes() / 4;
     if (fits) return true;
-    for (DeviceMem* m : {&rsBits_, &rsBoxF_, &rsSegs_, &rsRaw_}) m->release();
+    for (const Grow& g : grow) g.m->release();
     rsRawCap_ = 0;
     rsSkip_ = kRangeSkip;
     return false;
@@ -603,7 +605,7 @@ bool BatchEngine::rangeSweepReady(uint32_t nq, unsigned flags) const {
     const uint64_t DP = paddedDims(di_.D), upper = di_.height > 2 ? di_.meshCount[di_.height - 3] : 1;
     return rsBits_.bytes() >= rangeSweepBitBytes(upper, nq) && rsBoxF_.bytes() >= nq * (5 * DP + 1) * 4 &&
            rsSegs_.bytes() >= static_cast<uint64_t>(nq) * rangeSweepSlots(nq) * sizeof(RangeSegment) &&
-           rsRawCap_ >= caps_.results && nq <= qcap_ && (!(flags & kWantVals) || haveVals_);
+           rsSlices_.bytes() && rsRawCap_ >= caps_.results && nq <= qcap_ && (!(flags & kWantVals) || haveVals_);
 }
 
 void BatchEngine::enqueueRangeSweep(const double* dBoxes, uint32_t nq, unsigned flags) {
@@ -656,6 +658,10 @@ void BatchEngine::enqueueRangeSweep(const double* dBoxes, uint32_t nq, unsigned 
     auto* tickets = reinterpret_cast<uint32_t*>(z + offTickets_);
     a.ticket = tickets;
     a.rawCnt = tickets + 1;
+    a.sliceCnt = tickets + 2;
+    a.sliceTicket = tickets + 3;
+    a.idle = tickets + 4;
+    a.slices = rsSlices_.as<uint2>();
     a.qsegs = reinterpret_cast<uint32_t*>(z + offQsegs_);
     a.qcount = reinterpret_cast<uint32_t*>(z + offQcount_);
     a.hdr = hdrPtr(0);

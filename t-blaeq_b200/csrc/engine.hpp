@@ -277,7 +277,7 @@ private:
     uint32_t controlStatus() const { return controlWord(offStatus_); }
     uint32_t controlHeader(int level, int which) const { return controlWord(offHdr_ + (2 * level + which) * 4); }
     // Exact range batches as one sweep (rangesweep.cuh): workspace, and whether the last range batch ran it.
-    DeviceMem rsBits_, rsBoxF_, rsRaw_, rsSegs_;
+    DeviceMem rsBits_, rsBoxF_, rsRaw_, rsSegs_, rsSlices_;
     static constexpr uint32_t kRangeSkip = 16;  // batches that run level by level after one the sweep could not serve
     uint32_t rsSegWant_ = 0, rsSkip_ = 0;
     uint64_t rsRawCap_ = 0;

@@ -698,7 +698,7 @@ __device__ __noinline__ bool measure(const KnnSweepArgs& a, uint32_t row, uint32
 // (sweepSlices). A batch whose queries lie together, or far outside the data, reaches a hundred clusters with
 // nearly all of its queries; one warp for each of those took 11.9 ms (4,096 queries, K = 100, N = 1M, D = 3;
 // the level-synchronous walk 4.9) where spread queries take 0.36. In slices it takes 0.76; the second launch
-// costs 2 to 5 us where there are none. (Taken by the same launch's warps as they run out of clusters it took
+// (placed early, see launchEarly) costs 2 to 5 us where there are none. (Taken by the same launch's warps as they run out of clusters it took
 // 18 ms: most have left when the first slice appears.)
 template <bool SLICED, class Batch>
 __device__ __forceinline__ void sweepClusters(const KnnSweepArgs& a, uint32_t* list, Batch&& batch) {
@@ -835,6 +835,10 @@ template <int DP, bool SLICES>
 __global__ void __launch_bounds__(kSweepThreads) knnSweepKernel(const __grid_constant__ KnnSweepArgs a) {
     __shared__ uint32_t sList[kSweepWarps][kSweepList];
     __shared__ __align__(16) float sP[kSweepWarps][32][DP];
+    if constexpr (SLICES)
+        waitForEarlierLaunch();
+    else if (a.sliced)
+        letNextLaunchStart();
     __shared__ float sThr[kSweepWarps][32];
     __shared__ uint32_t sId[kSweepWarps][32];
     __shared__ __align__(16) float sBox[kSweepWarps][kSweepGroups][2 * DP];
@@ -1167,8 +1171,7 @@ void launchKnnSweepPoints(const KnnSweepArgs& a, cudaStream_t s) {
         TBLAEQ_LAUNCHED();
         if constexpr (DP <= 8) {
             if (!a.sliced) return;
-            knnSweepKernel<DP, true><<<std::min(grid, 296), kSweepThreads, 0, s>>>(a);
-            TBLAEQ_LAUNCHED();
+            launchEarly(knnSweepKernel<DP, true>, std::max(1, grid / 2), kSweepThreads, s, a);
         }
     });
 }

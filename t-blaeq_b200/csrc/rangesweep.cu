@@ -298,7 +298,13 @@ struct SweepShape {
 // that meet: node, groups, points), so resident warps count: registers are held to seven blocks an SM
 // and the rare exact tests are out of line. 24M (query, cluster) pairs of 4,096 boxes (N = 10M, D = 8):
 // 143 us; with 2 D float comparisons a pair 180 us.
-template <int DP, bool ROWS>
+//
+// Once a task has had kHeavyPairs (query, cluster) pairs and three quarters of the blocks' first warps have none any
+// more, the rest of it is left to a second launch (SLICES) in a few queries each: boxes that lie together meet
+// the same few units with all of their queries, and one warp a task took 6.0 ms (4,096 boxes of +-8% at one
+// place, N = 10M, D = 8; the level-synchronous launches 1.2), in slices 0.78.
+constexpr uint32_t kHeavyPairs = 64;
+template <int DP, bool ROWS, bool SLICES>
 __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<DP, ROWS>::kBlocks) rangeSweepKernel(RangeSweepArgs a, uint32_t nTasks,
                                                                                     uint32_t qPer, uint32_t parts) {
     constexpr int WARPS = SweepShape<DP, ROWS>::kWarps;
@@ -311,6 +317,10 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
     __shared__ uint32_t sHit[WARPS][kHits];
     // ROWS: the hits of the (query, cluster) pair at hand, a bit per row of the cluster.
     __shared__ uint32_t sPair[WARPS][ROWS ? kRangeRowsCluster / 32 : 1];
+    if constexpr (SLICES)
+        waitForEarlierLaunch();
+    else if (a.sliced)
+        letNextLaunchStart();
     if (ROWS && (threadIdx.x & 31) < kRangeRowsCluster / 32) sPair[threadIdx.x >> 5][threadIdx.x & 31] = 0;
     __syncwarp();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -321,12 +331,23 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
     const int hLast = H - 1;  // header of the clusters that survive
     uint32_t nEntries = 0, nItems = 0, nKept = 0, nTested = 0;
 
-    for (uint32_t task = blockIdx.x * WARPS + w; task < nTasks;) {
+    for (uint32_t task = blockIdx.x * WARPS + w; SLICES || task < nTasks;) {
+        uint32_t sliceFrom = 0, sliceN = 0;
+        if constexpr (SLICES) {  // the next slice
+            uint32_t t = 0;
+            if (lane == 0) t = atomicAdd(a.sliceTicket, 1u);
+            t = __shfl_sync(FULL, t, 0);
+            if (t >= min(*a.sliceCnt, kRangeSlices)) break;
+            const uint2 e = a.slices[t];
+            task = e.x;
+            sliceFrom = e.y & 0xffffu;
+            sliceN = e.y >> 16;
+        }
         const uint32_t qb = task / (a.nUnits * parts), up = task - qb * a.nUnits * parts;
         const uint32_t u = up / parts, part = up - u * parts;
         // The next task: the first ones are dealt out, the rest claimed.
         uint32_t next = 0;
-        if (lane == 0) next = warps + atomicAdd(a.ticket, 1u);
+        if (!SLICES && lane == 0) next = warps + atomicAdd(a.ticket, 1u);
         const RangeUnit un = a.units[u];
         // The task's queries: qPer of them (a power of two) from qb * qPer on; list entries count from qBase.
         const uint32_t qBase = qb * qPer / 32 * 32, wi = qBase / 32 + lane;
@@ -368,8 +389,9 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
                     (d + 3 < DP / 2 ? clo[d + 3] : chi[d + 3 - DP / 2]) = v.w;
                 }
             }
-            for (uint32_t from = 0; from < nLive; from += 32) {
-                const uint32_t nB = min(32u, nLive - from);
+            uint32_t taskPairs = 0;
+            for (uint32_t from = SLICES ? sliceFrom : 0u; from < (SLICES ? sliceFrom + sliceN : nLive); from += 32) {
+                const uint32_t nB = SLICES ? sliceN : min(32u, nLive - from);
                 const uint32_t myQ = qBase + (static_cast<uint32_t>(lane) < nB ? sList[w][from + lane] : sList[w][from]);
                 __syncwarp();
                 for (uint32_t i = lane; i < nB * (DP / 2); i += 32) {  // the outward box, in pieces of 16 bytes
@@ -408,6 +430,18 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
                 }
                 const uint32_t nPairs = __shfl_sync(FULL, inc, 31);
                 if (nPairs == 0) continue;
+                taskPairs += nPairs;
+                if (!SLICES && taskPairs > kHeavyPairs && a.sliced && *static_cast<volatile uint32_t*>(a.idle) > gridDim.x / 4 * 3) {
+                    const uint32_t per = min(32u, max(1u, 16u * kHeavyPairs / nPairs)), cnt = (nB + per - 1u) / per;
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(a.sliceCnt, cnt);
+                    at = __shfl_sync(FULL, at, 0);
+                    const bool fits = at < kRangeSlices && cnt <= kRangeSlices - at;  // else no queries, and the warp's own
+                    const uint32_t left = nB > lane * per ? nB - lane * per : 0u;
+                    if (static_cast<uint32_t>(lane) < cnt && at < kRangeSlices && static_cast<uint32_t>(lane) < kRangeSlices - at)
+                        a.slices[at + lane] = make_uint2(task, (from + lane * per) | (fits ? min(per, left) << 16 : 0u));
+                    if (fits) continue;
+                }
                 {
                     uint32_t at = inc - own;
                     while (bits) {
@@ -636,6 +670,7 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
         __syncwarp();
         task = next;
     }
+    if (!SLICES && threadIdx.x == 0 && a.sliced) atomicAdd(a.idle, 1u);
     nEntries = __reduce_add_sync(FULL, nEntries);
     nItems = __reduce_add_sync(FULL, nItems);
     nKept = __reduce_add_sync(FULL, nKept);
@@ -796,12 +831,18 @@ void launchPadded(const RangeSweepArgs& a, cudaStream_t s) {
     rangeUpperKernel<DP><<<chunks * wordBlocks, uw * 32, 0, s>>>(a, perBlock, wordBlocks, byUnit ? 1 : 0);
     TBLAEQ_LAUNCHED();
     constexpr int WARPS = SweepShape<DP, ROWS>::kWarps;
-    static const int full = residentBlocks(reinterpret_cast<const void*>(rangeSweepKernel<DP, ROWS>), WARPS * 32);
+    static const int full = residentBlocks(reinterpret_cast<const void*>(rangeSweepKernel<DP, ROWS, false>), WARPS * 32);
     const RangeSweepTasks t = rangeSweepTasks(a.nUnits, a.nq);
     const uint32_t nTasks = static_cast<uint32_t>(t.count);
     const uint32_t blocks = std::min<uint32_t>(static_cast<uint32_t>(full), (nTasks + WARPS - 1) / WARPS);
-    rangeSweepKernel<DP, ROWS><<<std::max(1u, blocks), WARPS * 32, 0, s>>>(a, nTasks, t.qPer, t.parts);
+    // (Tasks of fewer queries are short enough: the second launch costs about 5 us where it has nothing to do.)
+    RangeSweepArgs b = a;
+    b.sliced = std::min(a.nq, t.qPer) >= 128;
+    rangeSweepKernel<DP, ROWS, false><<<std::max(1u, blocks), WARPS * 32, 0, s>>>(b, nTasks, t.qPer, t.parts);
     TBLAEQ_LAUNCHED();
+    if (b.sliced) {
+        launchEarly(rangeSweepKernel<DP, ROWS, true>, std::max(1, full / 2), WARPS * 32, s, b, nTasks, t.qPer, t.parts);
+    }
     // A few queries may hold many results each, and every block of a query orders all of its segments: large
     // blocks share a query then, about as many as are resident at once, at least 4,096 results each. 20 boxes
     // with 6.4M results (N = 1M, D = 2): the gather takes 132 us; 590 us with 236 shares of 128 threads,

@@ -1,4 +1,4 @@
-// Exact range batches in three launches: upper test, sweep, gather.
+// Exact range batches in three launches (four with slices): upper test, sweep, gather.
 //
 //   upper   one thread per (node, 32 queries) over the meshes above the finest clusters: bit (node,
 //           query) of the last of them = the node and its ancestors survive for the query;
@@ -98,6 +98,8 @@ inline bool rangeSweepNarrow(uint64_t height, uint64_t top, uint64_t upper, uint
            (clusters < 4 * upper && (nUnits > 65536 || nq >= 2048)) || (height >= 5 && clusters < 8 * upper && nq >= 512);
 }
 
+constexpr uint32_t kRangeSlices = 1u << 18;  // slices of a launch; batches beyond are not sliced
+
 struct RangeSegment {
     uint64_t key;  // unit, then the run's number within it
     uint32_t pos;  // first hit
@@ -144,7 +146,12 @@ struct RangeSweepArgs {
     uint32_t rawCap;
     RangeSegment* segs;     // nq x segSlots
     uint32_t segSlots;
+    int sliced;             // set at the launch: batches of many pairs are left as slices
+    uint2* slices;          // kRangeSlices of (task, first list entry | queries << 16)
     // Zeroed before the launch:
+    uint32_t* sliceCnt;
+    uint32_t* sliceTicket;
+    uint32_t* idle;         // blocks of the sweep whose first warp has no task any more
     uint32_t* ticket;
     uint32_t* rawCnt;
     uint32_t* qsegs;        // segments per query

@@ -1,7 +1,7 @@
 """Which path a batch takes, and the level-synchronous walk's options on the walk itself.
 
 The sweeps' tests compare the default dispatch with the level-synchronous launches: this file asserts, by
-launch counts, that the default batches of those sizes do sweep (three launches for range, five for KNN, six
+launch counts, that the default batches of those sizes do sweep (three launches for range, four with slices, five for KNN, six
 above 512 queries, two more with a scorer) and which fall back. Options that only the walk knows (refinement, point groups in
 its point pass, wave 1) are tested with per-level counts asked for, which the sweeps don't serve: they
 change the walk's work and none of its results.
@@ -135,7 +135,7 @@ def test_narrow_indexes(tb, cuda, D, N, ratios, nq, sweeps):
     """Small fan-outs over many nodes: the level-synchronous launches, with the sweep's results."""
     h, pts = _index(tb, D, N, ratios)
     Q = _boxes(pts, nq, 5, 0.001, 0.01)
-    assert (_launches(tb, h, tb.QueryType.RANGE, Q) == 3) == sweeps
+    assert (_launches(tb, h, tb.QueryType.RANGE, Q) <= 4) == sweeps
     r = h.query_batch(tb.QueryType.RANGE, Q, tb.Mode.EXACT)
     offs, ids = r.offsets.numpy().astype(np.int64), r.ids.numpy()
     names = h.decode_points(np.arange(N))[1]
