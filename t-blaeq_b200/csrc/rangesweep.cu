@@ -317,10 +317,12 @@ __global__ void __launch_bounds__(SweepShape<DP, ROWS>::kWarps * 32, SweepShape<
     __shared__ uint32_t sHit[WARPS][kHits];
     // ROWS: the hits of the (query, cluster) pair at hand, a bit per row of the cluster.
     __shared__ uint32_t sPair[WARPS][ROWS ? kRangeRowsCluster / 32 : 1];
-    if constexpr (SLICES)
+    if constexpr (SLICES) {
         waitForEarlierLaunch();
-    else if (a.sliced)
+        if (*a.sliceCnt == 0) return;
+    } else if (a.sliced) {
         letNextLaunchStart();
+    }
     if (ROWS && (threadIdx.x & 31) < kRangeRowsCluster / 32) sPair[threadIdx.x >> 5][threadIdx.x & 31] = 0;
     __syncwarp();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
