@@ -240,8 +240,9 @@ int tblaeq_group_counts(tblaeq_handle* h, uint64_t* out3);
  * src/Kernel/SpMSpV.cuh:24) ----
  * Exact range batches whose shapes are all at their defaults (variant 0, 100%) run as one sweep over the
  * hierarchy instead of one launch per mesh (same results in the same order, same per-level counts); any
- * other shape asks for the level-synchronous launches. tblaeq_autotune leaves the defaults where the
- * sweep is the faster.
+ * other shape asks for the level-synchronous launches, which also serve indexes of small fan-outs and
+ * batches without memory for the sweep. tblaeq_autotune leaves the defaults where the sweep is the
+ * faster.
  * A launch shape per expand launch (one per mesh, `height` of them): the kernel variant (0 = direct,
  * 1 = staged) and the persistent grid as a percentage (1..100) of the kernel's full occupancy.
  * tblaeq_autotune searches variant x grid {100, 75, 50, 25}% per level on the live batch. */
@@ -285,7 +286,8 @@ int tblaeq_set_knn_probe(tblaeq_handle* h, uint32_t beam, int node_major_complet
  * each query's nearest clusters, their points bound its K-th distance, and every cluster is tested
  * against that bound at once. The options below then tune the probe (tblaeq_set_knn_wave1: its width,
  * twelve times as many clusters without a scorer) or do not apply (the refinement: the probe's bound
- * leaves it nothing). Other choices run the level-synchronous walk. Same results either way.
+ * leaves it nothing). Other choices run the level-synchronous walk, and so do batches with a K above
+ * 2,048 or above the points of 32 clusters. Same results either way.
  *
  * Wave 1 of a two-wave KNN batch reads every point of each query's ceil(scale * K / leaf) + 1
  * best-ranked finest clusters (at least 2, at most 32; leaf = the index's points per finest cluster)

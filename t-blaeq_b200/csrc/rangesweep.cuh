@@ -1,23 +1,24 @@
 // Exact range batches in three launches (four with slices): upper test, sweep, gather.
 //
-//   upper   one thread per (node, 32 queries) over the meshes above the finest clusters: bit (node,
-//           query) of the last of them = the node and its ancestors survive for the query;
-//   sweep   one warp per (unit, 1,024 queries), a unit being at most 32 sibling clusters: lanes are
+//   upper   a warp per word of 32 queries, a query a lane, over staged units of at most eight sibling
+//           nodes of the mesh above the finest clusters: bit (node, query) = the node and its ancestors
+//           survive for the query;
+//   sweep   one warp per (unit, up to 1,024 queries), a unit being at most 32 sibling clusters: lanes are
 //           clusters while their boxes are tested against the queries whose bit is set, then
 //           (query, cluster) pairs, then (query, group) pairs, then points. Hits go out as segments:
 //           runs of points of one query and one unit, in traversal order;
 //   gather  per query, its segments in the order of their units, as ids (and coordinates).
 //
 // Against one launch per level this keeps nothing between the levels in memory: no frontier with its
-// coordinates, no look-back, no per-level tail. Every (query, node) pair is decided by the same
-// tests as there -- float box, FP64 radius, float point with the FP64 test near a face -- so the same
+// coordinates, no look-back, no per-level tail. Every (query, node) pair is decided as there: float box, FP64
+// radius (in float first, outside a margin), float point with the FP64 test near a face. So the same
 // nodes survive at every level, the counts per level are the same, and so are the results and their
 // order (depth-first: queries, then the clusters in traversal order, then the points: in point-group
 // order at D = 4, 8 and 16, in row order elsewhere).
 //
 // Measured on B200 against the level-synchronous launches, device time of one batch: 4,096 boxes, N = 10M,
 // D = 8: 620 -> 220 us; 37 boxes there: 105 -> 46 us; 100 boxes, N = 500k, D = 5: 110 -> 60 us; one box:
-// 60 -> 28 us; 301 boxes with 1.0M results and their coordinates, N = 1.5M, D = 3: 180 -> 146 us.
+// 60 -> 28 us; 301 boxes with 1.0M results and their coordinates, N = 1.5M, D = 3: 180 -> 140 us.
 #pragma once
 
 #include <cstdint>
