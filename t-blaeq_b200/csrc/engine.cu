@@ -1528,7 +1528,7 @@ bool BatchEngine::useKnnSweep(uint32_t nq, unsigned flags, uint32_t maxK) const 
     // = 170, fan-outs 5, N = 1M: 133 against 29; at K = 155 the sweep is the faster). So it is for a few queries
     // over a wide mesh 0, which one CTA a query ranks (one query, 111,000 nodes: 411 us against 336; ten: as fast).
     const uint64_t nodes = di_.meshCount[0], clusters = di_.meshCount[di_.height - 2], points = di_.meshCount[di_.height - 1];
-    if (static_cast<uint64_t>(maxK) * clusters > 32 * points && points > kSweepFactorMax * (4ull * maxK + 64)) return false;
+    if (static_cast<uint64_t>(maxK) * clusters > 32 * points && points > kSweepWhole * (4ull * maxK + 64)) return false;
     if (di_.height > 2 && nodes > 65536 && nq < 8) return false;
     // Per-level counts and the scorer's training traces describe the level-synchronous walk, and so do
     // the options that change it; a streamed last interval has no decoded points on the device.
@@ -1559,8 +1559,11 @@ bool BatchEngine::reserveKnnSweep(uint32_t nq, uint64_t sumK, uint64_t cand) {
         entries = std::max<uint64_t>(swEntCap_, nq * each * 5 / 4 + 1024);
         if (entries > 0xffffffffull) return false;  // their counter has 32 bits
     }
-    // Candidates that only an earlier batch's ties asked for are given back.
-    const bool shrink = swCandGrown_ && 2 * cand < swCandCap_;
+    // Candidates that only an earlier batch's ties asked for are given back where they take more than 1 GiB; below,
+    // the next such batch finds them, and a growth takes a quarter more (an allocation waits for all lanes).
+    constexpr uint64_t kKept = (1ull << 30) / 16;
+    const bool shrink = swCandGrown_ && 2 * cand < swCandCap_ && swCandCap_ > kKept;
+    if (swCandCap_ < cand && cand <= kKept) cand += cand / 4;
     struct Grow {
         DeviceMem* m;
         uint64_t bytes;
@@ -1710,7 +1713,7 @@ void BatchEngine::enqueueKnnSweep(const double* dPoints, uint32_t nq, const uint
 
 bool BatchEngine::runKnnSweep(const double* dPoints, uint32_t nq, const uint32_t* dK, uint64_t sumK, BatchOutput& o) {
     // Candidate slots are 4 K + 64 a query (the bound is within a few percent of the K-th distance, so
-    // about 1.5 K pass); 4 to 64 times that once a batch needed it (D = 16: 1,000 queries, N = 5M, K = 20,
+    // about 1.5 K pass); 4 to 256 times that once a batch needed it (D = 16: 1,000 queries, N = 5M, K = 20,
     // some above 576), where that takes at most 8 GiB. Where ties or a loose bound pass more, every
     // query's count is known after the run, and a second one gives each its own; the batches after it don't
     // keep those.

@@ -299,7 +299,7 @@ private:
     uint64_t swCandCap_ = 0, swEntCap_ = 0;
     uint64_t *swOff_ = nullptr, *swCandOff_ = nullptr;
     uint32_t *swCnt_ = nullptr, *swWant_ = nullptr;
-    uint32_t swFactor_ = 1;     // 1, 4, 16 or 64: see runKnnSweep
+    uint32_t swFactor_ = 1;     // 1, 4, 16, 64 or 256: see runKnnSweep
     bool swCandGrown_ = false;  // swCand_ holds more than batches without many ties ask for
     bool swLast_ = false, knnTrace_ = false;
     bool useKnnSweep(uint32_t nq, unsigned flags, uint32_t maxK) const;

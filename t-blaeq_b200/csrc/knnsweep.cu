@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kProbeThreads) knnProbeKernel(const __grid_con
         // walk's case, unless slots that stay for the next batches hold them all (41 queries of K = 600,
         // fan-outs 4 and 3, N = 60,000: 1.8 ms against the walk's 5; N = 600,000: 18 ms against 11).
         const uint64_t r = min(static_cast<uint64_t>(K), a.nPoints);
-        if (isinf(tau) && a.nPoints > kSweepFactorMax * (4 * r + 64)) atomicOr(a.status, kStatusKnnFallback);
+        if (isinf(tau) && a.nPoints > kSweepWhole * (4 * r + 64)) atomicOr(a.status, kStatusKnnFallback);
         const double t = (tau + static_cast<double>(margin)) * (1.0 + 1e-7);
         a.tau[q] = tau;
         a.tauF[q] = __double2float_ru(t);

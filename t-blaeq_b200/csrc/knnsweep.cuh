@@ -47,8 +47,11 @@ constexpr uint32_t kSweepSliced = 512;
 // Points a probe reads at most (its selection stage), and so the largest K it can bound.
 constexpr uint32_t kProbePoints = 4096;
 constexpr uint32_t kSweepMaxHeight = 16;
-// Most times 4 K + 64 candidate slots a query that batches keep for the ones after them (a power of four).
-constexpr uint32_t kSweepFactorMax = 64;
+// Most times 4 K + 64 candidate slots a query that batches keep for the ones after them (a power of four): with a
+// scorer and small K single queries need more than 64 (N = 100M, D = 8), and a second run on every batch.
+constexpr uint32_t kSweepFactorMax = 256;
+// An index of at most this many times 4 K + 64 points is swept also without a bound.
+constexpr uint32_t kSweepWhole = 64;
 
 struct KnnSweepLevel {
     const float* x;        // centres, paddedDims floats per node
